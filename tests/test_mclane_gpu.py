@@ -44,6 +44,18 @@ def test_device_stream_equals_the_oracle(seed):
         assert np.array_equal(pathcube.chacha8_normals(seed, first, count), want[first:first + count])
 
 
+@pytest.mark.parametrize("first,count", [
+    (0, 1), (0, 31), (0, 2047), (0, 2049), (2040, 20),            # around one 2048-word segment
+    (0, 128 * 2048 - 3000), (128 * 2048 - 4000, 8000),            # around one group of 128 segments
+    (255 * 2048, 3 * 128 * 2048 + 77), (900_001, 1),
+])
+def test_stream_ranges_across_segments_and_groups(first, count):
+    """The parallel parse at its seams: ranges that start, end and straddle the parse's segments and
+    segment groups are the oracle's draws, bit for bit."""
+    want = np.frombuffer(O.chacha8_normals(99, first + count), dtype=np.float64)[first:]
+    assert np.array_equal(pathcube.chacha8_normals(99, first, count).view(np.uint64), want.view(np.uint64))
+
+
 def test_correlated_block_equals_the_oracle():
     for corr in ([[1.0, 0.5], [0.5, 1.0]], [[1.0, 0.3, 0.1], [0.3, 1.0, 0.2], [0.1, 0.2, 1.0]]):
         L = O.cholesky(corr)
