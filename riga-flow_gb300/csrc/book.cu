@@ -180,7 +180,7 @@ void plan_book(const rg_book_request* r, const BookScenarios& sc, BookPlan& B) {
     d.inc_a = (float)(d.coupon_rate / (double)d.ps_a);
     d.inc_b = (float)(d.coupon_rate / (double)(d.ps_a + 1));
   }
-  // work order: grouped by underlying count (one launch each), longest trades first in a group
+  // work order: grouped by underlying count, longest trades first in a group
   B.order.resize(B.n_trades);
   for (int j = 0; j < B.n_trades; ++j) B.order[j] = j;
   std::stable_sort(B.order.begin(), B.order.end(), [&](int a, int b) {
@@ -450,13 +450,16 @@ void increments_maps(const float* incr, uint64_t npaths, uint64_t rowlen, int U,
     maps[n - 1] = increments_map(incr, npaths, rowlen, U, TU, sh.Pb, book_stage_steps(n, sh.TT));
 }
 
-// Paths per generation chunk: a multiple of `unit` whose increments fit the budget.
+// Paths per generation chunk: a multiple of `unit` whose increments fit the budget, the chunks of a
+// book about equal (a short last chunk would leave the persistent scan's CTAs without items).
 uint64_t chunk_paths(uint64_t paths, int U, int64_t TU, size_t elem, uint64_t unit) {
   const uint64_t per_path = (uint64_t)U * (uint64_t)TU * elem;
   uint64_t cap = kIncrBudget / per_path;
   cap = cap / unit * unit;
   if (cap < unit) cap = unit;
-  return paths < cap ? paths : cap;
+  if (paths <= cap) return paths;
+  const uint64_t chunks = (paths + cap - 1) / cap, even = (paths + chunks - 1) / chunks;
+  return (even + unit - 1) / unit * unit;
 }
 
 }  // namespace bk
@@ -470,16 +473,8 @@ size_t estimate_book_bytes(const rg_book_request* r, int n_scen) {
   const uint64_t P = r->config.paths;
   const bool fp32 = r->config.precision == RG_PRECISION_FP32;
   const size_t elem = fp32 ? sizeof(float) : sizeof(double);
-  int group[RG_NMAX] = {0};
-  for (int32_t j = 0; j < r->n_trades; ++j) {
-    const int n = r->trades[j].terms.n_assets;
-    if (n >= 1 && n <= RG_NMAX) ++group[n - 1];
-  }
-  int gmin = 0;
-  for (int n = 0; n < RG_NMAX; ++n)
-    if (group[n] > 0 && (gmin == 0 || group[n] < gmin)) gmin = group[n];
   const uint64_t unit =
-      fp32 ? (uint64_t)book32_shape((int)std::min<size_t>(S, 32), device_sm_count(), P, gmin).blk_paths : 128;
+      fp32 ? (uint64_t)book32_shape((int)std::min<size_t>(S, 32), device_sm_count(), P, r->n_trades).blk_paths : 128;
   const uint64_t PC = chunk_paths(P, (int)U, (int64_t)TU, elem, unit);
   const uint64_t chunks = (P + PC - 1) / PC;
   size_t b = (size_t)PC * U * TU * elem * (fp32 && chunks > 1 ? 2 : 1);
@@ -546,8 +541,8 @@ void run_book(rg_engine* E, const rg_book_request* r, const BookScenarios& sc, r
   if (fp32) {
     // the path blocks (hence the sums) follow the device's SM count; the persistent scans' grid
     // follows the engine's SM cap
-    Book32Shape sh = book32_shape(B.S, device_sm_count(), P, B.min_group());
-    sh.grid = std::min(sh.grid, book32_shape(B.S, engine_sm_count(E), P, B.min_group()).grid);
+    Book32Shape sh = book32_shape(B.S, device_sm_count(), P, B.n_trades);
+    sh.grid = std::min(sh.grid, book32_shape(B.S, engine_sm_count(E), P, B.n_trades).grid);
     const uint64_t PC = chunk_paths(P, B.U, B.TU, sizeof(float), (uint64_t)sh.blk_paths);
     const uint64_t n_chunks = (P + PC - 1) / PC;
     const uint64_t blocks_per_chunk = (PC + sh.blk_paths - 1) / sh.blk_paths;
@@ -588,7 +583,8 @@ void run_book(rg_engine* E, const rg_book_request* r, const BookScenarios& sc, r
       }
       CUtensorMap maps[RG_NMAX];
       increments_maps(buf, np, rowlen, B.U, B.TU, sh, maps);
-      launch_book_trade32(st.bk, sh, maps, np, c * blocks_per_chunk, B.group_lo, B.group_n, partial, scratch, status, s0);
+      launch_book_trade32(st.bk, sh, maps, np, c * blocks_per_chunk, B.group_lo, B.group_n, partial, scratch + 8,
+                          status, s0);
       cuda_check(cudaEventRecord(E->book_ev[2 + (c & 1)], s0), "event");
     }
     double* dsums = static_cast<double*>(book_buf(E, BK_SUMS, sizeof(double) * pairs * RG_ACC));
@@ -598,8 +594,8 @@ void run_book(rg_engine* E, const rg_book_request* r, const BookScenarios& sc, r
     cuda_check(cudaMemcpyAsync(hs.data(), dsums, sizeof(double) * hs.size(), cudaMemcpyDeviceToHost, s0), "D2H");
     cuda_check(cudaMemcpyAsync(&hstat, status, sizeof(int), cudaMemcpyDeviceToHost, s0), "D2H");
     cuda_check(cudaStreamSynchronize(s0), "book pricing");
-    if (hstat == KSTAT_TIMEOUT) raise(RG_ERR_TIMEOUT, "book_trade32_kernel: a bounded stage wait ran out");
-    if (hstat) raise(RG_ERR_GPU_ERROR, "book_trade32_kernel reported a bad work item");
+    if (hstat == KSTAT_TIMEOUT) raise(RG_ERR_TIMEOUT, "book scan: a bounded stage wait ran out");
+    if (hstat) raise(RG_ERR_GPU_ERROR, "book scan reported a bad work item");
     for (size_t k = 0; k < hs.size(); ++k)
       if (!std::isfinite(hs[k])) raise(RG_ERR_GPU_ERROR, "book: non-finite path sums");
     for (int p = 0; p < pairs; ++p) finish(hs.data() + (size_t)p * RG_ACC, P, r->config.seed, &out[p]);

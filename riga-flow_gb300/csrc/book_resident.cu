@@ -4,8 +4,8 @@
 // Cholesky factor stay on the device, and so do the universe's FP32 increments of every path
 // (generated once at creation; they do not depend on the scenarios).  Each rg_book_price call
 // then only prices: it plans the scenario tables on the host, writes them to a pinned staging
-// buffer and replays a CUDA graph of the device work — the scenario upload, one persistent TMA
-// scan per underlying count, the fixed-order reduction and the download of the sums — captured
+// buffer and replays a CUDA graph of the device work — the scenario upload, the persistent TMA
+// scan, the fixed-order reduction and the download of the sums — captured
 // on the first call for that scenario count.  Before the capture, an autotuner times the scan's
 // stage depth (time steps per TMA stage) on a prefix of the paths and keeps the fastest; the
 // stage depth changes only the schedule, never the arithmetic, so results equal rg_price_book's
@@ -65,7 +65,7 @@ int autotune_stage(rg_book* b, const Book32Shape& base) {
   const int S = b->B.S;
   std::vector<int> cands;
   for (int tt : {8, 16, 32, 64})
-    if (2 * 5 * tt * base.Pb * 4 <= 168 * 1024) cands.push_back(tt);
+    if (book32_smem(tt, base.Pb) <= 168 * 1024) cands.push_back(tt);
   const uint64_t np = std::min<uint64_t>(b->P, (uint64_t)base.blk_paths * 4);
   const size_t pbytes = sizeof(double) * ((np + base.blk_paths - 1) / base.blk_paths) * b->B.n_trades * S * RG_ACC;
   DevBuf tpartial;
@@ -79,7 +79,6 @@ int autotune_stage(rg_book* b, const Book32Shape& base) {
   for (int tt : cands) {
     Book32Shape sh = base;
     sh.TT = tt;
-    sh.smem = 2 * 5 * tt * sh.Pb * 4 + 64;
     CUtensorMap maps[RG_NMAX];
     increments_maps(static_cast<float*>(b->incr.ptr), b->P, b->rowlen, b->B.U, b->B.TU, sh, maps);
     int32_t* scr = static_cast<int32_t*>(b->scratch.ptr);
@@ -88,7 +87,7 @@ int autotune_stage(rg_book* b, const Book32Shape& base) {
       cuda_check(cudaMemsetAsync(scr, 0, 256, E->stream), "tune status");
       cuda_check(cudaEventRecord(e0, E->stream), "event");
       launch_book_trade32(bkd, sh, maps, np, 0, b->B.group_lo, b->B.group_n, static_cast<double*>(tpartial.ptr),
-                          scr, scr + 1, E->stream);
+                          scr + 8, scr + 1, E->stream);
       cuda_check(cudaEventRecord(e1, E->stream), "event");
       cuda_check(cudaEventSynchronize(e1), "tune");
       cuda_check(cudaEventElapsedTime(&ms, e0, e1), "event time");
@@ -133,9 +132,8 @@ void price_resident(rg_book* b, const BookScenarios& spec, rg_price_result* out)
     memcpy(g.scen_host.ptr, sp.pk.host.data(), scen_bytes);
     cuda_check(cudaMemcpyAsync(g.scen_dev.ptr, g.scen_host.ptr, scen_bytes, cudaMemcpyHostToDevice, E->stream), "H2D");
     point_scenarios(sp, static_cast<uint8_t*>(g.scen_dev.ptr), S, b->st.bk);
-    Book32Shape sh = book32_shape(S, device_sm_count(), b->P, b->B.min_group());
+    Book32Shape sh = book32_shape(S, device_sm_count(), b->P, b->B.n_trades);
     sh.TT = autotune_stage(b, sh);
-    sh.smem = 2 * 5 * sh.TT * sh.Pb * 4 + 64;
     b->tuned[spec.per_trade ? 1000 + S : S] = sh.TT;
     const uint64_t blocks = (b->P + sh.blk_paths - 1) / sh.blk_paths;
     g.partial.ensure(sizeof(double) * blocks * pairs * RG_ACC);
@@ -152,7 +150,7 @@ void price_resident(rg_book* b, const BookScenarios& spec, rg_price_result* out)
                  "scenarios H2D");
       cuda_check(cudaMemsetAsync(scr, 0, 256, E->stream), "status reset");
       launch_book_trade32(b->st.bk, sh, maps, b->P, 0, b->B.group_lo, b->B.group_n, static_cast<double*>(g.partial.ptr),
-                          scr, scr + 1, E->stream);
+                          scr + 8, scr + 1, E->stream);
       launch_book_reduce_strided(static_cast<double*>(g.partial.ptr), (int64_t)blocks, (int64_t)pairs * RG_ACC, RG_ACC,
                                  pairs, static_cast<double*>(g.sums.ptr), E->stream);
       cuda_check(cudaMemcpyAsync(g.sums_host.ptr, g.sums.ptr, sizeof(double) * pairs * RG_ACC, cudaMemcpyDeviceToHost,

@@ -340,7 +340,7 @@ struct BookDev {
   const float* dfm_f;
   const double* L;             // [U][U] universe Cholesky factor (FP64)
   const float* L32;            // [U][U] the same in FP32
-  const int32_t* order;        // [n_trades] trade order of the work items (longest first)
+  const int32_t* order;        // [n_trades] trade order of the work items (by underlying count, longest first)
 };
 // Universe increments of paths [path0, path0 + npaths): incr[t][u][p], FP64 ΔW/√dt (parity) or
 // FP32 ΔW (production, rows of `rowlen` >= npaths floats so that tensor-map strides are aligned).
@@ -357,18 +357,25 @@ void launch_book_trade64(const DevTrade& gen, const BookDev& bk, const double* i
 // FP32 persistent scan: work items (path block, trade) with block-major order; every item's
 // FP64 sums land in partial[(block0 + b) * n_trades + j][S][RG_ACC].
 struct Book32Shape {
-  int threads, Sb, Pb, TT, grid, blk_paths, smem;
+  int threads, ns, Pb, TT, grid, blk_paths;  // ns: scenarios per thread
 };
-// `paths`: the book's path count; `min_group_trades`: trades in its smallest underlying-count group.
-Book32Shape book32_shape(int S, int sm_count, uint64_t paths, int min_group_trades);
-// `tmap` views the chunk's increments as [TU][U][npaths] floats (boxes of Pb paths × 1 asset × TT
-// steps) for the kernel's TMA stages.
-// One persistent launch per underlying count n with trades order[group_lo[n-1], + group_n[n-1]).
-// `maps[n - 1]`: the increments' tensor map with boxes of book_stage_steps(n, sh.TT) steps.
+// `paths`, `n_trades`: the book's path and trade counts.
+Book32Shape book32_shape(int S, int sm_count, uint64_t paths, int n_trades);
+// Steps per stage for trades on n underlyings: the stage buffers hold 5 × base steps of one
+// underlying, so fewer underlyings take proportionally deeper stages (fewer hand-overs per step) in
+// the same shared memory, a multiple of four steps and at most 160 (a box edge may not exceed 256).
+__host__ __device__ inline int book_stage_steps(int n, int base) {
+  const int tt = base * 5 / n & ~3;
+  return tt < 160 ? tt : 160;
+}
+// Shared-memory bytes of the two stage buffers at a base stage depth.
+inline int book32_smem(int base, int Pb) { return 2 * 5 * base * Pb * 4; }
+// `maps[n - 1]` views the chunk's increments as [TU][U][npaths] floats (boxes of Pb paths × 1 asset ×
+// book_stage_steps(n, sh.TT) steps) for the kernel's TMA stages of trades on n underlyings, which are
+// order[group_lo[n-1], + group_n[n-1]); `counter`: RG_NMAX words.
 void launch_book_trade32(const BookDev& bk, const Book32Shape& sh, const CUtensorMap* maps, uint64_t npaths,
                          uint64_t block0, const int* group_lo, const int* group_n, double* partial,
                          int32_t* counter, int* status, cudaStream_t s);
-int book_stage_steps(int n, int base);
 // The FP32 copy of the universe Cholesky factor.
 void launch_book_l32(const double* L, int U, float* L32, cudaStream_t s);
 // Fixed-order sums over path blocks: out[pair][k] = Σ_b partial[b·stride_b + pair·stride_pair + k].

@@ -146,6 +146,49 @@ def test_fp32_book_is_deterministic_across_calls(engine):
     assert [bytes(x) for x in a] == [bytes(x) for x in c]
 
 
+@pytest.mark.parametrize("paths", [1, 63, 65, 129, 2049])
+def test_fp32_scan_shapes_agree(engine, paths):
+    """Every launch shape of the FP32 scan (one or two scenarios a thread, 64 to 256 paths a tile,
+    idle scenario slots, ragged last tiles) gives a (trade, scenario) the same paths: event counts
+    equal and path sums equal up to the order of at most 2049 / 32 FP64 additions."""
+    b = workloads.small_book(paths=paths, n_trades=10, fp32=True)
+    sc = [m for _, m in workloads.book_scenarios(b.universe)]
+    sc = (sc * 3)[:32]
+    full = engine.price_book_raw(b, sc)
+    for S in (1, 2, 3, 4, 5, 8, 9, 16, 17, 31):
+        part = engine.price_book_raw(b, sc[:S])
+        for j in range(len(b.trades)):
+            for s in range(S):
+                a, w = part[j * S + s], full[j * 32 + s]
+                assert list(a.path_sums)[12:] == list(w.path_sums)[12:], (S, j, s)
+                for x, y in zip(list(a.path_sums)[:12], list(w.path_sums)[:12]):
+                    assert abs(x - y) <= 1e-13 * paths, (S, j, s)
+
+
+@pytest.mark.parametrize("edit", [
+    dict(coupon_periods=1), dict(coupon_periods=36), dict(coupon_periods=50), dict(coupon_periods=7),
+    dict(fixed_first_coupon=True), dict(call_start_step=0), dict(call_start_step=35), dict(call_start_step=100),
+    dict(call_start_step=None), dict(knock_out_barrier=None), dict(coupon_barrier=None), dict(memory_coupon=False),
+    dict(knock_out_barrier=0.5, call_start_step=0), dict(coupon_periods=3, fixed_first_coupon=True, call_start_step=12),
+])
+def test_fp32_scan_schedules_match_fp64(engine, edit):
+    """Schedules at the edges of the scan's step runs (one period, a period per step, more periods
+    than steps, a fixed first period, calls from the first or last step or never): events equal the
+    FP64 scan's on the same points, prices within the FP32 state's rounding (36 steps of 2^-24)."""
+    b64 = workloads.small_book(paths=256, n_trades=10)
+    for t in b64.trades:
+        t.terms.steps, t.terms.maturity_years = b64.universe_steps, b64.universe_maturity_years
+        for k, v in edit.items():
+            setattr(t.terms, k, v)
+    b32 = copy.deepcopy(b64)
+    b32.options = workloads.production_options()
+    r64 = engine.price_book_trade_bumps_raw(b64)
+    r32 = engine.price_book_trade_bumps_raw(b32)
+    for a, w in zip(r32, r64):
+        assert list(a.path_sums)[12:] == list(w.path_sums)[12:]
+        assert abs(a.pv - w.pv) <= 1e-5
+
+
 def test_book_errors_keep_the_reference_codes(engine):
     b = workloads.small_book(paths=64, n_trades=2)
     b.trades[1].underlyings[0] = 77
