@@ -369,7 +369,6 @@ BookStaged stage_book_static(DevBuf& tables, cudaStream_t st, const rg_book_requ
   const size_t o_tr = pk.add(B.trades), o_ord = pk.add(B.order);
   const size_t o_corr = pk.add(r->universe.correlation, (size_t)U * U);
   const size_t o_L = pk.reserve(sizeof(double) * U * U), o_L32 = pk.reserve(sizeof(float) * U * U);
-  const size_t o_work = pk.reserve(sizeof(double) * 2 * U * U);
   tables.ensure(pk.host.size());
   uint8_t* dev = static_cast<uint8_t*>(tables.ptr);
   cuda_check(cudaMemcpyAsync(dev, pk.host.data(), pk.host.size(), cudaMemcpyHostToDevice, st), "book H2D");
@@ -394,9 +393,7 @@ BookStaged stage_book_static(DevBuf& tables, cudaStream_t st, const rg_book_requ
   out.L32 = reinterpret_cast<float*>(dev + o_L32);
   bk.L = out.L;
   bk.L32 = out.L32;
-  launch_cholesky_big(reinterpret_cast<const double*>(dev + o_corr), U, out.L,
-                      reinterpret_cast<double*>(dev + o_work), st);
-  launch_book_l32(out.L, U, out.L32, st);
+  launch_cholesky_big(reinterpret_cast<const double*>(dev + o_corr), U, out.L, out.L32, st);
   return out;
 }
 

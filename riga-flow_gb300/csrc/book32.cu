@@ -553,16 +553,6 @@ void launch_book_trade32(const BookDev& bk, const Book32Shape& sh, const CUtenso
   else go(book_scan32_kernel<2, 64>);
 }
 
-__global__ void book_l32_kernel(const double* __restrict__ L, int n, float* __restrict__ L32) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) L32[i] = (float)L[i];
-}
-
-void launch_book_l32(const double* L, int U, float* L32, cudaStream_t s) {
-  book_l32_kernel<<<(U * U + 255) / 256, 256, 0, s>>>(L, U * U, L32);
-  cuda_check(cudaGetLastError(), "book_l32_kernel launch");
-}
-
 // out[pair][k] = Σ_b partial[b·stride_b + pair·stride_pair + k], b in order.
 __global__ void book_reduce_kernel(const double* __restrict__ partial, int64_t blocks, int64_t stride_b,
                                    int64_t stride_pair, int pairs, double* __restrict__ out) {

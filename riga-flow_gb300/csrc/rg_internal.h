@@ -295,11 +295,9 @@ void launch_phoenix32(const Prepared& P, const DevTables& tb, const DevScenario*
 void launch_reduce(const double* partial, int rows, int n_scen, double* out, cudaStream_t s);
 size_t reduce_scratch_doubles(int rows, int n_scen);
 
-// The 32-bit Sobol integers at which the inverse normal switches between its central and tail
-// branches (computed in FP64 so the FP32 kernels branch exactly as the reference does).
 // Cholesky factor (with the reference's PSD clamp) of one n×n correlation, n <= RG_BOOK_MAX_UNIVERSE,
-// by one device thread; `work` holds 2·n·n doubles.
-void launch_cholesky_big(const double* c, int n, double* l, double* work, cudaStream_t s);
+// by one warp, and the factor rounded to FP32.
+void launch_cholesky_big(const double* c, int n, double* l, float* l32, cudaStream_t s);
 
 // ------------------------------------------------------------------ books ---------------------
 // One book trade's constants on the device.
@@ -376,8 +374,6 @@ inline int book32_smem(int base, int Pb) { return 2 * 5 * base * Pb * 4; }
 void launch_book_trade32(const BookDev& bk, const Book32Shape& sh, const CUtensorMap* maps, uint64_t npaths,
                          uint64_t block0, const int* group_lo, const int* group_n, double* partial,
                          int32_t* counter, int* status, cudaStream_t s);
-// The FP32 copy of the universe Cholesky factor.
-void launch_book_l32(const double* L, int U, float* L32, cudaStream_t s);
 // Fixed-order sums over path blocks: out[pair][k] = Σ_b partial[b·stride_b + pair·stride_pair + k].
 void launch_book_reduce_strided(const double* partial, int64_t blocks, int64_t stride_b, int64_t stride_pair,
                                 int pairs, double* out, cudaStream_t s);

@@ -530,3 +530,21 @@ def test_production_halton_lane_matches_the_oracle(engine):
         want = engine.price_raw(r64)
         got = engine.price_raw(r32)
         assert abs(got.pv - want.pv) <= min(0.1 * want.mc_error, 1e-4), (paths, got.pv, want.pv)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("rho", [0.0, 0.5, 0.99, 0.99998, 0.99999999, 1.0 - 1e-11, -0.2, -0.9])
+def test_correlation_factor_across_conditioning(engine, n, rho):
+    """The device factor on well-conditioned matrices (no eigenvalue search), near-singular ones (the
+    search without a clamp) and ones the PSD clamp repairs: per-path records equal the oracle's
+    within the 1e-12 of every FP64 parity test, so the branch and the factor are the reference's."""
+    req = workloads.plain3(paths=64, steps=24)
+    req.trade = workloads.phoenix_trade(n, 24, 24 / 252)
+    req.market.spots, req.market.vols = [100.0] * n, [0.2 + 0.03 * f for f in range(n)]
+    req.market.dividend_yields = [0.01] * n
+    req.market.correlation = [[1.0 if i == j else rho ** (1 + (i + j) % 2) for j in range(n)] for i in range(n)]
+    got = engine.run_paths_raw(req, 0, 64)
+    for g, w in zip(got, O.run_paths(req, 0, 64)):
+        assert (g.ko_step, g.qualified_steps, g.paid_periods) == (w.ko_step, w.qualified_steps, w.paid_periods)
+        assert abs(g.pv - w.pv) <= 1e-12 * abs(w.pv)
+        assert abs(g.worst_final - w.worst_final) <= 1e-12 * abs(w.worst_final)
