@@ -1,12 +1,4 @@
-// book32.cu — FP32 production kernels of a book.
-//
-// book_gen32_kernel: the universe's correlated Brownian increments of a chunk of paths,
-// incr[t][u][p] = ΔW (variance dt), FP32, written once to HBM and read by every trade.  A CTA is
-// 32 paths × U assets (threadIdx.x = path lane, threadIdx.y = asset): at every bridge node each
-// thread draws its asset's QMC normal once into shared memory, then forms its correlated normal
-// y_u = Σ_{b<=u} L[u][b]·z_b from the shared row and advances the streamed bridge of (path, u).
-// The bridge is applied after the correlation, as in the reference (note.rs:89-106).  Each warp
-// writes 32 consecutive paths of one (step, asset): 128-byte coalesced stores.
+// book32.cu — the FP32 production scan of a book (its universe increments: book_gen32.cu).
 //
 // book_scan32_kernel: persistent, one launch for every trade.  Work items are (path block, trade),
 // taken from an atomic counter per underlying count, five underlyings first: the code of a count is
@@ -36,50 +28,6 @@
 #include "rg_internal.h"
 
 namespace rg {
-
-__global__ void __launch_bounds__(1024) book_gen32_kernel(DevTrade gen, DevTables tb,
-                                                          const float* __restrict__ L32, int U,
-                                                          uint64_t path0, uint64_t npaths, uint64_t rowlen,
-                                                          float* __restrict__ incr) {
-  __shared__ float zs[2][RG_BOOK_MAX_UNIVERSE][33];
-  const int lane = threadIdx.x, u = threadIdx.y;
-  const uint64_t p = (uint64_t)blockIdx.x * 32 + lane;
-  const bool ok = p < npaths;
-  const uint64_t point = path0 + (ok ? p : 0);
-  const int64_t T = gen.steps;
-  float lrow[RG_BOOK_MAX_UNIVERSE];
-#pragma unroll
-  for (int b = 0; b < RG_BOOK_MAX_UNIVERSE; ++b) lrow[b] = b <= u && b < U ? __ldg(L32 + u * U + b) : 0.0f;
-  float wcur = 0.0f, stk[RG_STACK_MAX];
-  int sp = 0, buf = 0;
-  for (int64_t t = 0; t < T; ++t) {
-    const int c0 = __ldg(tb.node_off + t), c1 = __ldg(tb.node_off + t + 1);
-    for (int c = c0; c < c1; ++c) {
-      const int k = __ldg(tb.node_k + c);
-      zs[buf][u][lane] = rg_qmc_normal32(gen, tb, point, (uint64_t)k * (uint64_t)U + (uint64_t)u);
-      __syncthreads();
-      float y = 0.0f;
-#pragma unroll
-      for (int b = 0; b < RG_BOOK_MAX_UNIVERSE; ++b)
-        if (b <= u) y = fmaf(lrow[b], zs[buf][b][lane], y);
-      const float cf = __ldg(tb.node_cf + c);
-      stk[sp] = c == 0 ? y * cf : fmaf(y, cf, 0.5f * (wcur + stk[sp - 1]));
-      ++sp;
-      buf ^= 1;  // the next node writes the other row: one barrier per node suffices
-    }
-    --sp;
-    const float wn = stk[sp];
-    if (ok) incr[((uint64_t)t * U + u) * rowlen + p] = wn - wcur;
-    wcur = wn;
-  }
-}
-
-void launch_book_gen32(const DevTrade& gen, const DevTables& tb, const float* L32, int U,
-                       uint64_t path0, uint64_t npaths, uint64_t rowlen, float* incr, cudaStream_t s) {
-  const unsigned blocks = (unsigned)((npaths + 31) / 32);
-  book_gen32_kernel<<<blocks, dim3(32, U), 0, s>>>(gen, tb, L32, U, path0, npaths, rowlen, incr);
-  cuda_check(cudaGetLastError(), "book_gen32_kernel launch");
-}
 
 // ------------------------------------------------------------------ TMA-staged scan ----------
 // The increments a (trade, path tile) stage needs — for each of the trade's N underlyings, TT

@@ -225,7 +225,7 @@ extern "C" int32_t rg_book_create(rg_engine* e, const rg_book_request* request, 
                                          " GiB) exceed the resident budget; price it with rg_price_book");
     b->incr.ensure(ibytes);
     b->scratch.ensure(256);
-    launch_book_gen32(b->B.gen, b->st.tb, b->st.L32, U, request->config.first_path, b->P, b->rowlen,
+    launch_book_gen32(b->B.gen, b->st.tb, b->st.L32, U, b->B.br.stack_max, request->config.first_path, b->P, b->rowlen,
                       static_cast<float*>(b->incr.ptr), e->stream);
     cuda_check(cudaStreamSynchronize(e->stream), "book generation");
     *out = b.release();

@@ -200,6 +200,22 @@ __device__ __forceinline__ double rg_probit64(double p) {
 // sqrt(w) - 3.7161102 beyond.  No division, one fast logarithm, no FP64; within 4e-7 relative of
 // the exact inverse normal, which the reference's Acklam approximation (qmc.rs:37-91) matches to
 // 1.15e-9.
+// The tail polynomial, w >= 5.
+__device__ __forceinline__ float rg_ninv32_tail(float w) {
+  const float v = sqrtf(w) - 3.716110200f;
+  float g = 5.467908077e-06f;
+  g = fmaf(g, v, -1.174909974e-05f);
+  g = fmaf(g, v, -2.363354380e-05f);
+  g = fmaf(g, v, 9.947906459e-05f);
+  g = fmaf(g, v, -1.555746239e-04f);
+  g = fmaf(g, v, 2.347132999e-04f);
+  g = fmaf(g, v, -4.239792245e-04f);
+  g = fmaf(g, v, 8.495624679e-04f);
+  g = fmaf(g, v, -1.928687814e-03f);
+  g = fmaf(g, v, 3.093904488e-03f);
+  g = fmaf(g, v, 1.426282266e+00f);
+  return fmaf(g, v, 5.025157229e+00f);
+}
 __device__ __forceinline__ float rg_ninv32_lower(float p2, float s) {
   const float w = -__logf(fmaf(p2, s, p2));
   float g;
@@ -215,19 +231,7 @@ __device__ __forceinline__ float rg_ninv32_lower(float p2, float s) {
     g = fmaf(g, t, 3.488026599e-01f);
     g = fmaf(g, t, 2.123313567e+00f);
   } else {
-    const float v = sqrtf(w) - 3.716110200f;
-    g = 5.467908077e-06f;
-    g = fmaf(g, v, -1.174909974e-05f);
-    g = fmaf(g, v, -2.363354380e-05f);
-    g = fmaf(g, v, 9.947906459e-05f);
-    g = fmaf(g, v, -1.555746239e-04f);
-    g = fmaf(g, v, 2.347132999e-04f);
-    g = fmaf(g, v, -4.239792245e-04f);
-    g = fmaf(g, v, 8.495624679e-04f);
-    g = fmaf(g, v, -1.928687814e-03f);
-    g = fmaf(g, v, 3.093904488e-03f);
-    g = fmaf(g, v, 1.426282266e+00f);
-    g = fmaf(g, v, 5.025157229e+00f);
+    g = rg_ninv32_tail(w);
   }
   return s * g;
 }
@@ -243,6 +247,42 @@ __device__ __forceinline__ float rg_probit32(uint32_t x) {
   const float s = fmaf((float)(0x7FFFFFFFu - xl), 4.656612873077393e-10f, 2.3283064365386963e-10f);
   const float q = rg_ninv32_lower(p2, s);
   return lower ? -q : q;
+}
+
+// rg_probit32 of two points in packed FP32x2 arithmetic, each with rg_probit32's operations; the
+// logarithm's argument is at least 2^-32, so the hardware's flush-to-zero form needs no scaling of
+// subnormals (three instructions of the general form).
+__device__ __forceinline__ float2 rg_probit32x2(uint32_t xa, uint32_t xb) {
+  auto both = [](float a) { return make_float2(a, a); };
+  auto neg_ln = [](float a) {
+    float l;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(a));
+    return l * -0.6931471805599453f;
+  };
+  const uint32_t ya = xa ^ (uint32_t)((int32_t)xa >> 31), yb = xb ^ (uint32_t)((int32_t)xb >> 31);  // min(x, ~x)
+  const float2 c = both(4.656612873077393e-10f), h = both(2.3283064365386963e-10f);
+  const float2 p2 = __ffma2_rn(make_float2((float)(int32_t)ya, (float)(int32_t)yb), c, h);
+  const float2 s = __ffma2_rn(make_float2((float)(int32_t)(ya ^ 0x7FFFFFFFu), (float)(int32_t)(yb ^ 0x7FFFFFFFu)), c, h);
+  const float2 v = __ffma2_rn(p2, s, p2);
+  const float2 w = make_float2(neg_ln(v.x), neg_ln(v.y));
+  const float2 t = __fadd2_rn(w, both(-2.5f));
+  float2 g = both(4.035466097e-08f);
+  g = __ffma2_rn(g, t, both(4.861039695e-07f));
+  g = __ffma2_rn(g, t, both(-4.990565522e-06f));
+  g = __ffma2_rn(g, t, both(-6.217993119e-06f));
+  g = __ffma2_rn(g, t, both(3.091502040e-04f));
+  g = __ffma2_rn(g, t, both(-1.773010155e-03f));
+  g = __ffma2_rn(g, t, both(-5.908170971e-03f));
+  g = __ffma2_rn(g, t, both(3.488026599e-01f));
+  g = __ffma2_rn(g, t, both(2.123313567e+00f));
+  if (fmaxf(w.x, w.y) >= 5.0f) {  // 0.7% of pairs
+    if (w.x >= 5.0f) g.x = rg_ninv32_tail(w.x);
+    if (w.y >= 5.0f) g.y = rg_ninv32_tail(w.y);
+  }
+  const float2 q = __fmul2_rn(s, g);
+  // negative in the lower half
+  return make_float2(__uint_as_float(__float_as_uint(q.x) ^ (~xa & 0x80000000u)),
+                     __uint_as_float(__float_as_uint(q.y) ^ (~xb & 0x80000000u)));
 }
 
 // ------------------------------------------------------------------ Halton -------------------

@@ -344,8 +344,13 @@ struct BookDev {
 // FP32 ΔW (production, rows of `rowlen` >= npaths floats so that tensor-map strides are aligned).
 void launch_book_gen64(const DevTrade& gen, const DevTables& tb, const double* L, int U,
                        uint64_t path0, uint64_t npaths, double* incr, cudaStream_t s);
-void launch_book_gen32(const DevTrade& gen, const DevTables& tb, const float* L32, int U,
+// `depth`: the bridge's anchor stack.
+void launch_book_gen32(const DevTrade& gen, const DevTables& tb, const float* L32, int U, int depth,
                        uint64_t path0, uint64_t npaths, uint64_t rowlen, float* incr, cudaStream_t s);
+// Builds the consumption-order Sobol tables of n factors over tr.steps nodes from tb.sobol and tb.node_k
+// into `out` (64·n·steps words) on the device, for launches whose first path is first_path modulo 32,
+// and points tb at them.
+void launch_sobol_lut(const DevTrade& tr, DevTables& tb, int n, uint64_t first_path, uint32_t* out, cudaStream_t s);
 // FP64 scan of every (trade, scenario) on the chunk's increments: one thread per (pair, path);
 // partial[pair][block][RG_ACC] over `blocks` blocks of 128 paths; records[p][pair] when given.
 // partial[pair][block][RG_ACC] with `blocks` blocks of 128 paths per pair.

@@ -21,6 +21,7 @@ import oracle as O
 from riga_gb300 import abi, workloads
 from riga_gb300.build import build_library
 from riga_gb300.engine import Engine
+from riga_gb300.types import BookTrade
 
 pytestmark = pytest.mark.gpu
 
@@ -163,6 +164,31 @@ def test_fp32_scan_shapes_agree(engine, paths):
                 assert list(a.path_sums)[12:] == list(w.path_sums)[12:], (S, j, s)
                 for x, y in zip(list(a.path_sums)[:12], list(w.path_sums)[:12]):
                     assert abs(x - y) <= 1e-13 * paths, (S, j, s)
+
+
+@pytest.mark.parametrize("assets,first,lane", [
+    (1, 0, "shift"), (3, 31, "shift"), (4, 1, "owen"), (5, 7, "shift"), (8, 30, "owen"), (13, 32, "shift"),
+    (20, 1000, "shift"), (21, 4095, "shift"), (32, 65503, "shift"), (32, 17, "owen"), (6, 3, "halton"),
+])
+def test_fp32_universe_generation_matches_fp64(engine, assets, first, lane):
+    """The FP32 universe increments (Sobol points from consumption-order tables at any offset within a
+    32-point block, the packed inverse normal, the correlation of 1 to 32 assets) through one-asset
+    trades on every asset: events equal the FP64 book's on the same points, prices within the FP32
+    state's rounding."""
+    b64 = workloads.small_book(paths=200, n_assets=assets, n_trades=1)
+    t = b64.trades[0].terms
+    t.initial_spots = [100.0]
+    b64.trades = [BookTrade(copy.deepcopy(t), [a]) for a in range(assets)]
+    b64.options.first_path = first
+    if lane == "owen":
+        b64.options.scrambler, b64.options.dim_mode = abi.SCRAMBLE_OWEN, abi.DIM_WRAP_REFERENCE
+    elif lane == "halton":
+        _halton(b64)
+    b32 = copy.deepcopy(b64)
+    b32.options.precision = abi.PRECISION_FP32
+    for a, w in zip(engine.price_book_raw(b32), engine.price_book_raw(b64)):
+        assert list(a.path_sums)[12:] == list(w.path_sums)[12:]
+        assert abs(a.pv - w.pv) <= 1e-5
 
 
 @pytest.mark.parametrize("edit", [
