@@ -307,6 +307,12 @@ static Staged stage(Workspace& W, const rg_price_request* req, Prepared& P) {
     o_hp = pk.add(hp);
   }
   size_t o_flags = pk.add(P.step_flags), o_per = pk.add(P.step_period), o_acc = pk.add(P.accr_inc);
+  // the FP64 lane's accrual sums, where it runs through a keeping workspace (path64.cu)
+  size_t o_accs = 0, o_acca = 0;
+  if (W.persistent()) {
+    o_accs = pk.add(P.accr_sum);
+    o_acca = pk.add(P.accr_at);
+  }
   size_t o_noff = pk.add(P.node_off), o_nk = pk.add(P.node_k), o_nc = pk.add(P.node_c),
          o_ncf = pk.add(P.node_cf), o_nfr = pk.add(P.nf_row), o_nfs = pk.add(P.nf_shift);
   size_t o_ti = pk.add(P.lv_ti), o_tw = pk.add(P.lv_tw), o_twf = pk.add(P.lv_twf);
@@ -424,6 +430,8 @@ static Staged stage(Workspace& W, const rg_price_request* req, Prepared& P) {
   tb.step_flags = reinterpret_cast<const uint32_t*>(base + o_flags);
   tb.step_period = reinterpret_cast<const int32_t*>(base + o_per);
   tb.accr_inc = reinterpret_cast<const double*>(base + o_acc);
+  tb.accr_sum = reinterpret_cast<const double*>(base + o_accs);
+  tb.accr_at = reinterpret_cast<const int32_t*>(base + o_acca);
   tb.node_off = reinterpret_cast<const int32_t*>(base + o_noff);
   tb.node_k = reinterpret_cast<const int32_t*>(base + o_nk);
   tb.node_c = reinterpret_cast<const double*>(base + o_nc);
@@ -589,14 +597,14 @@ void price_with(Workspace& W, const rg_price_request* req, const rg_scenario* sc
     Staged S = stage(W, req, P);
     LaunchOut lo{};
     lo.mcz = mcz;
-    // rows of partial sums: one per block of the FP64 kernel, one per 32-path chunk of the FP32 kernels
+    // rows of partial sums: one per block of the FP64 kernels, one per 32-path chunk of the FP32 kernels
     uint64_t rows;
     Fp32Shape sh{};
     if (fp32) {
       sh = phoenix32_shape(P, paths, W.sm_count);
       rows = p32_chunks(paths);
     } else {
-      rows = (uint64_t)phoenix64_grid(P, paths);
+      rows = W.persistent() ? path64_rows(P.n, paths) : (uint64_t)phoenix64_grid(paths);
     }
     if (rows > (uint64_t)INT32_MAX) raise(RG_ERR_INVALID_PATHS, "too many paths for one launch");
     const int grid = (int)rows;
@@ -613,11 +621,13 @@ void price_with(Workspace& W, const rg_price_request* req, const rg_scenario* sc
     if (fp32) {
       sh = phoenix32_tune(P, S.tb, S.scen, S.scen32, path0, paths, sh, lo, W.may_tune(), W.sm_count, W.stream);
       launch_phoenix32(P, S.tb, S.scen, S.scen32, path0, paths, sh, lo, W.stream);
+    } else if (W.persistent()) {
+      launch_path64(W, P, S.tb, S.scen, path0, paths, lo, W.stream);
     } else {
       launch_phoenix64(P, S.tb, S.scen, path0, paths, lo, W.stream);
     }
     if (W.timing) {
-      W.timing->block = fp32 ? sh.threads : 128;
+      W.timing->block = fp32 ? sh.threads : 64;
       W.timing->smem_bytes = fp32 ? sh.smem : 0;
       W.timing->tile_steps = fp32 && !sh.direct ? sh.TT : 0;
       W.timing->paths_per_thread = fp32 && !sh.direct ? sh.ppt : 1;
@@ -707,7 +717,8 @@ size_t estimate_price_bytes(const rg_price_request* r, int n_scen) {
   }
   if (fp32) b += T * 160;  // bridge plans of the tiled kernel
   // rows of partial sums: one per 32-path chunk (FP32 kernels) or per block (FP64 kernel)
-  const size_t grid = fp32 ? (size_t)p32_chunks(r->config.paths) : 152 * 16;
+  const size_t grid = (size_t)(fp32 ? p32_chunks(r->config.paths) : path64_rows((int)std::min<size_t>(n, RG_NMAX), r->config.paths));
+  if (!fp32) b += path64_bytes((int)std::min<size_t>(n, RG_NMAX), (int64_t)T, r->config.paths);
   b += grid * std::min<size_t>(S, 32) * RG_ACC * 8 + S * RG_ACC * 8;  // partial and reduced sums
   b += reduce_scratch_doubles((int)std::min<size_t>(grid, INT32_MAX), (int)std::min<size_t>(S, 32)) * 8;
   if (r->config.trace_level != RG_TRACE_OFF) b += (size_t)r->config.paths * 4;
@@ -956,7 +967,7 @@ static void run_path_range(rg_engine* e, const rg_price_request* req, uint64_t f
     lo.mcz = mcz;
     Fp32Shape sh{};
     if (fp32) sh = phoenix32_shape(P, m, engine_sm_count(e));
-    lo.grid = fp32 ? (int)p32_chunks(m) : phoenix64_grid(P, m);
+    lo.grid = (int)(fp32 ? p32_chunks(m) : path64_rows(P.n, m));
     lo.partial = static_cast<double*>(W.device(WS_PARTIAL, (size_t)lo.grid * P.n_scen * RG_ACC * sizeof(double)));
     if (out) lo.records = static_cast<rg_path_record*>(W.device(WS_RECORDS, m * sizeof(rg_path_record)));
     if (cube) lo.cube = static_cast<float*>(W.device(WS_CUBE, m * cube_row * sizeof(float)));
@@ -967,7 +978,7 @@ static void run_path_range(rg_engine* e, const rg_price_request* req, uint64_t f
       launch_phoenix32(P, S.tb, S.scen, S.scen32, path0, m, sh, lo, e->stream);
     }
     else
-      launch_phoenix64(P, S.tb, S.scen, path0, m, lo, e->stream);
+      launch_path64(W, P, S.tb, S.scen, path0, m, lo, e->stream);
     if (out)
       cuda_check(cudaMemcpyAsync(out + done, lo.records, m * sizeof(rg_path_record), cudaMemcpyDeviceToHost,
                                  e->stream), "D2H records");

@@ -354,6 +354,15 @@ void bridge_schedule_into(int64_t T, double dt, Prepared& P) {
   P.node_cf.assign(P.node_c.begin(), P.node_c.end());
 }
 
+// The smallest spot s >= 0 with s / init >= barrier as FP64 rounds the ratio (rounding is monotone, so
+// every larger spot reaches the barrier too and no smaller one does).
+static double smallest_spot(double barrier, double init) {
+  double s = std::max(barrier * init, 0.0);
+  while (s > 0.0 && s / init >= barrier) s = std::nextafter(s, 0.0);
+  while (!(s / init >= barrier) && s < INFINITY) s = std::nextafter(s, INFINITY);
+  return s;
+}
+
 void prepare(const rg_price_request* r, const rg_scenario* sc, int n_scen, Prepared& P) {
   const rg_phoenix_trade& t = r->trade;
   const rg_simulation_config& c = r->config;
@@ -382,6 +391,10 @@ void prepare(const rg_price_request* r, const rg_scenario* sc, int n_scen, Prepa
   tr.coupon_rate = t.has_coupon_rate ? t.coupon_rate : 0.0;
   tr.strike = t.strike;
   tr.ki = t.knock_in_barrier;
+  for (int f = 0; f < n; ++f) {
+    tr.cb_spot[f] = smallest_spot(tr.coupon_barrier, tr.init[f]);
+    tr.ko_spot[f] = smallest_spot(tr.call_barrier, tr.init[f]);
+  }
   tr.coupon_f = (float)tr.coupon_rate;
   tr.strike_f = (float)tr.strike;
   tr.neg_half_dt_f = (float)(-0.5 * tr.dt);
@@ -436,6 +449,15 @@ void prepare(const rg_price_request* r, const rg_scenario* sc, int n_scen, Prepa
     P.accr_inc[p] = tr.coupon_rate / (double)ps;
   }
   P.accr_f.assign(P.accr_inc.begin(), P.accr_inc.end());
+  // what a period's daily accruals add up to, in the order the reference adds them (note.rs:168)
+  std::vector<int32_t> period_len((size_t)PER, 0);
+  for (int64_t s = 0; s < T; ++s) ++period_len[P.step_period[s]];
+  P.accr_at.resize(PER);
+  for (int64_t p = 0; p < PER; ++p) {
+    P.accr_at[p] = (int32_t)P.accr_sum.size();
+    double sum = 0.0;
+    for (int32_t k = 0; k <= period_len[p]; ++k, sum += P.accr_inc[p]) P.accr_sum.push_back(sum);
+  }
 
   bridge_schedule_into(T, tr.dt, P);
   // per (node, factor): the QMC dimension n·k + f reduced to its table row, and its shift mask

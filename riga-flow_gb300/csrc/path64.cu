@@ -1,0 +1,444 @@
+// path64.cu — the FP64 parity kernels of an engine: normals, then stepping and payoff.
+//
+// The reference's arithmetic (crates/riga-engine/src/note.rs:81-259) in its own operation order,
+// product by product, as phoenix64.cu performs it in one kernel; here the work is split where its
+// shape changes, through a buffer of a chunk of paths:
+//   * normals64_kernel — correlated normals y = L·z of every bridge node, y[node][asset][path].  A
+//     CTA forms the normals of 256 paths × a few nodes; the 5% that fall into the inverse normal's
+//     tails (a logarithm, a square root and a division) are queued in shared memory and taken 32 at
+//     a time, where a warp of one path a lane would enter the tail for 54% of its normals on either
+//     side.  correlate64_kernel does the same from the pseudo-random lane's stream.
+//   * step64_kernel — a lane per (path, asset): the streamed bridge, the GBM / Dupire step, and the
+//     Phoenix state machine replicated over a path's lanes, which agree on the barriers by a vote.
+//     Barriers compare spots against the smallest spot whose ratio reaches the barrier (found on the
+//     host by rounding the ratio both ways), so no division and no FP64 comparison runs per step,
+//     and a period's accruals are counted and looked up.
+// What bounds it: the FP64 pipe (rg_fp64.cuh): per (path, step, asset) about 37 operations in the
+// normals, 34 in a flat step and 88 in a local-vol one; and, below about four warps an SM, the
+// latency of a step's dependent operations, which a lane per asset halves or better.
+// Measured: 3 assets flat, 2^16 paths × 756 steps 21.9 ms (normals 10.2, stepping 11.6, the FP64 pipe 83%
+// busy in both) against 77.2 ms in one kernel; 2 assets local vol, 30,000 paths × 501 steps of the
+// pseudo-random lane 6.3 against 11.1 ms; a replay of 4096 Owen-scrambled paths 2.4 against 13.8 ms.
+// Compiled with -fmad=false: products and sums round separately, as in the reference.
+#include <algorithm>
+
+#include "rg_fp64.cuh"
+#include "rg_internal.h"
+
+namespace rg {
+
+namespace {
+
+constexpr int kNormPaths = 256;                                            // paths (threads) per CTA
+__host__ __device__ constexpr int norm_nodes(int n) { return n <= 3 ? 4 : 2; }  // nodes per CTA
+
+template <int N>
+__global__ void __launch_bounds__(kNormPaths) normals64_kernel(DevTrade tr, DevTables tb,
+                                                               const DevScenario* __restrict__ scen, uint64_t path0,
+                                                               uint64_t npaths, uint64_t stride, int path_blocks,
+                                                               double* __restrict__ y) {
+  constexpr int KN = norm_nodes(N);
+  __shared__ double zs[KN * N][kNormPaths];
+  __shared__ uint16_t queue[KN * N * kNormPaths];
+  __shared__ int queued;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint64_t p = (uint64_t)(blockIdx.x % path_blocks) * kNormPaths + tid;
+  const int c0 = (int)(blockIdx.x / path_blocks) * KN, nn = min(KN, (int)tr.steps - c0);
+  if (tid == 0) queued = 0;
+  __syncthreads();
+  if (tr.vr == RG_VR_SOBOL) {
+    const uint64_t n1 = path0 + p - lane + 1;  // Sobol point of the warp's first path
+#pragma unroll
+    for (int j = 0; j < KN * N; ++j) {
+      if (j >= nn * N) break;
+      const int i = c0 * N + j;
+      const uint32_t g = rg_warp_sobol(tb.sobol + 32 * (size_t)__ldg(tb.nf_row + i), n1, lane);
+      const uint32_t x = tr.scrambler == RG_SCRAMBLE_DIGITAL_SHIFT
+                             ? g ^ __ldg(tb.nf_shift + i)
+                             : rg_owen(g, (uint64_t)__ldg(tb.node_k + c0 + j / N) * N + j % N, tr.seed);
+      if (probit64_is_tail(x)) {
+        zs[j][tid] = __longlong_as_double((long long)x);
+        queue[atomicAdd(&queued, 1)] = (uint16_t)(j * kNormPaths + tid);
+      } else {
+        zs[j][tid] = probit64_central(x);
+      }
+    }
+    __syncthreads();
+    for (int q = tid; q < queued; q += kNormPaths) {
+      double& z = (&zs[0][0])[queue[q]];
+      z = probit64_tail((uint32_t)__double_as_longlong(z));
+    }
+    __syncthreads();
+  } else {
+    for (int j = 0; j < nn * N; ++j)
+      zs[j][tid] = rg_qmc_normal64(tr, tb, path0 + p, (uint64_t)__ldg(tb.node_k + c0 + j / N) * N + j % N);
+  }
+  if (p >= npaths) return;
+  const DevScenario& sc = scen[0];
+  for (int j = 0; j < nn; ++j) {
+    // Cholesky::apply_into (correlation.rs:196-206)
+    double z[N];
+#pragma unroll
+    for (int f = 0; f < N; ++f) z[f] = zs[j * N + f][tid];
+#pragma unroll
+    for (int a = 0; a < N; ++a) {
+      double s = sc.L[a * N] * z[0];
+#pragma unroll
+      for (int b = 1; b <= a; ++b) s += sc.L[a * N + b] * z[b];
+      y[((uint64_t)(c0 + j) * N + a) * stride + p] = s;
+    }
+  }
+}
+
+// The pseudo-random lane (note.rs:123-127): y = L·z of the stream's draws z[path][step][asset], read
+// along a path's row and written along paths.
+constexpr int kCorPaths = 32, kCorSteps = 16;
+template <int N>
+__global__ void __launch_bounds__(kCorPaths * 8) correlate64_kernel(const DevScenario* __restrict__ scen,
+                                                                   const double* __restrict__ z, int64_t T,
+                                                                   uint64_t npaths, uint64_t stride, int path_blocks,
+                                                                   double* __restrict__ y) {
+  __shared__ double zs[kCorPaths][kCorSteps * N + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t p0 = (uint64_t)(blockIdx.x % path_blocks) * kCorPaths;
+  const int64_t t0 = (int64_t)(blockIdx.x / path_blocks) * kCorSteps;
+  const int nt = (int)min((int64_t)kCorSteps, T - t0);
+  for (int r = warp; r < kCorPaths; r += 8)
+    if (p0 + r < npaths)
+      for (int i = lane; i < nt * N; i += 32) zs[r][i] = z[((p0 + r) * (uint64_t)T + t0) * N + i];
+  __syncthreads();
+  const uint64_t p = p0 + lane;
+  if (p >= npaths) return;
+  const DevScenario& sc = scen[0];
+  for (int j = warp; j < nt; j += 8)
+#pragma unroll
+    for (int a = 0; a < N; ++a) {
+      double s = sc.L[a * N] * zs[lane][j * N];
+#pragma unroll
+      for (int b = 1; b <= a; ++b) s += sc.L[a * N + b] * zs[lane][j * N + b];
+      y[((uint64_t)(t0 + j) * N + a) * stride + p] = s;
+    }
+}
+
+// Per surface, the widths of the log-strike axis's cells and their reciprocals (rounded).
+__global__ void axis64_kernel(const double* __restrict__ logs, int gx, int n, double2* __restrict__ axis) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double d = i % gx + 1 < gx ? logs[i + 1] - logs[i] : 1.0;
+  axis[i] = make_double2(d, 1.0 / d);
+}
+
+// DupireLocalVol::sigma (riga-market/src/lib.rs:305-343) at a step's tenor rows.
+__device__ __forceinline__ double sigma64(const double* __restrict__ v, const double* __restrict__ ls,
+                                          const double2* __restrict__ axis, int gx, float l0, float inv, int2 ti,
+                                          double wt, double spot) {
+  // max(spot, 1e-12); the logarithm's fast form takes positive normals
+  const uint32_t h = (uint32_t)hi_word(spot);
+  const double x = h - 0x3d719800u < 0x7ff00000u - 0x3d719800u ? fast_log64(spot) : general_log64(spot > 1e-12 ? spot : 1e-12);
+  const long long kx = order_key(x);
+  int lo, hi;
+  double wx = 0.0;
+  if (kx <= order_key(__ldg(ls))) {
+    lo = hi = 0;
+  } else if (!(kx < order_key(__ldg(ls + gx - 1)))) {
+    lo = hi = gx - 1;
+  } else {
+    // first j with x <= ls[j+1], from an estimate on the uniform axis
+    int j = (int)(((float)x - l0) * inv);
+    j = j < 0 ? 0 : (j > gx - 2 ? gx - 2 : j);
+    while (j > 0 && kx <= order_key(__ldg(ls + j))) --j;
+    while (j + 1 < gx - 1 && kx > order_key(__ldg(ls + j + 1))) ++j;
+    lo = j;
+    hi = j + 1;
+    const double2 a = __ldg(axis + j);
+    wx = divide_by(x - __ldg(ls + j), a.x, a.y);
+  }
+  const double ox = 1.0 - wx;
+  const double v0 = ox * __ldg(v + ti.x * gx + lo) + wx * __ldg(v + ti.x * gx + hi);
+  const double v1 = ox * __ldg(v + ti.y * gx + lo) + wx * __ldg(v + ti.y * gx + hi);
+  return (1.0 - wt) * v0 + wt * v1;
+}
+
+constexpr int kStepWarps = 2;
+
+struct Step64Args {
+  DevTrade tr;
+  DevTables tb;
+  const DevScenario* scen;
+  const double* y;      // [node or step][asset][stride]
+  const double2* axis;  // [surface][gx]
+  uint64_t stride, path0, first, npaths;  // global index of path 0; the chunk's first path; its paths
+  double* partial;      // row of the chunk's first CTA
+  int32_t* ko_steps;
+  rg_path_record* records;
+  float* cube;
+};
+
+template <int N, bool LV, bool MC>
+__global__ void __launch_bounds__(32 * kStepWarps) step64_kernel(const __grid_constant__ Step64Args A) {
+  constexpr int G = 32 / N;  // paths per warp, a lane per asset
+  extern __shared__ double stk_mem[];  // [depth][thread] bridge anchors
+  __shared__ double red[kStepWarps * G][RG_ACC];
+  const DevTrade& tr = A.tr;
+  const DevTables& tb = A.tb;
+  const DevScenario& sc = A.scen[0];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = min(lane / N, G - 1), f = lane < G * N ? lane % N : 0;
+  const uint32_t mates = ((1u << N) - 1u) << (g * N);  // this path's lanes
+  const int slot = warp * G + g;                      // path within the CTA
+  const uint64_t p = (uint64_t)blockIdx.x * (kStepWarps * G) + slot;
+  const bool live = lane < G * N && p < A.npaths;
+  const uint64_t pl = min(p, A.npaths - 1);  // idle lanes follow the last path
+  const int64_t T = tr.steps;
+  const double init = tr.init[f], dt = tr.dt, sqrt_dt = tr.sqrt_dt, inv_sqrt_dt = tr.inv_sqrt_dt;
+  const double rq = sc.rate - sc.q[f], vol = sc.vols[f];
+  const double flat_drift = (rq - 0.5 * vol * vol) * dt, flat_vs = vol * sqrt_dt;
+  const long long cb_at = __double_as_longlong(tr.cb_spot[f]), ko_at = __double_as_longlong(tr.ko_spot[f]);
+  const double* v = LV ? tb.lv_v + sc.surf_off[f] : nullptr;
+  const double* ls = LV ? tb.lv_logs + sc.surf[f] * tr.gx : nullptr;
+  const double2* axis = LV ? A.axis + sc.surf[f] * tr.gx : nullptr;
+  float l0 = 0.0f, inv = 0.0f;
+  if (LV) {
+    l0 = (float)ls[0];
+    inv = (float)(tr.gx - 1) / (float)(ls[tr.gx - 1] - ls[0]);
+  }
+  const int2* ti = tb.lv_ti + f * T;
+  const double* tw = tb.lv_tw + f * T;
+  const double* yp = A.y + f * A.stride + pl;  // this lane's value of node c at yp[c·N·stride]
+  const uint64_t ystep = (uint64_t)N * A.stride;
+  float* cube = A.cube ? A.cube + (A.first + pl) * (uint64_t)T * N + f : nullptr;
+  double* stk = stk_mem + tid;
+  double spot = sc.spots[f], wcur = 0.0, top = 0.0;
+  int sp = 0, c = 0;
+  int qual = 0, ko_step = -1, qualified = 0, paid = 0;
+  bool ko = false, received = false;
+  double unpaid = 0.0, cpv = 0.0, mpv = 0.0;
+  double ynext = __ldg(yp);
+  for (int64_t t = 0; t < T; ++t) {
+    double shock;
+    if (MC) {
+      shock = ynext;
+      if (t + 1 < T) ynext = __ldg(yp + (uint64_t)(t + 1) * ystep);
+    } else {
+      // bridge nodes consumed at this step (note.rs:89-105 and qmc.rs:158-191)
+      const int c1 = __ldg(tb.node_off + t + 1);
+      for (; c < c1; ++c) {
+        const double yc = ynext * __ldg(tb.node_c + c);
+        if (c + 1 < (int)T) ynext = __ldg(yp + (uint64_t)(c + 1) * ystep);
+        top = c == 0 ? yc : halve(wcur + top) + yc;
+        stk[sp * (32 * kStepWarps)] = top;
+        ++sp;
+      }
+      --sp;
+      shock = (top - wcur) * inv_sqrt_dt;
+      wcur = top;
+      if (sp > 0) top = stk[(sp - 1) * (32 * kStepWarps)];
+    }
+    // GBM / Dupire step (note.rs:133-142)
+    if (LV) {
+      const double s = sigma64(v, ls, axis, tr.gx, l0, inv, __ldg(ti + t), __ldg(tw + t), spot);
+      spot *= fast_exp64((rq - halve(s) * s) * dt + s * sqrt_dt * shock);
+    } else {
+      spot *= fast_exp64(flat_drift + flat_vs * shock);
+    }
+    if (cube && live) cube[(uint64_t)t * N] = (float)spot;
+    // Phoenix state machine (note.rs:150-218)
+    const uint32_t fl = __ldg(tb.step_flags + t);
+    const long long sb = __double_as_longlong(spot);
+    bool above, up;
+    if (__any_sync(0xffffffffu, (uint32_t)(sb >> 32) >= 0x7ff00000u)) {
+      // an infinite or NaN spot in the warp: the ratios as they are
+      const double ratio = spot / init;
+      double worst = __shfl_sync(0xffffffffu, ratio, g * N);
+#pragma unroll
+      for (int a = 1; a < N; ++a) worst = fmin(worst, __shfl_sync(0xffffffffu, ratio, g * N + a));
+      above = worst >= tr.coupon_barrier;
+      up = (__ballot_sync(0xffffffffu, ratio >= tr.call_barrier) & mates) == mates;
+    } else {
+      above = (__ballot_sync(0xffffffffu, sb >= cb_at) & mates) == mates;
+      up = (__ballot_sync(0xffffffffu, sb >= ko_at) & mates) == mates;
+    }
+    if (ko) continue;
+    if (fl & STEP_PERIOD_RESET) qual = 0;
+    if ((fl & STEP_ACCRUE) && above) {
+      ++qual;
+      ++qualified;
+    }
+    auto due_now = [&] {
+      return (fl & STEP_FIXED_DUE) ? tr.coupon_rate : __ldg(tb.accr_sum + __ldg(tb.accr_at + __ldg(tb.step_period + t)) + qual);
+    };
+    if ((fl & STEP_CALL_ACTIVE) && up) {
+      ko = true;
+      ko_step = (int)t;
+      const double due = due_now();
+      const double carry = due > 0.0 ? unpaid : 0.0;
+      if (due + carry > 0.0) {
+        const double df = __ldg(tb.df + t);
+        cpv += due * df;
+        mpv += carry * df;
+        received = true;
+        ++paid;
+      }
+      continue;
+    }
+    if (fl & STEP_PERIOD_END) {
+      const double due = due_now();
+      if (due > 0.0) {
+        const double df = __ldg(tb.df + t);
+        cpv += due * df;
+        mpv += unpaid * df;
+        received = true;
+        unpaid = 0.0;
+        ++paid;
+      } else if (tr.memory) {
+        unpaid += tr.coupon_rate;
+      }
+    }
+  }
+  // path close (note.rs:221-258) on the path's first lane
+  const double ratio = spot / init;
+  double worst = __shfl_sync(0xffffffffu, ratio, g * N);
+#pragma unroll
+  for (int a = 1; a < N; ++a) worst = fmin(worst, __shfl_sync(0xffffffffu, ratio, g * N + a));
+  if (lane < G * N && f == 0) {
+    double out[RG_ACC];
+#pragma unroll
+    for (int k = 0; k < RG_ACC; ++k) out[k] = 0.0;
+    if (live) {
+      const double dfm = __ldg(tb.df_mat);
+      const double funding = ko ? __ldg(tb.df + ko_step) : dfm;
+      const bool hit_ki = worst <= tr.ki, put_ok = hit_ki && !ko;
+      const double put = put_ok ? fmax(tr.strike - worst, 0.0) * dfm : 0.0;
+      const double cn = cpv + mpv;
+      const double pv = funding + cn - put;
+      out[ACC_PV] = pv - 1.0;
+      out[ACC_PV2] = (pv - 1.0) * (pv - 1.0);
+      if (ko) {
+        out[ACC_KOF] = funding - 1.0;
+        out[ACC_KOF2] = (funding - 1.0) * (funding - 1.0);
+        out[ACC_NKO] = 1.0;
+      }
+      if (hit_ki) {
+        out[ACC_KIPUT] = put;
+        out[ACC_KIPUT2] = put * put;
+        out[ACC_NKI] = 1.0;
+      }
+      if (received) {
+        out[ACC_CPN] = cn;
+        out[ACC_CPN2] = cn * cn;
+        out[ACC_NCPN] = 1.0;
+      }
+      out[ACC_PUT] = put;
+      out[ACC_FUND] = funding;
+      out[ACC_CQ] = cn * 10.0 - mpv * 10.0;
+      out[ACC_MQ] = mpv * 10.0;
+      out[ACC_NPUT] = put_ok ? 1.0 : 0.0;
+      const uint64_t i = A.first + p;
+      if (A.ko_steps) A.ko_steps[i] = ko_step;
+      if (A.records) {
+        rg_path_record r;
+        r.path_id = A.path0 + i;
+        r.rng_seed = tr.seed;
+        r.sobol_index = MC ? 0 : A.path0 + i + 1;
+        r.worst_final = worst;
+        r.knocked_out = ko;
+        r.ko_step = ko_step;
+        r.ko_time = ko ? (double)(ko_step + 1) * dt : __longlong_as_double(0x7ff8000000000000LL);
+        r.ki_hit = hit_ki;
+        r.qualified_steps = qualified;
+        r.paid_periods = paid;
+        r.put_payoff = put;
+        r.coupon_pv = cn;
+        r.memory_coupon_pv = mpv;
+        r.funding = funding;
+        r.pv = pv;
+        A.records[i] = r;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < RG_ACC; ++k) red[slot][k] = out[k];
+  }
+  __syncthreads();
+  if (tid < RG_ACC) {
+    double s = 0.0;
+    for (int i = 0; i < kStepWarps * G; ++i) s += red[i][tid];
+    A.partial[(size_t)blockIdx.x * RG_ACC + tid] = s;
+  }
+}
+
+// Paths of one step64 CTA.
+uint64_t cta_paths(int n) { return (uint64_t)kStepWarps * (32 / n); }
+
+// Paths per chunk, in whole CTAs: chunks about equal, their correlated normals within a GiB each.
+uint64_t chunk_of(int n, int64_t T, uint64_t npaths) {
+  const uint64_t unit = cta_paths(n), fit = (uint64_t(1) << 30) / ((uint64_t)T * n * sizeof(double));
+  const uint64_t cap = std::max<uint64_t>(fit / unit, 1), ctas = (npaths + unit - 1) / unit;
+  const uint64_t chunks = (ctas + cap - 1) / cap;
+  return (ctas + chunks - 1) / chunks * unit;
+}
+
+template <int N>
+void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen, uint64_t path0, uint64_t npaths,
+         const LaunchOut& out, cudaStream_t st) {
+  const int64_t T = P.T;
+  const bool lv = P.trade.has_lv != 0;
+  const uint64_t chunk = chunk_of(N, T, npaths);
+  const size_t axis_bytes = lv ? (size_t)P.n_surf * P.trade.gx * sizeof(double2) : 0;
+  uint8_t* buf = static_cast<uint8_t*>(W.device(WS_NORMALS64, axis_bytes + chunk * (uint64_t)T * N * sizeof(double)));
+  double* y = reinterpret_cast<double*>(buf + axis_bytes);
+  Step64Args a{P.trade, tb, scen, y, reinterpret_cast<const double2*>(buf), chunk, path0, 0, 0, out.partial,
+               out.ko_steps, out.records, out.cube};
+  if (lv) {
+    const int n = P.n_surf * P.trade.gx;
+    axis64_kernel<<<(n + 127) / 128, 128, 0, st>>>(tb.lv_logs, P.trade.gx, n, reinterpret_cast<double2*>(buf));
+    cuda_check(cudaGetLastError(), "axis64_kernel launch");
+  }
+  const size_t smem = out.mcz ? 0 : (size_t)P.stack_max * 32 * kStepWarps * sizeof(double);
+  for (a.first = 0; a.first < npaths; a.first += chunk) {
+    a.npaths = std::min(chunk, npaths - a.first);
+    if (out.mcz) {
+      const int pb = (int)((a.npaths + kCorPaths - 1) / kCorPaths);
+      const int64_t tb_n = (T + kCorSteps - 1) / kCorSteps;
+      correlate64_kernel<N><<<(unsigned)(pb * tb_n), kCorPaths * 8, 0, st>>>(
+          scen, out.mcz + a.first * (uint64_t)T * N, T, a.npaths, chunk, pb, y);
+    } else {
+      const int pb = (int)((a.npaths + kNormPaths - 1) / kNormPaths);
+      const int64_t nb = (T + norm_nodes(N) - 1) / norm_nodes(N);
+      normals64_kernel<N><<<(unsigned)(pb * nb), kNormPaths, 0, st>>>(P.trade, tb, scen, path0 + a.first, a.npaths,
+                                                                      chunk, pb, y);
+    }
+    cuda_check(cudaGetLastError(), "normals64 launch");
+    const unsigned blocks = (unsigned)((a.npaths + cta_paths(N) - 1) / cta_paths(N));
+    if (lv) {
+      if (out.mcz) step64_kernel<N, true, true><<<blocks, 32 * kStepWarps, smem, st>>>(a);
+      else step64_kernel<N, true, false><<<blocks, 32 * kStepWarps, smem, st>>>(a);
+    } else {
+      if (out.mcz) step64_kernel<N, false, true><<<blocks, 32 * kStepWarps, smem, st>>>(a);
+      else step64_kernel<N, false, false><<<blocks, 32 * kStepWarps, smem, st>>>(a);
+    }
+    cuda_check(cudaGetLastError(), "step64_kernel launch");
+    a.partial += (size_t)blocks * RG_ACC;
+  }
+}
+
+}  // namespace
+
+uint64_t path64_rows(int n, uint64_t npaths) { return (npaths + cta_paths(n) - 1) / cta_paths(n); }
+
+size_t path64_bytes(int n, int64_t T, uint64_t npaths) {
+  return (size_t)(chunk_of(n, T, npaths) * (uint64_t)T * n * sizeof(double));
+}
+
+void launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen, uint64_t path0,
+                   uint64_t npaths, const LaunchOut& out, cudaStream_t st) {
+  switch (P.n) {
+    case 1: run<1>(W, P, tb, scen, path0, npaths, out, st); break;
+    case 2: run<2>(W, P, tb, scen, path0, npaths, out, st); break;
+    case 3: run<3>(W, P, tb, scen, path0, npaths, out, st); break;
+    case 4: run<4>(W, P, tb, scen, path0, npaths, out, st); break;
+    case 5: run<5>(W, P, tb, scen, path0, npaths, out, st); break;
+    default: raise(RG_ERR_INVALID_MARKET_SHAPE, "unsupported asset count");
+  }
+}
+
+}  // namespace rg

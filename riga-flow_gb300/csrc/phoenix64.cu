@@ -1,9 +1,10 @@
-// phoenix64.cu — the FP64 parity kernel: generation + bridge + step + payoff fused per path.
+// phoenix64.cu — the FP64 parity kernel of the static entry point: generation + bridge + step + payoff
+// fused per path, with no buffer beyond its partial sums (engines run path64.cu's kernels, three to
+// four times faster, which pass a chunk's normals through device memory; same bits per path).
 //
 // One thread prices one path of one scenario in the reference's own operation order
 // (crates/riga-engine/src/note.rs:81-259): QMC normals per step, y = L·z, the depth-first
-// Brownian bridge of each factor (or, in the pseudo-random lane, the path's slice of the ChaCha8
-// normal stream and y = L·z with no bridge, note.rs:123-127), the multiplicative GBM/Dupire step, the Phoenix state machine
+// Brownian bridge of each factor, the multiplicative GBM/Dupire step, the Phoenix state machine
 // and the path close.  The bridge is streamed: an in-order traversal of the bisection tree needs
 // only the current point and a stack of right anchors, so no per-path O(T) buffer exists.  The
 // node schedule (which preorder index and standard deviation each step consumes) is a host table
@@ -39,15 +40,12 @@ __device__ __forceinline__ double lv_sigma64(const double* __restrict__ v, const
   return (1.0 - wt) * v0 + wt * v1;
 }
 
-template <int N, bool LV, bool MC>
+template <int N, bool LV>
 __global__ void __launch_bounds__(128) phoenix64_kernel(DevTrade tr, DevTables tb,
                                                         const DevScenario* __restrict__ scen,
                                                         uint64_t path0, uint64_t npaths,
                                                         double* __restrict__ partial,
-                                                        int32_t* __restrict__ ko_steps,
-                                                        rg_path_record* __restrict__ records,
-                                                        const double* __restrict__ mcz,
-                                                        float* __restrict__ cube) {
+                                                        int32_t* __restrict__ ko_steps) {
   __shared__ double red[128][RG_ACC + 1];
   __shared__ double acc_blk[RG_ACC];
   const int tid = threadIdx.x;
@@ -83,24 +81,11 @@ __global__ void __launch_bounds__(128) phoenix64_kernel(DevTrade tr, DevTables t
         wcur[f] = 0.0;
       }
       int sp = 0;
-      int ko = 0, received = 0, ko_step = -1, qualified = 0, paid = 0;
+      int ko = 0, received = 0, ko_step = -1;
       double accrual = 0.0, unpaid = 0.0, cpv = 0.0, mpv = 0.0, final_worst = 1.0;
       for (int64_t t = 0; t < T; ++t) {
         double shock[N];
-        if (MC) {
-          // pseudo-random lane (note.rs:123-127): n draws of the sequential stream, then L·z
-          const double* zp = mcz + (i * (uint64_t)T + (uint64_t)t) * N;
-          double z[N];
-#pragma unroll
-          for (int f = 0; f < N; ++f) z[f] = zp[f];
-#pragma unroll
-          for (int a = 0; a < N; ++a) {
-            double s = 0.0;
-#pragma unroll
-            for (int b = 0; b <= a; ++b) s += L[a * N + b] * z[b];
-            shock[a] = s;
-          }
-        } else {
+        {
           // bridge nodes consumed at this step (note.rs:89-105 and qmc.rs:158-191)
           const int c0 = __ldg(tb.node_off + t), c1 = __ldg(tb.node_off + t + 1);
           for (int c = c0; c < c1; ++c) {
@@ -151,11 +136,6 @@ __global__ void __launch_bounds__(128) phoenix64_kernel(DevTrade tr, DevTables t
           double drift = (rate - qd[f] - 0.5 * v * v) * dt;
           spots[f] *= rg_exp64(drift + v * sqrt_dt * shock[f]);
         }
-        if (cube) {  // PathCube slice: the spots this step leaves (pathcube.rs:19-35 layout)
-          float* cp = cube + (i * (uint64_t)T + (uint64_t)t) * N;
-#pragma unroll
-          for (int f = 0; f < N; ++f) cp[f] = (float)spots[f];
-        }
         double worst = spots[0] / tr.init[0];
 #pragma unroll
         for (int f = 1; f < N; ++f) worst = fmin(worst, spots[f] / tr.init[f]);
@@ -167,7 +147,6 @@ __global__ void __launch_bounds__(128) phoenix64_kernel(DevTrade tr, DevTables t
         if (fl & STEP_PERIOD_RESET) accrual = 0.0;
         if ((fl & STEP_ACCRUE) && worst >= tr.coupon_barrier) {
           accrual += __ldg(tb.accr_inc + per);
-          ++qualified;
         }
         bool up = (fl & STEP_CALL_ACTIVE) != 0;
 #pragma unroll
@@ -182,7 +161,6 @@ __global__ void __launch_bounds__(128) phoenix64_kernel(DevTrade tr, DevTables t
             cpv += due * df;
             mpv += carry * df;
             received = 1;
-            ++paid;
           }
           continue;
         }
@@ -194,7 +172,6 @@ __global__ void __launch_bounds__(128) phoenix64_kernel(DevTrade tr, DevTables t
             mpv += unpaid * df;
             received = 1;
             unpaid = 0.0;
-            ++paid;
           } else if (tr.memory) {
             unpaid += tr.coupon_rate;
           }
@@ -231,25 +208,6 @@ __global__ void __launch_bounds__(128) phoenix64_kernel(DevTrade tr, DevTables t
       out[ACC_MQ] = mpv * 10.0;
       out[ACC_NPUT] = put_ok ? 1.0 : 0.0;
       if (ko_steps) ko_steps[i] = ko_step;
-      if (records) {
-        rg_path_record r;
-        r.path_id = path;
-        r.rng_seed = tr.seed;
-        r.sobol_index = MC ? 0 : path + 1;
-        r.worst_final = final_worst;
-        r.knocked_out = ko;
-        r.ko_step = ko_step;
-        r.ko_time = ko ? (double)(ko_step + 1) * dt : __longlong_as_double(0x7ff8000000000000LL);
-        r.ki_hit = hit_ki;
-        r.qualified_steps = qualified;
-        r.paid_periods = paid;
-        r.put_payoff = put;
-        r.coupon_pv = cn;
-        r.memory_coupon_pv = mpv;
-        r.funding = funding;
-        r.pv = pv;
-        records[i] = r;
-      }
     }
     // fixed-order block reduction of this round
 #pragma unroll
@@ -266,8 +224,7 @@ __global__ void __launch_bounds__(128) phoenix64_kernel(DevTrade tr, DevTables t
   if (tid < RG_ACC) partial[(size_t)blockIdx.x * RG_ACC + tid] = acc_blk[tid];
 }
 
-int phoenix64_grid(const Prepared& P, uint64_t npaths) {
-  (void)P;
+int phoenix64_grid(uint64_t npaths) {
   uint64_t blocks = (npaths + 127) / 128;
   const uint64_t cap = 152 * 16;  // a few rounds of resident CTAs on 152 SMs
   return (int)(blocks < cap ? blocks : cap);
@@ -276,14 +233,7 @@ int phoenix64_grid(const Prepared& P, uint64_t npaths) {
 template <int N, bool LV>
 static void launch_n(const Prepared& P, const DevTables& tb, const DevScenario* scen, uint64_t path0,
                      uint64_t npaths, const LaunchOut& out, cudaStream_t s) {
-  if (out.mcz)
-    phoenix64_kernel<N, LV, true><<<out.grid, 128, 0, s>>>(P.trade, tb, scen, path0, npaths, out.partial,
-                                                           out.ko_steps, out.records, out.mcz,
-                                                           out.cube);
-  else
-    phoenix64_kernel<N, LV, false><<<out.grid, 128, 0, s>>>(P.trade, tb, scen, path0, npaths, out.partial,
-                                                            out.ko_steps, out.records, nullptr,
-                                                            out.cube);
+  phoenix64_kernel<N, LV><<<out.grid, 128, 0, s>>>(P.trade, tb, scen, path0, npaths, out.partial, out.ko_steps);
 }
 
 void launch_phoenix64(const Prepared& P, const DevTables& tb, const DevScenario* scen,

@@ -45,6 +45,8 @@ struct DevTrade {
   double dt, sqrt_dt, inv_sqrt_dt, maturity;
   double init[RG_NMAX];
   double call_barrier, coupon_barrier, coupon_rate, strike, ki;
+  // the smallest spot of each asset whose ratio to its initial spot, rounded, reaches the barrier
+  double cb_spot[RG_NMAX], ko_spot[RG_NMAX];
   float coupon_f, strike_f;  // coupon_rate and strike rounded to FP32 for the FP32 kernels
   float neg_half_dt_f;       // -dt / 2 rounded to FP32 (the FP32 kernels' Euler drift term)
   int32_t memory;
@@ -68,6 +70,8 @@ struct DevTables {
   const uint32_t* step_flags;  // [T]
   const int32_t* step_period;  // [T]
   const double* accr_inc;      // [periods] coupon_rate / period_steps
+  const double* accr_sum;      // accr_inc[q] added k times, at accr_at[q] + k (k up to the period's steps)
+  const int32_t* accr_at;      // [periods]
   const int32_t* node_off;     // [T+1] first bridge node consumed at step t
   const int32_t* node_k;       // [T] preorder index (QMC step) of each node, consumption order
   const double* node_c;        // [T] bridge standard deviation of each node

@@ -100,6 +100,8 @@ struct Prepared {
   std::vector<uint32_t> step_flags;
   std::vector<int32_t> step_period;
   std::vector<double> accr_inc;
+  std::vector<double> accr_sum;  // DevTables::accr_sum, accr_at
+  std::vector<int32_t> accr_at;
   std::vector<float> accr_f;  // accr_inc in FP32 (the FP32 kernels read no FP64 per step)
   std::vector<int32_t> node_off, node_k;
   std::vector<double> node_c;
@@ -128,6 +130,7 @@ enum WsSlot {
   WS_ARENA = 0, WS_CALIB, WS_LVROWS, WS_PARTIAL, WS_SUMS, WS_KOSTEPS, WS_RECORDS,
   WS_MCZ, WS_MCKEYS, WS_MCAUX,  // the pseudo-random lane's normals, keystream and parse tables
   WS_CUBE,                      // f32 spot cube of a materialised path range
+  WS_NORMALS64,                 // correlated normals of a chunk of the FP64 lane's paths
   WS_NSLOTS
 };
 struct SurfaceCache;
@@ -241,7 +244,14 @@ struct LaunchOut {
 };
 // StandardNormal draws [first, first + count) of ChaCha8Rng::seed_from_u64(seed) into d_out.
 void mc_normals(uint64_t seed, uint64_t first, uint64_t count, double* d_out, Workspace& W);
-int phoenix64_grid(const Prepared& P, uint64_t npaths);
+// The FP64 lane through a workspace that keeps its buffers (path64.cu): rows of partial sums for an
+// asset count, device bytes of its chunk buffer, and the launch.
+uint64_t path64_rows(int n, uint64_t npaths);
+size_t path64_bytes(int n, int64_t T, uint64_t npaths);
+void launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen_dev, uint64_t path0,
+                   uint64_t npaths, const LaunchOut& out, cudaStream_t s);
+// The same in one kernel and no buffer, for the static entry point (phoenix64.cu).
+int phoenix64_grid(uint64_t npaths);
 void launch_phoenix64(const Prepared& P, const DevTables& tb, const DevScenario* scen_dev,
                       uint64_t path0, uint64_t npaths, const LaunchOut& out, cudaStream_t s);
 struct Fp32Shape {

@@ -20,7 +20,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
           "--expt-relaxed-constexpr",
           "-Xptxas", "-warn-spills"]
-NO_FMA = {"phoenix64.cu", "prologue.cu", "book64.cu", "mclane.cu"}
+NO_FMA = {"phoenix64.cu", "path64.cu", "prologue.cu", "book64.cu", "mclane.cu"}
 # RG_PHASE_CLOCKS=1 builds the tiled FP32 kernel with per-phase clock counters (rg_phase_clocks)
 PHASE_CLOCKS = os.environ.get("RG_PHASE_CLOCKS", "0") not in ("", "0")
 

@@ -1,0 +1,95 @@
+"""The FP64 lane's kernels of an engine against the one-kernel form of the static entry point.
+
+Both run the reference's arithmetic product by product, one path at a time, so every event count is
+equal and the path sums differ only by the order of the FP64 additions over paths: at most `paths`
+roundings of 2^-53 on sums of terms below 10 (coupon quotes are on the x10 scale).
+"""
+from __future__ import annotations
+
+import ctypes as C
+
+import pytest
+
+from riga_gb300 import abi, workloads
+from riga_gb300.build import build_library
+from riga_gb300.engine import Engine
+from riga_gb300.types import VarianceReduction
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engine():
+    build_library()
+    e = Engine(0)
+    yield e
+    e.close()
+
+
+def _request(n, paths, steps, smile=None, lane="shift", **terms):
+    if smile:
+        req = workloads.lv3(paths, steps, fp32=False)
+        req.local_vol, _ = workloads.svi_grids(n, seed=n, n_k=smile[0], n_t=smile[1], years=steps / 252)
+        req.options.lv_grid_x = smile[2]
+    else:
+        req = workloads.plain3(paths, steps)
+    req.trade = workloads.phoenix_trade(n, steps, steps / 252)
+    m = req.market
+    m.spots, m.vols = [100.0 + f for f in range(n)], [0.18 + 0.05 * f for f in range(n)]
+    m.dividend_yields = [0.01] * n
+    m.correlation = [[1.0 if i == j else 0.45 for j in range(n)] for i in range(n)]
+    if lane == "owen":
+        req.options.scrambler, req.options.dim_mode = abi.SCRAMBLE_OWEN, abi.DIM_WRAP_REFERENCE
+    elif lane.startswith("halton"):
+        req.config.variance_reduction = VarianceReduction("halton", n * steps)
+        if lane == "halton512":
+            req.options.dim_mode = abi.DIM_WRAP_REFERENCE
+    for k, v in terms.items():
+        setattr(req.trade, k, v)
+    return req
+
+
+def _check(engine, req):
+    a = req.to_abi()
+    want = abi.PriceResult()
+    abi.check(engine.lib, engine.lib.rg_price_put_leg_static(a.ptr, C.byref(want)))
+    got = engine.price_raw(req)
+    assert list(got.path_sums)[12:] == list(want.path_sums)[12:]
+    for x, y in zip(list(got.path_sums)[:12], list(want.path_sums)[:12]):
+        assert abs(x - y) <= 10.0 * req.config.paths ** 2 * 2.0 ** -53
+    return got
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("paths,steps", [(1, 1), (31, 2), (257, 63), (1000, 100)])
+@pytest.mark.parametrize("smile", [None, (13, 1, 2), (20, 5, 96)])
+def test_engine_and_static_kernels_agree(engine, n, paths, steps, smile):
+    _check(engine, _request(n, paths, steps, smile))
+
+
+@pytest.mark.parametrize("lane", ["owen", "halton", "halton512"])
+@pytest.mark.parametrize("first", [0, 5, 31, 1000])
+def test_lanes_and_offsets_agree(engine, lane, first):
+    req = _request(3, 300, 40, (13, 3, 40), lane)
+    req.options.first_path = first
+    _check(engine, req)
+
+
+@pytest.mark.parametrize("terms", [
+    dict(coupon_periods=1), dict(coupon_periods=90), dict(coupon_periods=200), dict(fixed_first_coupon=True),
+    dict(knock_out_barrier=None), dict(coupon_barrier=None), dict(memory_coupon=False), dict(call_start_step=0),
+    dict(call_start_step=1000), dict(knock_out_barrier=0.5, call_start_step=0), dict(knock_in_barrier=5.0),
+    dict(coupon_rate=None), dict(coupon_periods=7, fixed_first_coupon=True, call_start_step=3),
+])
+def test_schedules_agree(engine, terms):
+    _check(engine, _request(2, 400, 90, None, **terms))
+
+
+@pytest.mark.parametrize("vol,years", [(0.0, 1.0), (6.0, 30.0), (40.0, 60.0), (1e-9, 1e-6)])
+def test_extreme_paths_agree(engine, vol, years):
+    """Steps beyond the exponential's short range, spots that underflow to zero or overflow, and paths
+    that do not move."""
+    req = _request(3, 128, 30)
+    req.trade.maturity_years = years
+    req.market.vols = [vol] * 3
+    _check(engine, req)
