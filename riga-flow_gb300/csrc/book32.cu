@@ -51,12 +51,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
-// min of three (one instruction from sm_100 on).
-__device__ __forceinline__ float min3(float a, float b, float c) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
 // a >= b as 1.0f or 0.0f.
 __device__ __forceinline__ float ge_one(float a, float b) {
   float d;
@@ -68,12 +62,12 @@ template <int N>
 __device__ __forceinline__ float2 worst_of_n(const float2 (&x)[N]) {
   if constexpr (N == 1) return x[0];
   else if constexpr (N == 2) return make_float2(fminf(x[0].x, x[1].x), fminf(x[0].y, x[1].y));
-  else if constexpr (N == 3) return make_float2(min3(x[0].x, x[1].x, x[2].x), min3(x[0].y, x[1].y, x[2].y));
+  else if constexpr (N == 3) return make_float2(rg_min3(x[0].x, x[1].x, x[2].x), rg_min3(x[0].y, x[1].y, x[2].y));
   else if constexpr (N == 4)
-    return make_float2(min3(fminf(x[0].x, x[1].x), x[2].x, x[3].x), min3(fminf(x[0].y, x[1].y), x[2].y, x[3].y));
+    return make_float2(rg_min3(fminf(x[0].x, x[1].x), x[2].x, x[3].x), rg_min3(fminf(x[0].y, x[1].y), x[2].y, x[3].y));
   else
-    return make_float2(min3(min3(x[0].x, x[1].x, x[2].x), x[3].x, x[4].x),
-                       min3(min3(x[0].y, x[1].y, x[2].y), x[3].y, x[4].y));
+    return make_float2(rg_min3(rg_min3(x[0].x, x[1].x, x[2].x), x[3].x, x[4].x),
+                       rg_min3(rg_min3(x[0].y, x[1].y, x[2].y), x[3].y, x[4].y));
 }
 
 // What a CTA's threads share over the launch.

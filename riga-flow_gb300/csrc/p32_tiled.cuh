@@ -323,10 +323,10 @@ __global__ void __launch_bounds__(PPT == 1 ? 1024 : 512, 1) phoenix32_kernel(
       }
       {
         // kGB items per warp at a time in straight-line code, so that their global loads, shuffles
-        // and inverse normals overlap (three: four spilled registers, measured 0.7% slower); a
-        // warp's surplus slots recompute its last item (the same values stored twice), and items
-        // of paths past the request compute values nobody reads
-        constexpr int kGB = 3;
+        // and inverse normals (packed in pairs over the items' factors) overlap; a warp's surplus
+        // slots recompute its last item (the same values stored twice), and items of paths past the
+        // request compute values nobody reads
+        constexpr int kGB = N == 1 ? 4 : (N == 2 ? 3 : 2);
         const int nitems = nn << lg_ngrp;
         const bool shift_lane = tr.vr == RG_VR_SOBOL && tr.scrambler == RG_SCRAMBLE_DIGITAL_SHIFT;
         for (int base = wid; base < nitems; base += kGB * nwarp) {
@@ -337,37 +337,40 @@ __global__ void __launch_bounds__(PPT == 1 ? 1024 : 512, 1) phoenix32_kernel(
             jj[u] = it >> lg_ngrp;
             hh[u] = it & (ngrp - 1);
           }
+          // the normals of the items' points into their Z rows, two at a time
+          auto store_normals = [&](const uint32_t (&xs)[kGB * N]) {
+#pragma unroll
+            for (int i = 0; i < kGB * N; i += 2) {
+              const float2 z = rg_probit32x2(xs[i], xs[i + 1]);
+              Z[(size_t)jj[i / N] * zs + i % N * (Pb + 4) + (hh[i / N] << 5) + lane] = z.x;
+              Z[(size_t)jj[(i + 1) / N] * zs + (i + 1) % N * (Pb + 4) + (hh[(i + 1) / N] << 5) + lane] = z.y;
+            }
+          };
+          uint32_t xs[kGB * N];
           if (lut_tile) {
             // x = the group's high-bit term (this lane's block) ^ the lane's low-bit term, with the
             // digital shift folded into the low-bit table
-            uint32_t xs[kGB][N];
 #pragma unroll
             for (int u = 0; u < kGB; ++u) {
               const int hb = (hh[u] * 2 + (upper ? 1 : 0)) * hs + jj[u] * N;
               const uint32_t* lt = tb.sob_lut + (size_t)(n0 + jj[u]) * N * 32 + lane;
 #pragma unroll
-              for (int f = 0; f < N; ++f) xs[u][f] = s_hq[hb + f] ^ __ldg(lt + f * 32);
+              for (int f = 0; f < N; ++f) xs[u * N + f] = s_hq[hb + f] ^ __ldg(lt + f * 32);
             }
+            if (!shift_lane)
 #pragma unroll
-            for (int u = 0; u < kGB; ++u)
-#pragma unroll
-              for (int f = 0; f < N; ++f)
-                Z[(size_t)jj[u] * zs + f * (Pb + 4) + (hh[u] << 5) + lane] =
-                    rg_probit32(shift_lane ? xs[u][f] : rg_owen(xs[u][f], (uint64_t)s_nodek[jj[u]] * N + f, tr.seed));
+              for (int i = 0; i < kGB * N; ++i)
+                xs[i] = rg_owen(xs[i], (uint64_t)s_nodek[jj[i / N]] * N + i % N, tr.seed);
+            store_normals(xs);
           } else if (shift_lane) {
-            uint32_t xs[kGB][N];
 #pragma unroll
             for (int u = 0; u < kGB; ++u) {
               const uint64_t n1 = path0 + tile0 + ((uint64_t)hh[u] << 5) + 1;  // Sobol point of lane 0
 #pragma unroll
               for (int f = 0; f < N; ++f)
-                xs[u][f] = rg_warp_sobol(tb.sobol + 32 * (size_t)s_nfrow[jj[u] * N + f], n1, lane) ^ s_nfsh[jj[u] * N + f];
+                xs[u * N + f] = rg_warp_sobol(tb.sobol + 32 * (size_t)s_nfrow[jj[u] * N + f], n1, lane) ^ s_nfsh[jj[u] * N + f];
             }
-#pragma unroll
-            for (int u = 0; u < kGB; ++u)
-#pragma unroll
-              for (int f = 0; f < N; ++f)
-                Z[(size_t)jj[u] * zs + f * (Pb + 4) + (hh[u] << 5) + lane] = rg_probit32(xs[u][f]);
+            store_normals(xs);
           } else {
 #pragma unroll
             for (int u = 0; u < kGB; ++u) {
@@ -480,8 +483,6 @@ __global__ void __launch_bounds__(PPT == 1 ? 1024 : 512, 1) phoenix32_kernel(
             y[a] = acc_y;
           }
 #pragma unroll
-          for (int j = 0; j < PPT; ++j) wmin[j] = INFINITY;
-#pragma unroll
           for (int f = 0; f < N; ++f) {
             V sg;
             if (LV) {
@@ -504,8 +505,14 @@ __global__ void __launch_bounds__(PPT == 1 ? 1024 : 512, 1) phoenix32_kernel(
               sg = sig[f];
             }
             x[f] = V::add(V::fma(sg, V::fma(nhdt, sg, y[f]), x[f]), mu[f]);
+          }
 #pragma unroll
-            for (int j = 0; j < PPT; ++j) wmin[j] = fminf(wmin[j], x[f].v[j]);
+          for (int j = 0; j < PPT; ++j) {
+            wmin[j] = x[0].v[j];
+            if constexpr (N == 2) wmin[j] = fminf(wmin[j], x[1].v[j]);
+            if constexpr (N >= 3) wmin[j] = rg_min3(wmin[j], x[1].v[j], x[2].v[j]);
+            if constexpr (N == 4) wmin[j] = fminf(wmin[j], x[3].v[j]);
+            if constexpr (N == 5) wmin[j] = rg_min3(wmin[j], x[3].v[j], x[4].v[j]);
           }
         };
         // Phoenix state machine (note.rs:150-218) of one step in full: steps that reset or close a

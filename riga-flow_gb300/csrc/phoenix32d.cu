@@ -138,13 +138,21 @@ __global__ void __launch_bounds__(P32D_THREADS, N <= 3 ? 4 : 3) phoenix32d_kerne
             lcur[f] = lnext[f];
             if (more) lnext[f] = __ldg(tb.sob_lut + ((size_t)(c + 1) * N + f) * 32 + lane);
           }
+          uint32_t xs[N];
 #pragma unroll
           for (int f = 0; f < N; ++f) {
-            const uint32_t xs = s_hi[wib][hb + f] ^ lcur[f];
-            zf[f] = rg_probit32(tr.scrambler == RG_SCRAMBLE_DIGITAL_SHIFT
-                                    ? xs
-                                    : rg_owen(xs, (uint64_t)__ldg(tb.node_k + c) * N + f, tr.seed));
+            xs[f] = s_hi[wib][hb + f] ^ lcur[f];
+            if (tr.scrambler != RG_SCRAMBLE_DIGITAL_SHIFT)
+              xs[f] = rg_owen(xs[f], (uint64_t)__ldg(tb.node_k + c) * N + f, tr.seed);
           }
+          // the inverse normals in packed pairs
+#pragma unroll
+          for (int f = 0; f + 1 < N; f += 2) {
+            const float2 z = rg_probit32x2(xs[f], xs[f + 1]);
+            zf[f] = z.x;
+            zf[f + 1] = z.y;
+          }
+          if constexpr (N % 2) zf[N - 1] = rg_probit32(xs[N - 1]);
         } else if (tr.vr == RG_VR_SOBOL) {
 #pragma unroll
           for (int f = 0; f < N; ++f) {
@@ -181,7 +189,6 @@ __global__ void __launch_bounds__(P32D_THREADS, N <= 3 ? 4 : 3) phoenix32d_kerne
         for (int b = 0; b <= a; ++b) acc_y = fmaf(Lf[q++], d[b], acc_y);
         y[a] = acc_y;
       }
-      float wmin = INFINITY;
 #pragma unroll
       for (int f = 0; f < N; ++f) {
         float sg;
@@ -199,8 +206,12 @@ __global__ void __launch_bounds__(P32D_THREADS, N <= 3 ? 4 : 3) phoenix32d_kerne
           sg = sig[f];
         }
         x[f] = fmaf(sg, fmaf(nhdt, sg, y[f]), x[f]) + mu[f];
-        wmin = fminf(wmin, x[f]);
       }
+      float wmin = x[0];
+      if constexpr (N == 2) wmin = fminf(wmin, x[1]);
+      if constexpr (N >= 3) wmin = rg_min3(wmin, x[1], x[2]);
+      if constexpr (N == 4) wmin = fminf(wmin, x[3]);
+      if constexpr (N == 5) wmin = rg_min3(wmin, x[3], x[4]);
       worst = wmin;
       if (ph.alive)  // Phoenix state machine (note.rs:150-218)
         p32_phoenix_step<REC>(ph, __ldg(tb.step_flags + t), t, wmin, ln_cb, ln_ko, tr, tb, tb.df_f + (size_t)s * T,

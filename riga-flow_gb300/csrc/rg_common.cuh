@@ -167,6 +167,13 @@ __device__ __forceinline__ uint32_t rg_warp_sobol(const uint32_t* __restrict__ r
   return d;
 }
 
+// min of three (one instruction from sm_100 on).
+__device__ __forceinline__ float rg_min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 // ------------------------------------------------------------------ inverse normal ------------
 // Acklam's rational approximation (qmc.rs:37-91), FP64, reference operation order.
 __device__ __forceinline__ double rg_probit64(double p) {
@@ -204,6 +211,13 @@ __device__ __forceinline__ double rg_probit64(double p) {
 // sqrt(w) - 3.7161102 beyond.  No division, one fast logarithm, no FP64; within 4e-7 relative of
 // the exact inverse normal, which the reference's Acklam approximation (qmc.rs:37-91) matches to
 // 1.15e-9.
+// -ln(a) for a normal a by the hardware's base-2 logarithm (flush-to-zero form: no scaling of
+// subnormals, three instructions of the general form; the arguments here are at least 2e-12).
+__device__ __forceinline__ float rg_neg_ln(float a) {
+  float l;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(a));
+  return l * -0.6931471805599453f;
+}
 // The tail polynomial, w >= 5.
 __device__ __forceinline__ float rg_ninv32_tail(float w) {
   const float v = sqrtf(w) - 3.716110200f;
@@ -221,7 +235,7 @@ __device__ __forceinline__ float rg_ninv32_tail(float w) {
   return fmaf(g, v, 5.025157229e+00f);
 }
 __device__ __forceinline__ float rg_ninv32_lower(float p2, float s) {
-  const float w = -__logf(fmaf(p2, s, p2));
+  const float w = rg_neg_ln(fmaf(p2, s, p2));
   float g;
   if (w < 5.0f) {
     const float t = w - 2.5f;
@@ -253,22 +267,15 @@ __device__ __forceinline__ float rg_probit32(uint32_t x) {
   return lower ? -q : q;
 }
 
-// rg_probit32 of two points in packed FP32x2 arithmetic, each with rg_probit32's operations; the
-// logarithm's argument is at least 2^-32, so the hardware's flush-to-zero form needs no scaling of
-// subnormals (three instructions of the general form).
+// rg_probit32 of two points in packed FP32x2 arithmetic, each with rg_probit32's operations.
 __device__ __forceinline__ float2 rg_probit32x2(uint32_t xa, uint32_t xb) {
   auto both = [](float a) { return make_float2(a, a); };
-  auto neg_ln = [](float a) {
-    float l;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(a));
-    return l * -0.6931471805599453f;
-  };
   const uint32_t ya = xa ^ (uint32_t)((int32_t)xa >> 31), yb = xb ^ (uint32_t)((int32_t)xb >> 31);  // min(x, ~x)
   const float2 c = both(4.656612873077393e-10f), h = both(2.3283064365386963e-10f);
   const float2 p2 = __ffma2_rn(make_float2((float)(int32_t)ya, (float)(int32_t)yb), c, h);
   const float2 s = __ffma2_rn(make_float2((float)(int32_t)(ya ^ 0x7FFFFFFFu), (float)(int32_t)(yb ^ 0x7FFFFFFFu)), c, h);
   const float2 v = __ffma2_rn(p2, s, p2);
-  const float2 w = make_float2(neg_ln(v.x), neg_ln(v.y));
+  const float2 w = make_float2(rg_neg_ln(v.x), rg_neg_ln(v.y));
   const float2 t = __fadd2_rn(w, both(-2.5f));
   float2 g = both(4.035466097e-08f);
   g = __ffma2_rn(g, t, both(4.861039695e-07f));
