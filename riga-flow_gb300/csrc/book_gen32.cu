@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "rg_internal.h"
+#include "rg_packed.cuh"
 
 namespace rg {
 

@@ -1,6 +1,7 @@
 // p32_path.cuh — the path close shared by the FP32 kernels (phoenix32.cu, phoenix32d.cu).
 #pragma once
 #include "rg_common.cuh"
+#include "rg_packed.cuh"
 
 namespace rg {
 
