@@ -6,13 +6,13 @@
 // The FP32 production kernel: one fused launch prices S common-random-number scenarios of one
 // trade.
 //
-// A CTA owns Pb consecutive paths × Sb scenario slots (Sb = S rounded up to a power of two, at least
-// 4; Pb = 1024 / Sb; a single scenario runs on the direct kernel of phoenix32d.cu).  In the
-// stepping phase a thread serves one scenario and PPT paths: PPT = 2 (512 threads) steps a pair of
-// paths in packed FP32x2 arithmetic (fma/add .f32x2, one instruction for both paths), PPT = 1
-// (1024 threads) one path; a warp is 32·PPT paths of one scenario, so its local-vol lookups all
-// read one surface.  Time is walked in tiles of TT steps, each in three phases separated by CTA
-// barriers:
+// A CTA owns Pb consecutive paths × the S scenarios (large single-scenario launches run on the direct
+// kernel of phoenix32d.cu).  In the stepping phase a thread serves one scenario and PPT paths: PPT = 2
+// steps a pair of paths in packed FP32x2 arithmetic (fma/add .f32x2, one instruction for both paths),
+// PPT = 1 one path; a warp is 32·PPT paths of one scenario (at Pb = 32·PPT or more; else of the
+// Pb-path columns of two), so its local-vol lookups all read one surface.  Threads past the last
+// scenario share generation and bridge only.  Time is walked in tiles of TT steps, each in three
+// phases separated by CTA barriers:
 //   G. generation — warp-wide items (bridge node, 32-path group): the Sobol integers of the group's
 //      32 consecutive points by a warp cooperation (rg_warp_sobol: shuffle reduction of the first
 //      point's Gray code, XOR scan of the Gray recurrence), the digital shift (or Owen scramble) and
@@ -153,8 +153,12 @@ static inline int p32_phase_clocks_tu(unsigned long long out[4], bool reset) {
 #endif
 }
 
+// Threads of the largest CTA: at two paths per thread 512 keep 128 registers each; up to three assets
+// 96 registers do without spilling, so that CTA may have 640.
+__host__ __device__ constexpr int p32_max_threads(int n, int ppt) { return ppt == 1 ? 1024 : (n <= 3 ? 640 : 512); }
+
 template <int N, bool LV, bool REC, int PPT>
-__global__ void __launch_bounds__(PPT == 1 ? 1024 : 512, 1) phoenix32_kernel(
+__global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
     DevTrade tr, DevTables tb, const DevScenario* __restrict__ scen,
     const DevScen32* __restrict__ scen32, int S, int Pb, int TT, int NNmax, int stack_max,
     float ln_ko, float ln_cb, float ln_ki, uint64_t path0, uint64_t npaths, const uint32_t* __restrict__ plan,

@@ -23,15 +23,8 @@ static const void* select_kernel(int n, bool lv, bool rec, int ppt) {
 #undef RG_SEL
 }
 
-// Paths per thread of the formula shape: two (packed FP32x2 stepping, 512 threads) unless the
-// autotuner measured one faster for the launch shape.
-static constexpr int kDefaultPpt = 2;
-
-// Formula tile depth of a block of Pb paths.
-static int formula_tt(const Prepared& P, int Pb) {
-  int tt = (32768 / (Pb * P.n) - P.stack_max) / 2;
-  return tt < 8 ? 8 : (tt > 64 ? 64 : tt);
-}
+// Tile depths a tiled launch may take; each has a bridge plan.
+static const int kTileDepths[] = {24, 32, 48, 64, 80, 96, 128};
 
 // Shared-memory bytes of a tiled shape: Pb paths per tile at `ppt` paths per thread, `tt` steps per
 // tile.
@@ -41,24 +34,38 @@ static uint32_t p32_smem(const Prepared& P, int Pb, int ppt, int tt) {
 // Whether the shape fits in 227 KB of shared memory.
 static bool p32_fits(const Prepared& P, int Pb, int ppt, int tt) { return p32_smem(P, Pb, ppt, tt) <= 227u * 1024u; }
 
-// The tiled kernel's block and formula tile depth.  Scenario slots: S rounded up to a power of
-// two, at least 4 (two scenarios run padded: a CTA on half the slots beats both the direct kernel
-// and a smaller CTA); Pb = 1024 / slots paths per tile (at least 32: the path chunks of the sums
-// lie inside one tile), served by 1024 threads (one path per thread) or 512 (two).
-static void tiled_shape(const Prepared& P, Fp32Shape& sh, int ppt) {
-  int sb = 4;
-  while (sb < P.n_scen) sb <<= 1;
-  sh.Sb = sb;
-  sh.Pb = 1024 / sb;
-  sh.TT = formula_tt(P, sh.Pb);
-  if (ppt == 2 && !p32_fits(P, sh.Pb, 2, sh.TT)) ppt = 1;
+// Sets the block (Pb paths per tile), paths per thread and tile depth of a tiled shape, if its
+// threads and its layout fit.  The CTA has a thread per (scenario, ppt paths) and at least 512:
+// the ones without a scenario share generation and bridge, which at few scenarios take most of the
+// time (S = 1, 2^14 paths, 64 paths a tile: 0.17 ms with 512 threads, 0.25 with 128).
+static bool p32_set_shape(const Prepared& P, Fp32Shape& sh, int pb, int ppt, int tt) {
+  const int stepping = (P.n_scen * pb / ppt + 31) / 32 * 32;
+  if (pb < 32 || (pb & (pb - 1)) || stepping > p32_max_threads(P.n, ppt) || !p32_fits(P, pb, ppt, tt)) return false;
+  sh.Pb = pb;
   sh.ppt = ppt;
-  sh.threads = sb * sh.Pb / ppt;
-  sh.smem = (int)p32_smem(P, sh.Pb, ppt, sh.TT);
+  sh.TT = tt;
+  sh.threads = std::max(stepping, 512);
+  sh.smem = (int)p32_smem(P, pb, ppt, tt);
+  return true;
 }
 
-// Tile depths the autotuner times besides the formula depth.
-static const int kTileCandidates[] = {24, 32, 48, 64, 80, 96, 128};
+// The formula shape, taken below the autotuner's launch size.  Two paths per thread, and the largest
+// tile (up to 256 paths) whose stepping threads the CTA may have: 9 scenarios of 3 assets on 128 paths
+// a tile 1.31 ms against 1.65 on 64 (2^17 paths × 252 steps), 17 on 64 paths 1.92 against 2.80 on 32,
+// where a warp steps two scenarios.  When that leaves SMs without a tile, the fewest paths per tile
+// (at least 32) that still give every SM at most one: a tile's time hardly depends on its paths
+// (3 assets, 252 steps: 0.12 ms on 32 paths, 0.19 on 128, 0.29 on 256).  Then the deepest tile that
+// fits: phase changes cost more than occupancy gains (16 scenarios: 10.1 ms at 128 steps, 10.8 at 64,
+// 13.4 at 24).
+static void formula_shape(const Prepared& P, Fp32Shape& sh, uint64_t npaths, int sm_count) {
+  int pb = 256;
+  while (pb > 32 && P.n_scen * pb / 2 > p32_max_threads(P.n, 2)) pb >>= 1;
+  while (pb > 32 && (npaths + pb / 2 - 1) / (pb / 2) <= (uint64_t)sm_count) pb >>= 1;
+  for (; pb >= 32; pb >>= 1)
+    for (int i = (int)(sizeof kTileDepths / sizeof kTileDepths[0]) - 1; i >= 0; --i)
+      if (p32_set_shape(P, sh, pb, 2, kTileDepths[i])) return;
+  raise(RG_ERR_GPU_ERROR, "phoenix32: the tile does not fit in shared memory");
+}
 
 // ----------------------------------------------------------------------- bridge plans --------
 // The plan of one tile depth TT, word offsets relative to its start:
@@ -161,22 +168,16 @@ static void build_bridge_plan(const std::vector<int32_t>& node_off, int64_t T, i
 }
 
 std::shared_ptr<const BridgePlans> p32_bridge_plans(const Prepared& P) {
-  Fp32Shape sh{};
-  tiled_shape(P, sh, kDefaultPpt);
   static std::mutex mu;
-  static std::map<std::pair<int64_t, int>, std::shared_ptr<const BridgePlans>> cache;
-  const std::pair<int64_t, int> key{P.T, sh.TT};
+  static std::map<int64_t, std::shared_ptr<const BridgePlans>> cache;
   {
     std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(key);
+    auto it = cache.find(P.T);
     if (it != cache.end()) return it->second;
   }
   auto out = std::make_shared<BridgePlans>();
-  std::vector<int> tts{sh.TT};
-  for (int tt : kTileCandidates)
-    if (std::find(tts.begin(), tts.end(), tt) == tts.end()) tts.push_back(tt);
-  for (int tt : tts) {
-    if (out->n == RG_BPLAN_MAX) break;
+  static_assert(sizeof kTileDepths / sizeof kTileDepths[0] <= RG_BPLAN_MAX, "a plan per tile depth");
+  for (int tt : kTileDepths) {
     out->tt[out->n] = tt;
     out->at[out->n] = (int32_t)out->words.size();
     build_bridge_plan(P.node_off, P.T, tt, P.stack_max, out->words);
@@ -184,7 +185,7 @@ std::shared_ptr<const BridgePlans> p32_bridge_plans(const Prepared& P) {
   }
   std::lock_guard<std::mutex> lock(mu);
   if (cache.size() >= 256) cache.clear();  // bounded: one entry per step count in use
-  cache[key] = out;
+  cache[P.T] = out;
   return out;
 }
 
@@ -232,15 +233,13 @@ Fp32Shape phoenix32_shape(const Prepared& P, uint64_t npaths, int sm_count) {
   if (p32_direct(P, npaths)) {
     // nothing for the scenarios to share: the per-thread kernel without shared-memory tiles
     sh.direct = 1;
-    sh.Sb = P.n_scen;
     sh.threads = 256;
     sh.ppt = 1;
     sh.grid = phoenix32d_grid(P, npaths, sm_count);
     sh.smem = P.stack_max * P.n * 256 * (int)sizeof(float);  // the bridge stacks (dynamic)
     return sh;
   }
-  tiled_shape(P, sh, kDefaultPpt);
-  if (sh.smem > 227 * 1024) raise(RG_ERR_GPU_ERROR, "phoenix32: the tile does not fit in shared memory");
+  formula_shape(P, sh, npaths, sm_count);
   p32_set_attributes();
   sh.grid = tiled_grid(P, sh, npaths, sm_count);
   return sh;
@@ -256,18 +255,6 @@ struct TiledKnobs {
   int pb, ppt, tt;
   bool operator==(const TiledKnobs& o) const { return pb == o.pb && ppt == o.ppt && tt == o.tt; }
 };
-
-// Sets the block (Pb paths per tile), paths per thread and tile depth of a tiled shape if the
-// block keeps a warp on 32·ppt paths of one scenario and its layout fits.
-bool p32_with(const Prepared& P, Fp32Shape& sh, TiledKnobs k) {
-  if (k.pb < 32 * k.ppt || (k.pb & (k.pb - 1)) || k.pb * sh.Sb > 1024 || !p32_fits(P, k.pb, k.ppt, k.tt)) return false;
-  sh.Pb = k.pb;
-  sh.ppt = k.ppt;
-  sh.threads = sh.Sb * k.pb / k.ppt;
-  sh.TT = k.tt;
-  sh.smem = (int)p32_smem(P, k.pb, k.ppt, k.tt);
-  return true;
-}
 
 std::mutex g_tune_mu;
 std::map<std::vector<int64_t>, TiledKnobs> g_tuned;  // launch shape -> (block, paths per thread, tile depth)
@@ -290,7 +277,7 @@ void p32_force_shape(int ppt, int tt, int pb) {
   if (pb != 0 && (pb < 32 * ppt || pb > 1024 || (pb & (pb - 1))))
     raise(RG_ERR_INVALID_ARGUMENT, "tiled shape: the block must be a power of two of 32 x paths per thread to 1024 paths");
   bool plan = tt == 0;
-  for (int c : kTileCandidates) plan = plan || c == tt;
+  for (int c : kTileDepths) plan = plan || c == tt;
   if (!plan) raise(RG_ERR_INVALID_ARGUMENT, "tiled shape: the tile depth must be one of the autotuner's candidates");
   std::lock_guard<std::mutex> lock(g_tune_mu);
   g_forced = TiledKnobs{pb, ppt, tt};
@@ -306,11 +293,11 @@ Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenar
   if (sh.direct) return sh;
   int dev = 0;
   cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-  const std::vector<int64_t> key{dev, sm_count, P.n, P.trade.has_lv, P.n_scen, sh.Sb, P.T, P.stack_max,
+  const std::vector<int64_t> key{dev, sm_count, P.n, P.trade.has_lv, P.n_scen, P.T, P.stack_max,
                                  P.trade.vr, P.trade.scrambler, P.trade.gx};
   auto apply = [&](TiledKnobs c, uint64_t paths) {
     Fp32Shape t = sh;
-    if (!p32_with(P, t, c)) return sh;
+    if (!p32_set_shape(P, t, c.pb, c.ppt, c.tt)) return sh;
     t.grid = tiled_grid(P, t, paths, sm_count);
     t.tuned = 1;
     return t;
@@ -331,14 +318,11 @@ Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenar
   const uint64_t prefix = (uint64_t)sh.grid * (uint64_t)sh.Pb * 2;
   if (!may_tune || npaths < prefix * 4) return sh;
   std::vector<TiledKnobs> cand;
-  std::vector<int> tts{sh.TT};
-  tts.insert(tts.end(), std::begin(kTileCandidates), std::end(kTileCandidates));
   for (int pb : {sh.Pb, sh.Pb / 2})
     for (int ppt = 1; ppt <= 2; ++ppt)
-      for (int tt : tts) {
+      for (int tt : kTileDepths) {
         Fp32Shape c = sh;
-        const TiledKnobs k{pb, ppt, tt};
-        if (std::find(cand.begin(), cand.end(), k) == cand.end() && p32_with(P, c, k)) cand.push_back(k);
+        if (p32_set_shape(P, c, pb, ppt, tt)) cand.push_back({pb, ppt, tt});
       }
   LaunchOut lo = out;  // the partial sums are overwritten by the real launch afterwards
   lo.ko_steps = nullptr;
@@ -381,7 +365,8 @@ void launch_phoenix32(const Prepared& P, const DevTables& tb, const DevScenario*
   for (int i = 0; i < tb.n_bplan; ++i)
     if (tb.bplan_tt[i] == sh.TT) plan = tb.bplan + tb.bplan_at[i];
   if (!plan) raise(RG_ERR_GPU_ERROR, "phoenix32: no bridge plan staged for the tile depth");
-  if (sh.Pb < 32 || (sh.Pb & (sh.Pb - 1)) || sh.threads * sh.ppt != sh.Sb * sh.Pb || (sh.ppt != 1 && sh.ppt != 2))
+  if (sh.Pb < 32 || (sh.Pb & (sh.Pb - 1)) || sh.threads * sh.ppt < P.n_scen * sh.Pb || (sh.ppt != 1 && sh.ppt != 2) ||
+      sh.threads > p32_max_threads(P.n, sh.ppt))
     raise(RG_ERR_GPU_ERROR, "phoenix32: invalid tile shape");
   const bool lvk = P.trade.has_lv != 0;
   const P32Args a{P.trade, tb, scen, scen32, P.n_scen, sh.Pb, sh.TT, NNmax, P.stack_max, ln_ko, ln_cb, ln_ki,

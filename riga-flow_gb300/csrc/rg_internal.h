@@ -255,7 +255,7 @@ int phoenix64_grid(uint64_t npaths);
 void launch_phoenix64(const Prepared& P, const DevTables& tb, const DevScenario* scen_dev,
                       uint64_t path0, uint64_t npaths, const LaunchOut& out, cudaStream_t s);
 struct Fp32Shape {
-  int Sb, Pb, TT, threads, grid, smem;
+  int Pb, TT, threads, grid, smem;
   int ppt;     // paths per thread of the tiled kernel (1 or 2)
   int tuned;   // 1: Pb, ppt and TT came from the autotuner's cache (or were forced)
   int direct;  // 1: the per-thread kernel of phoenix32d.cu; then only grid and threads are used
@@ -275,15 +275,14 @@ Fp32Shape phoenix32_shape(const Prepared& P, uint64_t npaths, int sm_count);
 // Rows of the FP32 kernels' partial sums partial[chunk][scenario][RG_ACC]: one per 32 paths.
 uint64_t p32_chunks(uint64_t npaths);
 // The level-ordered evaluation plans of the streamed Brownian bridge for every tile depth the tiled
-// FP32 kernel may launch with (its formula depth and the autotuner's candidates): packed words,
-// and per depth its value and word offset.
+// FP32 kernel may launch with: packed words, and per depth its value and word offset.
 struct BridgePlans {
   std::vector<uint32_t> words;
   int32_t tt[RG_BPLAN_MAX], at[RG_BPLAN_MAX];
   int n = 0;
 };
-// A plan depends only on the step count (the node schedule and stack depth) and the tile depths,
-// so the plans are built once per (steps, formula depth) and shared process-wide.
+// A plan depends only on the step count (the node schedule and stack depth) and the tile depth, so the
+// plans are built once per step count and shared process-wide.
 std::shared_ptr<const BridgePlans> p32_bridge_plans(const Prepared& P);
 // The tiled kernel's step tiling from the autotuner: a cached choice for the launch's shape, or —
 // when `may_tune` and the launch is large enough to amortise it — one tuning pass that times the

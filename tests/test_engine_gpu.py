@@ -548,3 +548,25 @@ def test_correlation_factor_across_conditioning(engine, n, rho):
         assert (g.ko_step, g.qualified_steps, g.paid_periods) == (w.ko_step, w.qualified_steps, w.paid_periods)
         assert abs(g.pv - w.pv) <= 1e-12 * abs(w.pv)
         assert abs(g.worst_final - w.worst_final) <= 1e-12 * abs(w.worst_final)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("paths", [1, 33, 4097, 20000])
+def test_tiled_formula_shapes_price_identically(engine, n, paths):
+    """The tiled kernel's formula shape follows the scenario and path counts (32 to 256 paths a tile,
+    512 to 640 threads, warps of two scenarios); a scenario's price does not: each of a batch's
+    scenarios has the same bytes in every longer batch."""
+    req = workloads.plain3(paths, steps=60, fp32=True)
+    req.trade = workloads.phoenix_trade(n, 60, 60 / 252)
+    req.market.spots, req.market.vols = [100.0] * n, [0.2 + 0.03 * f for f in range(n)]
+    req.market.dividend_yields = [0.01] * n
+    req.market.correlation = [[1.0 if i == j else 0.4 for j in range(n)] for i in range(n)]
+    scen = []
+    for k in range(32):
+        m = copy.deepcopy(req.market)
+        m.spots[k % n] *= 1.0 + 0.002 * k
+        m.risk_free_rate += 1e-4 * (k % 3)
+        scen.append((m, None))
+    full = [bytes(r) for r in engine.price_scenarios_raw(req, scen)]
+    for S in (1, 2, 3, 4, 5, 8, 9, 10, 16, 17, 20, 21, 25):
+        assert [bytes(r) for r in engine.price_scenarios_raw(req, scen[:S])] == full[:S], S
