@@ -369,7 +369,7 @@ BookStaged stage_book_static(DevBuf& tables, cudaStream_t st, const rg_book_requ
   const size_t o_tr = pk.add(B.trades), o_ord = pk.add(B.order);
   const size_t o_corr = pk.add(r->universe.correlation, (size_t)U * U);
   const size_t o_L = pk.reserve(sizeof(double) * U * U), o_L32 = pk.reserve(sizeof(float) * U * U);
-  const size_t lut_words = book_lut_words(r->config, U, B.TU), o_lut = (pk.host.size() + 255) & ~size_t(255);
+  const size_t lut_words = sobol_lut_words(r->config, U, B.TU), o_lut = (pk.host.size() + 255) & ~size_t(255);
   tables.ensure(o_lut + lut_words * sizeof(uint32_t));
   uint8_t* dev = static_cast<uint8_t*>(tables.ptr);
   cuda_check(cudaMemcpyAsync(dev, pk.host.data(), pk.host.size(), cudaMemcpyHostToDevice, st), "book H2D");
@@ -480,7 +480,7 @@ size_t estimate_book_bytes(const rg_book_request* r, int n_scen) {
   const uint64_t blocks = fp32 ? (P + unit - 1) / unit : ((PC + 127) / 128) * chunks;
   b += (size_t)blocks * pairs * RG_ACC * 8 + pairs * RG_ACC * 8;
   size_t sob_rows = r->config.dim_mode == RG_DIM_FULL ? U * TU : 512;
-  b += sob_rows * 128 + book_lut_words(r->config, (int64_t)U, (int64_t)TU) * 4 + TU * 32 + S * TU * 12 + pairs * 100 + (size_t)r->n_trades * 256 + (size_t(64) << 10);
+  b += sob_rows * 128 + sobol_lut_words(r->config, (int64_t)U, (int64_t)TU) * 4 + TU * 32 + S * TU * 12 + pairs * 100 + (size_t)r->n_trades * 256 + (size_t(64) << 10);
   return b + b / 8 + (size_t(1) << 20);
 }
 

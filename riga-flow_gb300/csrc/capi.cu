@@ -325,17 +325,6 @@ static Staged stage(Workspace& W, const rg_price_request* req, Prepared& P) {
     bp = p32_bridge_plans(P);
     o_bplan = pk.add(bp->words);
   }
-  // the FP32 kernels' consumption-order Sobol tables (1.1 MB per 1,000 steps of 3 assets), for
-  // launches long enough that generating from them pays for their upload
-  size_t o_sobt = 0, o_slut = 0;
-  int32_t lut_o = -1;
-  if (req->config.precision == RG_PRECISION_FP32 && tr.vr == RG_VR_SOBOL && req->config.paths >= (uint64_t(1) << 16)) {
-    lut_o = (int32_t)((req->config.first_path + 1) & 31);
-    std::shared_ptr<const SobolLut> t =
-        sobol_lut_tables(P, tr.sob_dim, (uint32_t)lut_o, tr.scrambler == RG_SCRAMBLE_DIGITAL_SHIFT);
-    o_sobt = pk.add(t->st);
-    o_slut = pk.add(t->lut);
-  }
   size_t o_scen = pk.add(P.scen), o_s32 = pk.add(P.scen32);
   // local-vol surfaces: inputs (grids) and outputs
   const int gx = tr.gx;
@@ -380,7 +369,14 @@ static Staged stage(Workspace& W, const rg_price_request* req, Prepared& P) {
       o_ax[j] = same >= 0 ? o_ax[same] : pk.add(calib_axes(req->local_vol[key.asset], key.spot, key.rate, gx));
     }
   }
-  uint8_t* base = static_cast<uint8_t*>(W.device(WS_ARENA, pk.host.size()));
+  // behind the packed tables, the FP32 kernels' consumption-order Sobol tables, built on the device for
+  // launches that gain more from them than the building kernel takes (4096 paths: 54 us with and
+  // without, and 4 us to build; 2^14 paths 0.50 against 0.55 ms); the static region holds them from
+  // 2^16 paths only
+  const size_t o_lut = (pk.host.size() + 255) & ~size_t(255);
+  const uint64_t lut_from = W.persistent() ? uint64_t(1) << 13 : uint64_t(1) << 16;
+  const size_t lut_words = req->config.paths >= lut_from ? sobol_lut_words(req->config, P.n, P.T) : 0;
+  uint8_t* base = static_cast<uint8_t*>(W.device(WS_ARENA, o_lut + lut_words * sizeof(uint32_t)));
   if (tr.has_lv) {
     if (SurfaceCache* cache = W.surfaces()) cache->begin_call();
     double* sc = static_cast<double*>(W.device(WS_CALIB, scratch * sizeof(double)));
@@ -456,10 +452,10 @@ static Staged stage(Workspace& W, const rg_price_request* req, Prepared& P) {
     tb.bplan_at[i] = i < tb.n_bplan ? bp->at[i] : 0;
   }
   tb.lv_nt = P.lv_nt_max;
-  tb.sob_t = lut_o >= 0 ? reinterpret_cast<const uint32_t*>(base + o_sobt) : nullptr;
-  tb.sob_lut = lut_o >= 0 ? reinterpret_cast<const uint32_t*>(base + o_slut) : nullptr;
-  tb.sob_nq = (int32_t)(P.T * P.n);
-  tb.sob_lut_o = lut_o;
+  if (lut_words) {
+    launch_sobol_lut(tr, tb, P.n, req->config.first_path, reinterpret_cast<uint32_t*>(base + o_lut), W.stream);
+    if (W.timing) W.timing->kernel_launches += 1;
+  }
   S.scen = reinterpret_cast<DevScenario*>(base + o_scen);
   S.scen32 = reinterpret_cast<DevScen32*>(base + o_s32);
   if (tr.has_lv) {
@@ -601,7 +597,7 @@ void price_with(Workspace& W, const rg_price_request* req, const rg_scenario* sc
     uint64_t rows;
     Fp32Shape sh{};
     if (fp32) {
-      sh = phoenix32_shape(P, paths, W.sm_count);
+      sh = phoenix32_shape(P, S.tb, req->config.first_path, paths, W.sm_count);
       rows = p32_chunks(paths);
     } else {
       rows = W.persistent() ? path64_rows(P.n, paths) : (uint64_t)phoenix64_grid(paths);
@@ -715,7 +711,7 @@ size_t estimate_price_bytes(const rg_price_request* r, int n_scen) {
     b += surf * ((2 * nt * gx + gx) * 8 + (4 * nt * gx + gx + 6 * nt * nk) * 8);  // calibration
     if (fp32) b += surf * T * gx * 8;                                            // step rows
   }
-  if (fp32) b += T * 160;  // bridge plans of the tiled kernel
+  if (fp32) b += T * 160 + sobol_lut_words(r->config, (int)n, (int64_t)T) * 4;  // bridge plans, Sobol tables
   // rows of partial sums: one per 32-path chunk (FP32 kernels) or per block (FP64 kernel)
   const size_t grid = (size_t)(fp32 ? p32_chunks(r->config.paths) : path64_rows((int)std::min<size_t>(n, RG_NMAX), r->config.paths));
   if (!fp32) b += path64_bytes((int)std::min<size_t>(n, RG_NMAX), (int64_t)T, r->config.paths);
@@ -966,7 +962,7 @@ static void run_path_range(rg_engine* e, const rg_price_request* req, uint64_t f
     LaunchOut lo{};
     lo.mcz = mcz;
     Fp32Shape sh{};
-    if (fp32) sh = phoenix32_shape(P, m, engine_sm_count(e));
+    if (fp32) sh = phoenix32_shape(P, S.tb, req->config.first_path + first + done, m, engine_sm_count(e));
     lo.grid = (int)(fp32 ? p32_chunks(m) : path64_rows(P.n, m));
     lo.partial = static_cast<double*>(W.device(WS_PARTIAL, (size_t)lo.grid * P.n_scen * RG_ACC * sizeof(double)));
     if (out) lo.records = static_cast<rg_path_record*>(W.device(WS_RECORDS, m * sizeof(rg_path_record)));

@@ -227,10 +227,10 @@ static int tiled_grid(const Prepared& P, const Fp32Shape& sh, uint64_t npaths, i
   return grid < 1 ? 1 : grid;
 }
 
-Fp32Shape phoenix32_shape(const Prepared& P, uint64_t npaths, int sm_count) {
+Fp32Shape phoenix32_shape(const Prepared& P, const DevTables& tb, uint64_t path0, uint64_t npaths, int sm_count) {
   Fp32Shape sh{};
   if (P.n_scen > 32) raise(RG_ERR_INVALID_ARGUMENT, "at most 32 scenarios per fused launch");
-  if (p32_direct(P, npaths)) {
+  if (p32_direct(P, npaths, tb.sob_lut && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o)) {
     // nothing for the scenarios to share: the per-thread kernel without shared-memory tiles
     sh.direct = 1;
     sh.threads = 256;

@@ -3,13 +3,12 @@
 //
 // The tiled kernel (phoenix32.cu) stages a tile's normals and Brownian increments in shared
 // memory so that the scenarios of a path share one generation; with one scenario there is nothing
-// to share and the staging only costs occupancy.  (Measured on the 3-asset local-vol trade at 2^20
-// paths: 17.5 ms here against 24.4 ms for the tiled kernel on four padded scenario slots; the
-// tiled kernel wins with two or more scenarios, and below about 2^18 paths, where one path per
-// thread leaves too few warps to hide the per-step latency.)  Here a warp walks 32 consecutive
+// to share and the staging only costs occupancy; the tiled kernel wins with two or more scenarios, and
+// on few paths, where one path per thread leaves too few warps to hide the per-step latency
+// (p32_direct, rg_internal.h, has the line and both sides).  Here a warp walks 32 consecutive
 // paths of one scenario through time:
-//   * Sobol points from consumption-order tables staged for the launch (host_prep.cu,
-//     direct_sobol_tables): the warp's 32 points lie in at most two aligned 32-point blocks, and
+//   * Sobol points from consumption-order tables staged for the launch (sobol_lut_kernel,
+//     book_gen32.cu): the warp's 32 points lie in at most two aligned 32-point blocks, and
 //     Gray codes are linear over XOR, so a point is the block's high-bit term X(gray(a)) — one
 //     coalesced row of transposed directions per set bit of gray(a), for a batch of the next
 //     32 / N nodes' dimensions at once, kept in shared memory — XOR the lane's low-bit term, one

@@ -51,12 +51,6 @@ struct BookStaged {
   double* L = nullptr;
   float* L32 = nullptr;
 };
-// Words of the consumption-order Sobol tables of the FP32 generation (none for other lanes, and none
-// beyond half a gigabyte: it then forms every point from the direction table).
-inline size_t book_lut_words(const rg_simulation_config& c, int64_t U, int64_t TU) {
-  const size_t w = (size_t)64 * (size_t)U * (size_t)TU;
-  return c.precision == RG_PRECISION_FP32 && c.variance_reduction == RG_VR_SOBOL && w <= (size_t(1) << 27) ? w : 0;
-}
 // QMC tables, bridge schedule, trades, work order and the universe factor (FP64 Cholesky on the
 // device, then its FP32 copy) into `tables`, enqueued on `st`.
 BookStaged stage_book_static(DevBuf& tables, cudaStream_t st, const rg_book_request* r, const BookPlan& B);

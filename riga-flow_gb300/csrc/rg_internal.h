@@ -163,14 +163,12 @@ void bridge_schedule_into(int64_t T, double dt, Prepared& P);
 // The Sobol direction table for `dim` dimensions (process-wide cache).
 const std::vector<uint32_t>& sobol_table(int64_t dim);
 std::vector<double> calib_axes(const rg_implied_vol_grid& g, double spot, double rate, int gx);
-// The FP32 kernels' consumption-order Sobol tables for points starting at offset o within a
-// 32-point block (host_prep.cu): transposed directions st[32][n·T] and the lanes' low-bit terms
-// lut[n·T][32]; built once per (directions, assets, steps, seed, scrambler, o) and shared
-// process-wide.
-struct SobolLut {
-  std::vector<uint32_t> st, lut;
-};
-std::shared_ptr<const SobolLut> sobol_lut_tables(const Prepared& P, int64_t sob_dim, uint32_t o, bool shift);
+// Words of the FP32 kernels' consumption-order Sobol tables of n factors over T nodes: none for other
+// lanes, and none beyond half a gigabyte (the kernels then form every point from the direction table).
+inline size_t sobol_lut_words(const rg_simulation_config& c, int64_t n, int64_t T) {
+  const size_t w = (size_t)64 * (size_t)n * (size_t)T;
+  return c.precision == RG_PRECISION_FP32 && c.variance_reduction == RG_VR_SOBOL && w <= (size_t(1) << 27) ? w : 0;
+}
 // The first `count` primes (a copy of a process-wide cache; at least `count` entries).
 std::vector<uint32_t> first_primes(int count);
 // Halton bases and permutations.
@@ -260,18 +258,23 @@ struct Fp32Shape {
   int tuned;   // 1: Pb, ppt and TT came from the autotuner's cache (or were forced)
   int direct;  // 1: the per-thread kernel of phoenix32d.cu; then only grid and threads are used
 };
-// Scenario counts up to this value run on the direct kernel (phoenix32d.cu), when the launch has
-// at least p32_direct_min_paths(n) paths: one path per thread needs enough warps to fill the GPU
-// (measured crossover against the tiled kernel: about 2^18 paths for 1-3 assets, 2^16 for 4-5).
-constexpr int kP32DirectMaxScen = 1;
-inline uint64_t p32_direct_min_paths(int n) { return n >= 4 ? (uint64_t(1) << 16) : (uint64_t(3) << 16); }
-inline bool p32_direct(const Prepared& P, uint64_t npaths) {
-  return P.n_scen <= kP32DirectMaxScen && npaths >= p32_direct_min_paths(P.n);
+// A single scenario runs on the direct kernel (phoenix32d.cu) from a path count that fills the GPU with
+// one path per thread.  Where the two kernels cross was measured at 252 steps: on digitally shifted
+// Sobol points from the tables (`lut`) 2^16 paths for one asset (0.147 ms against the tiled kernel's
+// 0.151), 49,152 for two, 2^15 for three (0.20 against 0.21 flat, 0.24 against 0.27 local vol) and
+// 24,576 for four or five (2^15 paths: 0.31 against 0.46); lanes that cost more per normal spread it
+// over more threads in the tiled kernel, which keeps them up to 3·2^16 paths (1-3 assets) or 2^16.
+inline bool p32_direct(const Prepared& P, uint64_t npaths, bool lut) {
+  const int n = P.n;
+  const bool cheap = lut && P.trade.scrambler == RG_SCRAMBLE_DIGITAL_SHIFT;
+  const uint64_t from = !cheap ? (n >= 4 ? 65536 : 196608) : (n == 1 ? 65536 : (n == 2 ? 49152 : (n == 3 ? 32768 : 24576)));
+  return P.n_scen == 1 && npaths >= from;
 }
 int phoenix32d_grid(const Prepared& P, uint64_t npaths, int sm_count);
 void launch_phoenix32d(const Prepared& P, const DevTables& tb, const DevScenario* scen, const DevScen32* scen32,
                        uint64_t path0, uint64_t npaths, int grid, const LaunchOut& out, cudaStream_t st);
-Fp32Shape phoenix32_shape(const Prepared& P, uint64_t npaths, int sm_count);
+// `tb`, `path0`: whether the launch draws its points from staged Sobol tables.
+Fp32Shape phoenix32_shape(const Prepared& P, const DevTables& tb, uint64_t path0, uint64_t npaths, int sm_count);
 // Rows of the FP32 kernels' partial sums partial[chunk][scenario][RG_ACC]: one per 32 paths.
 uint64_t p32_chunks(uint64_t npaths);
 // The level-ordered evaluation plans of the streamed Brownian bridge for every tile depth the tiled
