@@ -25,13 +25,16 @@
 //      the next tile.
 //   S. scenario stepping — every (path, scenario) correlates dW with its scenario's Cholesky
 //      factor (the bridge is linear, so L·bridge(z) = bridge(L·z)), steps ln(S/S0) under flat vol
-//      or its scenario's Dupire surface and runs the Phoenix state machine.
+//      or its scenario's Dupire surface and runs the Phoenix state machine.  The surfaces' rows are
+//      gathered from global memory, or, where shared memory has room, from buffers of the next RT steps
+//      of every surface, which one warp fills by bulk copies.
 // Generation is paid once per path, not once per scenario.  Path state and a path's payoff values
 // are FP32; each 32-path chunk is summed in FP32 by a fixed shuffle butterfly and written as FP64
 // to partial[chunk][scenario], and the chunks are reduced in chunk order, so the sums — and the
 // prices — are the same for every launch shape (paths per thread, tile depth, block).
 #pragma once
 #include "p32_path.cuh"
+#include "rg_async.cuh"
 #include "rg_internal.h"
 
 namespace rg {
@@ -39,7 +42,7 @@ namespace rg {
 // Byte offsets of the kernel's dynamic shared-memory regions, 16-byte aligned, and their total.
 // Computed by the same function on the host (to size the launch) and in the kernel (to carve).
 struct P32Layout {
-  uint32_t flags, per, thr, noff, ncf, qmc, node4, plan, z, dw, total;
+  uint32_t flags, per, thr, noff, ncf, qmc, node4, plan, z, dw, rows, bars, total;
 };
 
 // Floats per row of the Z array: N·(Pb + 4) and one more, so that rows start in different banks.
@@ -48,7 +51,9 @@ __host__ __device__ inline int p32_zrow(int N, int Pb) { return N * (Pb + 4) + 1
 // path + 1) pairs are read as one aligned 8-byte load.
 __host__ __device__ inline int p32_dwstep(int N, int Pb, int ppt) { return Pb * N + (ppt == 2 ? 2 : 1); }
 
-__host__ __device__ inline P32Layout p32_layout(int N, int Pb, int TT, int NNmax, int stack_max, int ppt) {
+// `row_words`: 8-byte words of one staging buffer of local-vol rows (surfaces × steps × grid points), or 0.
+__host__ __device__ inline P32Layout p32_layout(int N, int Pb, int TT, int NNmax, int stack_max, int ppt,
+                                                uint32_t row_words) {
   P32Layout L;
   uint32_t o = 0;
   auto put = [&o](uint32_t& field, uint32_t bytes) {
@@ -72,6 +77,8 @@ __host__ __device__ inline P32Layout p32_layout(int N, int Pb, int TT, int NNmax
   put(L.plan, (uint32_t)(NNmax + (NNmax + 1) + (TT + 1) + stack_max) * 4u);
   put(L.z, zb);
   put(L.dw, (uint32_t)TT * (uint32_t)p32_dwstep(N, Pb, ppt) * 4u);  // dW[step][factor][path]
+  put(L.rows, 2u * row_words * 8u);                                  // [buffer][surface][step][grid point]
+  put(L.bars, row_words ? 32u : 0u);                                 // full[2], empty[2]
   L.total = o;
   return L;
 }
@@ -157,10 +164,13 @@ static inline int p32_phase_clocks_tu(unsigned long long out[4], bool reset) {
 // 96 registers do without spilling, so that CTA may have 640.
 __host__ __device__ constexpr int p32_max_threads(int n, int ppt) { return ppt == 1 ? 1024 : (n <= 3 ? 640 : 512); }
 
-template <int N, bool LV, bool REC, int PPT>
+// LV: flat vol, Dupire rows gathered from global memory, or staged in shared memory.
+enum { P32_FLAT = 0, P32_LV = 1, P32_LV_STAGED = 2 };
+
+template <int N, int LV, bool REC, int PPT>
 __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
     DevTrade tr, DevTables tb, const DevScenario* __restrict__ scen,
-    const DevScen32* __restrict__ scen32, int S, int Pb, int TT, int NNmax, int stack_max,
+    const DevScen32* __restrict__ scen32, int S, int Pb, int TT, int NNmax, int stack_max, int RT, int n_surf,
     float ln_ko, float ln_cb, float ln_ki, uint64_t path0, uint64_t npaths, const uint32_t* __restrict__ plan,
     double* __restrict__ partial, int32_t* __restrict__ ko_steps, rg_path_record* __restrict__ records) {
   using V = PVec<PPT>;
@@ -172,7 +182,8 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
   const int T = (int)tr.steps;
   const uint64_t nchunks = (npaths + 31) / 32;
   // ---- shared-memory carve-up (the host sizes the launch from the same layout)
-  const P32Layout L = p32_layout(N, Pb, TT, NNmax, stack_max, PPT);
+  const uint32_t row_words = LV == P32_LV_STAGED ? (uint32_t)(n_surf * RT * tr.gx) : 0u;
+  const P32Layout L = p32_layout(N, Pb, TT, NNmax, stack_max, PPT, row_words);
   uint32_t dyn_bytes;
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
   if (L.total > dyn_bytes) {
@@ -200,6 +211,9 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
   uint32_t* s_pstk = reinterpret_cast<uint32_t*>(s_poff + TT + 1);
   float* Z = reinterpret_cast<float*>(smem_raw + L.z);
   float* dW = reinterpret_cast<float*>(smem_raw + L.dw);
+  const float2* s_rows = reinterpret_cast<const float2*>(smem_raw + L.rows);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + L.bars);
+  uint64_t* empty = full + 2;
 
   // stepping: thread tid serves scenario s and paths pl0 .. pl0 + PPT - 1 of each tile
   const int tps = Pb / PPT;  // threads per scenario
@@ -235,7 +249,9 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
       sig[f] = V::splat(s3.sig[f]);
       lva[f] = s3.a_u[f] * inv_gxm1;
       lvb[f] = s3.inv_h[f] * inv_gxm1;
-      lvo[f] = (uint32_t)s3.surf_off[f] - 0x4B000000u;
+      // staged: the surface's first row in a buffer
+      lvo[f] = (LV == P32_LV_STAGED ? (uint32_t)(s3.surf_off[f] / (T * gx)) * (uint32_t)(RT * gx)
+                                    : (uint32_t)s3.surf_off[f]) - 0x4B000000u;
       x0[f] = s3.x0[f];
     }
   }
@@ -245,6 +261,40 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
   // for this launch's offset within a 32-point block; a lane's point may lie in the next block
   const bool sob_lut = tr.vr == RG_VR_SOBOL && tb.sob_lut != nullptr && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o;
   const bool upper = (uint32_t)tb.sob_lut_o + (uint32_t)lane >= 32u;
+  // staged rows: RT steps of every surface at a time in one of two buffers.  The first warp past the
+  // stepping ones fills them by bulk copies (one per surface) counted on a buffer's "full" barrier; every
+  // stepping warp releases a buffer on its "empty" barrier.  (Filled by a stepping warp they cost 1.8 us
+  // a buffer at 3 surfaces and 3.8 at 18: the whole CTA waits while that warp waits and copies.)  The
+  // first two buffers of a time tile are filled while its normals are generated.  Waits are bounded: one
+  // that runs out poisons the launch's sums and ends all waiting.
+  uint32_t use = 0;  // buffers used so far, in every thread
+  bool stuck = false;
+  const int n_step_warps = (S * tps + 31) >> 5;
+  const bool producer = LV == P32_LV_STAGED && wid == n_step_warps;
+  if (LV == P32_LV_STAGED) {
+    if (tid == 0) {
+      for (int b = 0; b < 2; ++b) {
+        mbar_init(&full[b], 1);
+        mbar_init(&empty[b], (uint32_t)n_step_warps);
+      }
+      mbar_init_fence();
+    }
+    __syncthreads();
+  }
+  // use u holds the rows of steps [t, t + steps); called by all lanes of the producer
+  auto stage_rows = [&](uint32_t u, int t, int steps) {
+    const uint32_t b = u & 1u;
+    if (u >= 2 && !stuck && !mbar_wait_bounded(&empty[b], ((u >> 1) - 1u) & 1u)) stuck = true;
+    if (__any_sync(0xffffffffu, stuck)) {
+      stuck = true;
+      return;
+    }
+    if (lane == 0) mbar_expect_tx(&full[b], (uint32_t)(n_surf * steps * gx) * 8u);
+    __syncwarp();
+    float2* dst = reinterpret_cast<float2*>(smem_raw + L.rows) + b * row_words;
+    for (int k = lane; k < n_surf; k += 32)
+      bulk_g2s(dst + k * RT * gx, tb.lv_rows + ((size_t)k * T + t) * gx, (uint32_t)(steps * gx) * 8u, &full[b]);
+  };
   RG_PHASE_BEGIN();
   const uint64_t ntiles = (npaths + Pb - 1) / Pb;
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -266,6 +316,10 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
       const int tn = min(TT, T - t0);
       const int n0 = __ldg(tb.node_off + t0), n1 = __ldg(tb.node_off + t0 + tn);
       const int nn = n1 - n0;
+      if (producer) {
+        stage_rows(use, t0, min(RT, tn));
+        if (tn > RT) stage_rows(use + 1, t0 + RT, min(RT, tn - RT));
+      }
       // ---- G: standard normals of the tile's bridge nodes, and the tile's step schedule
       for (int i = tid; i < tn; i += blockDim.x) {
         const uint32_t fl = __ldg(tb.step_flags + t0 + i);
@@ -467,10 +521,12 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
       // Phoenix machine of both in order, so that the second step's local-vol lookups overlap the
       // first step's barrier tests and one vote serves two steps.
       if (warp_on) {
+        int sub0 = 0;
         // one Euler step of every asset (correlated increment, local-vol lookup, log-space update);
         // returns the worst-of log performance of each path after the step
         auto euler = [&](int tt, float (&wmin)[PPT]) {
-          const int tg = (t0 + tt) * gx;
+          // the step's row within a surface (staged: within the buffer of steps from sub0)
+          const int tg = LV == P32_LV_STAGED ? (int)((use & 1u) * row_words) + (tt - sub0) * gx : (t0 + tt) * gx;
           V d[N], y[N];
 #pragma unroll
           for (int f = 0; f < N; ++f) {
@@ -502,7 +558,7 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
 #pragma unroll
               for (int j = 0; j < PPT; ++j) {
                 const uint32_t idx = lvo[f] + (uint32_t)tg + (uint32_t)__float_as_int(fl.v[j]);
-                const float2 r = __ldg(tb.lv_rows + idx);
+                const float2 r = LV == P32_LV_STAGED ? s_rows[idx] : __ldg(tb.lv_rows + idx);
                 sg.v[j] = fmaf(u01.v[j], r.y, r.x);
               }
             } else {
@@ -550,44 +606,58 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
             }
           }
         };
-        int tt = 0;
-        for (; tt + 1 < tn; tt += 2) {
-          float w0[PPT], w1[PPT];
-          euler(tt, w0);
-          euler(tt + 1, w1);
+        const int per_buf = LV == P32_LV_STAGED ? RT : tn;
+        for (; sub0 < tn; sub0 += per_buf) {
+          const int sub1 = min(tn, sub0 + per_buf);
+          if (LV == P32_LV_STAGED && !stuck && !mbar_wait_bounded(&full[use & 1u], (use >> 1) & 1u)) stuck = true;
+          int tt = sub0;
+          for (; tt + 1 < sub1; tt += 2) {
+            float w0[PPT], w1[PPT];
+            euler(tt, w0);
+            euler(tt + 1, w1);
 #pragma unroll
-          for (int j = 0; j < PPT; ++j) worst[j] = w1[j];
-          const uint32_t f0 = s_flags[tt], f1 = s_flags[tt + 1];
-          if ((f0 | f1) & (STEP_PERIOD_RESET | STEP_PERIOD_END)) {
-            phoenix(tt, w0);
-            phoenix(tt + 1, w1);
-          } else {
-            // two plain steps: when no path of the warp knocks out in either, both only accrue
-            const float2 th0 = s_thr[tt], th1 = s_thr[tt + 1];
-            bool any = false;
-#pragma unroll
-            for (int j = 0; j < PPT; ++j) any |= ph[j].alive & ((w0[j] >= th0.y) | (w1[j] >= th1.y));
-            if (__any_sync(0xffffffffu, any)) {
+            for (int j = 0; j < PPT; ++j) worst[j] = w1[j];
+            const uint32_t f0 = s_flags[tt], f1 = s_flags[tt + 1];
+            if ((f0 | f1) & (STEP_PERIOD_RESET | STEP_PERIOD_END)) {
               phoenix(tt, w0);
               phoenix(tt + 1, w1);
             } else {
+              // two plain steps: when no path of the warp knocks out in either, both only accrue
+              const float2 th0 = s_thr[tt], th1 = s_thr[tt + 1];
+              bool any = false;
 #pragma unroll
-              for (int j = 0; j < PPT; ++j) {
-                const bool a = ph[j].alive;
-                const int acc = (int)(a & (w0[j] >= th0.x)) + (int)(a & (w1[j] >= th1.x));
-                ph[j].qual += acc;
-                if (REC) ph[j].qualified += acc;
+              for (int j = 0; j < PPT; ++j) any |= ph[j].alive & ((w0[j] >= th0.y) | (w1[j] >= th1.y));
+              if (__any_sync(0xffffffffu, any)) {
+                phoenix(tt, w0);
+                phoenix(tt + 1, w1);
+              } else {
+#pragma unroll
+                for (int j = 0; j < PPT; ++j) {
+                  const bool a = ph[j].alive;
+                  const int acc = (int)(a & (w0[j] >= th0.x)) + (int)(a & (w1[j] >= th1.x));
+                  ph[j].qual += acc;
+                  if (REC) ph[j].qualified += acc;
+                }
               }
             }
           }
-        }
-        if (tt < tn) {
-          float w0[PPT];
-          euler(tt, w0);
+          if (tt < sub1) {
+            float w0[PPT];
+            euler(tt, w0);
 #pragma unroll
-          for (int j = 0; j < PPT; ++j) worst[j] = w0[j];
-          phoenix(tt, w0);
+            for (int j = 0; j < PPT; ++j) worst[j] = w0[j];
+            phoenix(tt, w0);
+          }
+          if (LV == P32_LV_STAGED) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[use & 1u]);
+            ++use;
+          }
         }
+      } else if (LV == P32_LV_STAGED) {
+        if (producer)
+          for (int sub = 2; sub * RT < tn; ++sub) stage_rows(use + sub, t0 + sub * RT, min(RT, tn - sub * RT));
+        use += (uint32_t)((tn + RT - 1) / RT);
       }
       __syncthreads();
       RG_PHASE_MARK(2);
@@ -619,7 +689,7 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
       }
       const uint64_t chunk = (tile0 + (uint64_t)(pl0 & ~31)) >> 5;
       if (lane_ok && lk < RG_ACC && chunk < nchunks)
-        partial[((size_t)chunk * S + s) * RG_ACC + lk] = (double)mine;
+        partial[((size_t)chunk * S + s) * RG_ACC + lk] = stuck ? __longlong_as_double(0x7ff8000000000000LL) : (double)mine;
     }
     RG_PHASE_MARK(3);
   }
@@ -632,7 +702,7 @@ struct P32Args {
   DevTables tb;
   const DevScenario* scen;
   const DevScen32* scen32;
-  int S, Pb, TT, NNmax, stack_max;
+  int S, Pb, TT, NNmax, stack_max, RT, n_surf;
   float ln_ko, ln_cb, ln_ki;
   uint64_t path0, npaths;
   const uint32_t* plan;
@@ -645,8 +715,8 @@ struct P32Args {
 // vol; rec: path records), its launch, and the phase clocks of that translation unit's kernels
 // (RG_PHASE_CLOCKS builds).
 #define RG_P32_DECLARE(NN, PP)                                                                      \
-  const void* p32_kernel_ptr_n##NN##p##PP(bool lv, bool rec);                                      \
-  void p32_kernel_launch_n##NN##p##PP(bool lv, bool rec, int grid, int threads, int smem,           \
+  const void* p32_kernel_ptr_n##NN##p##PP(int lv, bool rec);                                       \
+  void p32_kernel_launch_n##NN##p##PP(int lv, bool rec, int grid, int threads, int smem,           \
                                       cudaStream_t st, const P32Args& a);                          \
   int p32_phase_clocks_n##NN##p##PP(unsigned long long out[4], bool reset);
 RG_P32_DECLARE(1, 1) RG_P32_DECLARE(1, 2)
@@ -656,28 +726,39 @@ RG_P32_DECLARE(4, 1) RG_P32_DECLARE(4, 2)
 RG_P32_DECLARE(5, 1) RG_P32_DECLARE(5, 2)
 #undef RG_P32_DECLARE
 
-// The definitions of one (N, PPT)'s entry points (one use per translation unit).
+// The staged kernel exists at two paths a thread (at one, 64 registers spill); null otherwise.
+template <int N, int PPT>
+static const void* p32_staged() {
+  if constexpr (PPT == 2) return reinterpret_cast<const void*>(&phoenix32_kernel<N, P32_LV_STAGED, false, PPT>);
+  return nullptr;
+}
+
+// The definitions of one (N, PPT)'s entry points (one use per translation unit); records are written
+// by the unstaged kernels only.
 #define RG_P32_DEFINE(NN, PP)                                                                       \
-  const void* p32_kernel_ptr_n##NN##p##PP(bool lv, bool rec) {                                     \
-    if (lv) return rec ? reinterpret_cast<const void*>(&phoenix32_kernel<NN, true, true, PP>)      \
-                       : reinterpret_cast<const void*>(&phoenix32_kernel<NN, true, false, PP>);    \
-    return rec ? reinterpret_cast<const void*>(&phoenix32_kernel<NN, false, true, PP>)             \
-               : reinterpret_cast<const void*>(&phoenix32_kernel<NN, false, false, PP>);           \
+  const void* p32_kernel_ptr_n##NN##p##PP(int lv, bool rec) {                                      \
+    if (lv == P32_LV_STAGED) return p32_staged<NN, PP>();                                           \
+    if (lv) return rec ? reinterpret_cast<const void*>(&phoenix32_kernel<NN, P32_LV, true, PP>)    \
+                       : reinterpret_cast<const void*>(&phoenix32_kernel<NN, P32_LV, false, PP>);  \
+    return rec ? reinterpret_cast<const void*>(&phoenix32_kernel<NN, P32_FLAT, true, PP>)          \
+               : reinterpret_cast<const void*>(&phoenix32_kernel<NN, P32_FLAT, false, PP>);        \
   }                                                                                                 \
-  template <bool LV, bool REC>                                                                      \
+  template <int LV, bool REC>                                                                       \
   static void p32_go(int grid, int threads, int smem, cudaStream_t st, const P32Args& a) {          \
     phoenix32_kernel<NN, LV, REC, PP><<<grid, threads, smem, st>>>(                                 \
-        a.tr, a.tb, a.scen, a.scen32, a.S, a.Pb, a.TT, a.NNmax, a.stack_max, a.ln_ko, a.ln_cb,     \
-        a.ln_ki, a.path0, a.npaths, a.plan, a.partial, a.ko_steps, a.records);                      \
+        a.tr, a.tb, a.scen, a.scen32, a.S, a.Pb, a.TT, a.NNmax, a.stack_max, a.RT, a.n_surf,       \
+        a.ln_ko, a.ln_cb, a.ln_ki, a.path0, a.npaths, a.plan, a.partial, a.ko_steps, a.records);    \
   }                                                                                                 \
-  void p32_kernel_launch_n##NN##p##PP(bool lv, bool rec, int grid, int threads, int smem,           \
+  void p32_kernel_launch_n##NN##p##PP(int lv, bool rec, int grid, int threads, int smem,            \
                                       cudaStream_t st, const P32Args& a) {                         \
-    if (lv) {                                                                                       \
-      if (rec) p32_go<true, true>(grid, threads, smem, st, a);                                      \
-      else p32_go<true, false>(grid, threads, smem, st, a);                                         \
+    if (lv == P32_LV_STAGED) {                                                                      \
+      if constexpr (PP == 2) p32_go<P32_LV_STAGED, false>(grid, threads, smem, st, a);              \
+    } else if (lv) {                                                                                  \
+      if (rec) p32_go<P32_LV, true>(grid, threads, smem, st, a);                                    \
+      else p32_go<P32_LV, false>(grid, threads, smem, st, a);                                       \
     } else {                                                                                        \
-      if (rec) p32_go<false, true>(grid, threads, smem, st, a);                                     \
-      else p32_go<false, false>(grid, threads, smem, st, a);                                        \
+      if (rec) p32_go<P32_FLAT, true>(grid, threads, smem, st, a);                                  \
+      else p32_go<P32_FLAT, false>(grid, threads, smem, st, a);                                     \
     }                                                                                               \
   }                                                                                                 \
   int p32_phase_clocks_n##NN##p##PP(unsigned long long out[4], bool reset) { return p32_phase_clocks_tu(out, reset); }

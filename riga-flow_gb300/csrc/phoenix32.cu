@@ -10,7 +10,7 @@
 
 namespace rg {
 
-static const void* select_kernel(int n, bool lv, bool rec, int ppt) {
+static const void* select_kernel(int n, int lv, bool rec, int ppt) {
 #define RG_SEL(NN) return ppt == 2 ? p32_kernel_ptr_n##NN##p2(lv, rec) : p32_kernel_ptr_n##NN##p1(lv, rec);
   switch (n) {
     case 1: RG_SEL(1)
@@ -28,24 +28,36 @@ static const int kTileDepths[] = {24, 32, 48, 64, 80, 96, 128};
 
 // Shared-memory bytes of a tiled shape: Pb paths per tile at `ppt` paths per thread, `tt` steps per
 // tile.
-static uint32_t p32_smem(const Prepared& P, int Pb, int ppt, int tt) {
-  return p32_layout(P.n, Pb, tt, tt + P.stack_max, P.stack_max, ppt).total;
+static uint32_t p32_smem(const Prepared& P, int Pb, int ppt, int tt, int rt) {
+  return p32_layout(P.n, Pb, tt, tt + P.stack_max, P.stack_max, ppt, (uint32_t)(P.n_surf * rt * P.trade.gx)).total;
 }
 // Whether the shape fits in 227 KB of shared memory.
-static bool p32_fits(const Prepared& P, int Pb, int ppt, int tt) { return p32_smem(P, Pb, ppt, tt) <= 227u * 1024u; }
+static bool p32_fits(const Prepared& P, int Pb, int ppt, int tt, int rt) {
+  return p32_smem(P, Pb, ppt, tt, rt) <= 227u * 1024u;
+}
+// Steps per buffer that local-vol rows are staged by, most first.
+static const int kRowSteps[] = {32, 16, 8};
+// Whether a launch's local-vol rows may be staged at `ppt` paths per thread: rows of whole 16-byte words,
+// which bulk copies take, and the two-path kernel.
+static bool p32_stageable(const Prepared& P, int ppt) { return P.trade.has_lv && P.trade.gx % 2 == 0 && ppt == 2; }
 
 // Sets the block (Pb paths per tile), paths per thread and tile depth of a tiled shape, if its
 // threads and its layout fit.  The CTA has a thread per (scenario, ppt paths) and at least 512:
 // the ones without a scenario share generation and bridge, which at few scenarios take most of the
 // time (S = 1, 2^14 paths, 64 paths a tile: 0.17 ms with 512 threads, 0.25 with 128).
-static bool p32_set_shape(const Prepared& P, Fp32Shape& sh, int pb, int ppt, int tt) {
-  const int stepping = (P.n_scen * pb / ppt + 31) / 32 * 32;
-  if (pb < 32 || (pb & (pb - 1)) || stepping > p32_max_threads(P.n, ppt) || !p32_fits(P, pb, ppt, tt)) return false;
+// `rt`: steps of local-vol rows per staging buffer, which a further warp fills (0: rows gathered from
+// global memory).
+static bool p32_set_shape(const Prepared& P, Fp32Shape& sh, int pb, int ppt, int tt, int rt) {
+  const int stepping = (P.n_scen * pb / ppt + 31) / 32 * 32 + (rt ? 32 : 0);
+  if (pb < 32 || (pb & (pb - 1)) || stepping > p32_max_threads(P.n, ppt) || !p32_fits(P, pb, ppt, tt, rt) ||
+      (rt && !p32_stageable(P, ppt)))
+    return false;
+  sh.RT = rt;
   sh.Pb = pb;
   sh.ppt = ppt;
   sh.TT = tt;
   sh.threads = std::max(stepping, 512);
-  sh.smem = (int)p32_smem(P, pb, ppt, tt);
+  sh.smem = (int)p32_smem(P, pb, ppt, tt, rt);
   return true;
 }
 
@@ -56,14 +68,25 @@ static bool p32_set_shape(const Prepared& P, Fp32Shape& sh, int pb, int ppt, int
 // (at least 32) that still give every SM at most one: a tile's time hardly depends on its paths
 // (3 assets, 252 steps: 0.12 ms on 32 paths, 0.19 on 128, 0.29 on 256).  Then the deepest tile that
 // fits: phase changes cost more than occupancy gains (16 scenarios: 10.1 ms at 128 steps, 10.8 at 64,
-// 13.4 at 24).
+// 13.4 at 24).  Local-vol rows are staged when buffers of 32 steps fit beside that depth, or of 16 or 8
+// beside more than half of it.  Gathers in shared memory cost less latency than cached ones, which
+// counts at few warps: 4 scenarios of 3 assets, 756 steps 0.37 ms against 0.51; one to eight scenarios
+// at 4096 paths × 252 steps 0.06-0.08 against 0.10-0.12, 12 scenarios of one asset on 2^17 paths 0.83
+// against 1.21.  16 warps and 18 surfaces gain nothing: buffers of 8 steps beside half the depth
+// 10.08 ms against 10.04, 17 scenarios 2.98 against 2.92.
 static void formula_shape(const Prepared& P, Fp32Shape& sh, uint64_t npaths, int sm_count) {
   int pb = 256;
   while (pb > 32 && P.n_scen * pb / 2 > p32_max_threads(P.n, 2)) pb >>= 1;
   while (pb > 32 && (npaths + pb / 2 - 1) / (pb / 2) <= (uint64_t)sm_count) pb >>= 1;
+  const int nd = (int)(sizeof kTileDepths / sizeof kTileDepths[0]);
   for (; pb >= 32; pb >>= 1)
-    for (int i = (int)(sizeof kTileDepths / sizeof kTileDepths[0]) - 1; i >= 0; --i)
-      if (p32_set_shape(P, sh, pb, 2, kTileDepths[i])) return;
+    for (int i = nd - 1; i >= 0; --i)
+      if (p32_set_shape(P, sh, pb, 2, kTileDepths[i], 0)) {
+        for (int rt : kRowSteps)
+          for (int k = i; k >= 0 && (rt == 32 ? k == i : 2 * kTileDepths[k] > kTileDepths[i]); --k)
+            if (p32_set_shape(P, sh, pb, 2, kTileDepths[k], rt)) return;
+        return;
+      }
   raise(RG_ERR_GPU_ERROR, "phoenix32: the tile does not fit in shared memory");
 }
 
@@ -203,9 +226,10 @@ static void p32_set_attributes() {
   cuda_check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "smem opt-in");
   for (int ppt = 1; ppt <= 2; ++ppt)
     for (int n = 1; n <= RG_NMAX; ++n)
-      for (int lv = 0; lv < 2; ++lv)
-        for (int rec = 0; rec < 2; ++rec) {
-          const void* kr = select_kernel(n, lv != 0, rec != 0, ppt);
+      for (int lv = 0; lv < 3; ++lv)
+        for (int rec = 0; rec < (lv == P32_LV_STAGED ? 1 : 2); ++rec) {
+          const void* kr = select_kernel(n, lv, rec != 0, ppt);
+          if (!kr) continue;
           cuda_check(cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, optin),
                      "phoenix32 smem attribute");
           cuda_check(cudaFuncSetAttribute(kr, cudaFuncAttributePreferredSharedMemoryCarveout, 100),
@@ -214,9 +238,13 @@ static void p32_set_attributes() {
   done[dev] = 1;
 }
 
+static int p32_lv_kind(const Prepared& P, const Fp32Shape& sh) {
+  return !P.trade.has_lv ? P32_FLAT : (sh.RT ? P32_LV_STAGED : P32_LV);
+}
+
 // Grid of a tiled shape: as many CTAs as are resident on the SMs, at most one per tile.
 static int tiled_grid(const Prepared& P, const Fp32Shape& sh, uint64_t npaths, int sm_count) {
-  const void* k = select_kernel(P.n, P.trade.has_lv != 0, false, sh.ppt);
+  const void* k = select_kernel(P.n, p32_lv_kind(P, sh), false, sh.ppt);
   int per_sm = 0;
   cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, sh.threads, sh.smem),
              "phoenix32 occupancy");
@@ -250,16 +278,16 @@ uint64_t p32_chunks(uint64_t npaths) { return (npaths + 31) / 32; }
 
 // ---------------------------------------------------------------------- tiled-shape autotuner --
 namespace {
-// A tiled launch shape: paths per CTA tile, paths per thread, tile depth.
+// A tiled launch shape: paths per CTA tile, paths per thread, tile depth, steps per buffer of staged rows
+// (0: rows gathered from global memory; a forced shape's are).
 struct TiledKnobs {
-  int pb, ppt, tt;
-  bool operator==(const TiledKnobs& o) const { return pb == o.pb && ppt == o.ppt && tt == o.tt; }
+  int pb, ppt, tt, rt;
 };
 
 std::mutex g_tune_mu;
 std::map<std::vector<int64_t>, TiledKnobs> g_tuned;  // launch shape -> (block, paths per thread, tile depth)
 bool g_tune_enabled = true;
-TiledKnobs g_forced{0, 0, 0};  // the shape every tiled launch takes, or none (ppt 0); pb 0: the
+TiledKnobs g_forced{0, 0, 0, 0};  // the shape every tiled launch takes, or none (ppt 0); pb 0: the
                                // formula block
 
 
@@ -280,7 +308,7 @@ void p32_force_shape(int ppt, int tt, int pb) {
   for (int c : kTileDepths) plan = plan || c == tt;
   if (!plan) raise(RG_ERR_INVALID_ARGUMENT, "tiled shape: the tile depth must be one of the autotuner's candidates");
   std::lock_guard<std::mutex> lock(g_tune_mu);
-  g_forced = TiledKnobs{pb, ppt, tt};
+  g_forced = TiledKnobs{pb, ppt, tt, 0};
 }
 
 // Times every (block, paths per thread, tile depth) candidate on a prefix of the launch's paths and
@@ -297,7 +325,7 @@ Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenar
                                  P.trade.vr, P.trade.scrambler, P.trade.gx};
   auto apply = [&](TiledKnobs c, uint64_t paths) {
     Fp32Shape t = sh;
-    if (!p32_set_shape(P, t, c.pb, c.ppt, c.tt)) return sh;
+    if (!p32_set_shape(P, t, c.pb, c.ppt, c.tt, c.rt)) return sh;
     t.grid = tiled_grid(P, t, paths, sm_count);
     t.tuned = 1;
     return t;
@@ -305,7 +333,7 @@ Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenar
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     if (g_forced.ppt) {
-      Fp32Shape t = apply({g_forced.pb ? g_forced.pb : sh.Pb, g_forced.ppt, g_forced.tt}, npaths);
+      Fp32Shape t = apply({g_forced.pb ? g_forced.pb : sh.Pb, g_forced.ppt, g_forced.tt, 0}, npaths);
       if (!t.tuned) raise(RG_ERR_INVALID_ARGUMENT, "tiled shape: the forced tile does not fit in shared memory");
       return t;
     }
@@ -322,7 +350,8 @@ Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenar
     for (int ppt = 1; ppt <= 2; ++ppt)
       for (int tt : kTileDepths) {
         Fp32Shape c = sh;
-        if (p32_set_shape(P, c, pb, ppt, tt)) cand.push_back({pb, ppt, tt});
+        for (int rt : {0, 8, 16, 32})
+          if (p32_set_shape(P, c, pb, ppt, tt, rt)) cand.push_back({pb, ppt, tt, rt});
       }
   LaunchOut lo = out;  // the partial sums are overwritten by the real launch afterwards
   lo.ko_steps = nullptr;
@@ -368,10 +397,11 @@ void launch_phoenix32(const Prepared& P, const DevTables& tb, const DevScenario*
   if (sh.Pb < 32 || (sh.Pb & (sh.Pb - 1)) || sh.threads * sh.ppt < P.n_scen * sh.Pb || (sh.ppt != 1 && sh.ppt != 2) ||
       sh.threads > p32_max_threads(P.n, sh.ppt))
     raise(RG_ERR_GPU_ERROR, "phoenix32: invalid tile shape");
-  const bool lvk = P.trade.has_lv != 0;
-  const P32Args a{P.trade, tb, scen, scen32, P.n_scen, sh.Pb, sh.TT, NNmax, P.stack_max, ln_ko, ln_cb, ln_ki,
+  const P32Args a{P.trade, tb, scen, scen32, P.n_scen, sh.Pb, sh.TT, NNmax, P.stack_max, sh.RT, P.n_surf, ln_ko, ln_cb, ln_ki,
                   path0, npaths, plan, out.partial, out.ko_steps, out.records};
   const bool rec = out.records != nullptr;
+  // records come from the unstaged kernels (the layout is then larger than they need)
+  const int lvk = rec && sh.RT ? P32_LV : p32_lv_kind(P, sh);
 #define RG_GO(NN)                                                                         \
   if (sh.ppt == 2) p32_kernel_launch_n##NN##p2(lvk, rec, sh.grid, sh.threads, sh.smem, st, a); \
   else p32_kernel_launch_n##NN##p1(lvk, rec, sh.grid, sh.threads, sh.smem, st, a);

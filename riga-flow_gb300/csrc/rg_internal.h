@@ -254,6 +254,7 @@ void launch_phoenix64(const Prepared& P, const DevTables& tb, const DevScenario*
                       uint64_t path0, uint64_t npaths, const LaunchOut& out, cudaStream_t s);
 struct Fp32Shape {
   int Pb, TT, threads, grid, smem;
+  int RT;      // steps per buffer of staged local-vol rows of the tiled kernel (0: not staged)
   int ppt;     // paths per thread of the tiled kernel (1 or 2)
   int tuned;   // 1: Pb, ppt and TT came from the autotuner's cache (or were forced)
   int direct;  // 1: the per-thread kernel of phoenix32d.cu; then only grid and threads are used

@@ -570,3 +570,34 @@ def test_tiled_formula_shapes_price_identically(engine, n, paths):
     full = [bytes(r) for r in engine.price_scenarios_raw(req, scen)]
     for S in (1, 2, 3, 4, 5, 8, 9, 10, 16, 17, 20, 21, 25):
         assert [bytes(r) for r in engine.price_scenarios_raw(req, scen[:S])] == full[:S], S
+
+
+@pytest.mark.parametrize("n,gx", [(1, 24), (2, 40), (3, 25), (3, 64), (5, 40)])
+@pytest.mark.parametrize("steps", [1, 7, 33, 130, 300])
+def test_staged_local_vol_rows_price_identically(engine, n, gx, steps):
+    """Local-vol rows come from shared-memory buffers of a few steps where they fit (even grid widths)
+    and from global memory in a forced shape: the same bytes either way, for one set of surfaces and for
+    one set per scenario, at step counts around the buffers' and the time tiles' edges."""
+    lib = engine.lib
+    r = workloads.lv5_large(paths=2093, steps=steps)
+    r.trade = workloads.phoenix_trade(n, steps, 5.0 * steps / 1260)
+    r.local_vol, r.options = r.local_vol[:n], workloads.production_options(gx)
+    m = r.market
+    m.spots, m.vols, m.dividend_yields = m.spots[:n], m.vols[:n], m.dividend_yields[:n]
+    m.correlation = [row[:n] for row in m.correlation[:n]]
+    r.config.variance_reduction = VarianceReduction("sobol", n * steps)
+    for bumped in (0, 1):
+        scen = []
+        for k in range(5):
+            mk = copy.deepcopy(m)
+            mk.spots[k % n] *= 1.0 + 0.01 * k
+            mk.vols = [v + 0.01 * bumped * k for v in mk.vols]
+            scen.append((mk, [0.01 * bumped * k] * n))
+        for s in (scen[:1], scen):
+            got = [bytes(x) for x in engine.price_scenarios_raw(r, s)]
+            try:
+                abi.check(lib, lib.rg_set_tiled_shape(2, 24, 0))
+                want = [bytes(x) for x in engine.price_scenarios_raw(r, s)]
+            finally:
+                abi.check(lib, lib.rg_set_tiled_shape(0, 0, 0))
+            assert got == want
