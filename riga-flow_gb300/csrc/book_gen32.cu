@@ -115,7 +115,8 @@ __global__ void __launch_bounds__(32 * kGenWarps, 2) book_gen32_kernel(const __g
         for (uint32_t g = ga & ~gb; g; g &= g - 1u) a ^= __ldg(col + (size_t)(__ffs(g) - 1) * tb.sob_nq);
         for (uint32_t g = gb & ~ga; g; g &= g - 1u) b ^= __ldg(col + (size_t)(__ffs(g) - 1) * tb.sob_nq);
         hi[i] = make_uint2(a, b);
-        hi[hi_n + i] = make_uint2(a ^ __ldg(col + (size_t)ra * tb.sob_nq), b ^ __ldg(col + (size_t)rb * tb.sob_nq));
+        const uint32_t v4 = __ldg(col + (size_t)4 * tb.sob_nq);
+        hi[hi_n + i] = make_uint2(a ^ v4 ^ __ldg(col + (size_t)ra * tb.sob_nq), b ^ v4 ^ __ldg(col + (size_t)rb * tb.sob_nq));
       }
     }
     if (tid < nb) {
@@ -132,31 +133,41 @@ __global__ void __launch_bounds__(32 * kGenWarps, 2) book_gen32_kernel(const __g
       const uint2* hl = hi + (upper ? hi_n : 0) + (c0 - hi0) * U;
       const uint32_t* low = tb.sob_lut + (size_t)c0 * U * 32 + lane;
       const int items = nb * U;
-      auto draw = [&](int it, uint32_t l, auto shifted) {
-        const uint2 h = hl[it];
-        uint32_t xa = l ^ h.x, xb = l ^ h.y;
-        if constexpr (!decltype(shifted)::value) {
-          const uint64_t dim = (uint64_t)__ldg(tb.node_k + c0 + it / U) * U + it % U;
-          xa = rg_owen(xa, dim, A.gen.seed);
-          xb = rg_owen(xb, dim, A.gen.seed);
+      // the normals of `K` items, kGenWarps apart
+      auto draw = [&](int it, auto shifted, auto count) {
+        constexpr int K = decltype(count)::value;
+        uint32_t l[K], xa[K], xb[K];
+#pragma unroll
+        for (int i = 0; i < K; ++i) l[i] = __ldg(low + (it + i * kGenWarps) * 32);
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+          const uint2 h = hl[it + i * kGenWarps];
+          xa[i] = l[i] ^ h.x;
+          xb[i] = l[i] ^ h.y;
+          if constexpr (!decltype(shifted)::value) {
+            const int e = it + i * kGenWarps;
+            const uint64_t dim = (uint64_t)__ldg(tb.node_k + c0 + e / U) * U + e % U;
+            xa[i] = rg_owen(xa[i], dim, A.gen.seed);
+            xb[i] = rg_owen(xb[i], dim, A.gen.seed);
+          }
         }
-        const float2 v = rg_probit32x2(xa, xb);
-        z[it * kGenPaths + lane] = v.x;
-        z[it * kGenPaths + 32 + lane] = v.y;
+        float2 v[K];
+        rg_probit32x2(xa, xb, v);
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+          z[(it + i * kGenWarps) * kGenPaths + lane] = v[i].x;
+          z[(it + i * kGenWarps) * kGenPaths + 32 + lane] = v[i].y;
+        }
       };
+      using One = std::integral_constant<int, 1>;
       if (shift) {
         constexpr int kI = 5;  // items in flight
         int it = warp;
-        for (; it + (kI - 1) * kGenWarps < items; it += kI * kGenWarps) {
-          uint32_t l[kI];
-#pragma unroll
-          for (int i = 0; i < kI; ++i) l[i] = __ldg(low + (it + i * kGenWarps) * 32);
-#pragma unroll
-          for (int i = 0; i < kI; ++i) draw(it + i * kGenWarps, l[i], std::true_type{});
-        }
-        for (; it < items; it += kGenWarps) draw(it, __ldg(low + it * 32), std::true_type{});
+        for (; it + (kI - 1) * kGenWarps < items; it += kI * kGenWarps)
+          draw(it, std::true_type{}, std::integral_constant<int, kI>{});
+        for (; it < items; it += kGenWarps) draw(it, std::true_type{}, One{});
       } else {
-        for (int it = warp; it < items; it += kGenWarps) draw(it, __ldg(low + it * 32), std::false_type{});
+        for (int it = warp; it < items; it += kGenWarps) draw(it, std::false_type{}, One{});
       }
     } else {
       for (int it = warp; it < nb * U; it += kGenWarps) {
@@ -255,8 +266,7 @@ void launch_book_gen32(const DevTrade& gen, const DevTables& tb, const float* L3
 // point is n1 + j, n1 = a + o with a a multiple of 32.  Gray codes are linear over XOR, so for
 // o + j < 32 x(n1 + j) = X(gray(a)) ^ X(gray(o + j)), and otherwise x = X(gray(a + 32)) ^
 // X(gray(o + j - 32)) with X(gray(a + 32)) = X(gray(a)) ^ v[4] ^ v[ctz(a/32 + 1) + 5]; lut holds the
-// lane's low-bit term X(gray((o + j) mod 32)) — with v[4] for the upper lanes and the digital shift
-// folded in — and the kernels add the 32-path group's high-bit terms.  A CTA per 32 dimensions,
+// lane's low-bit term X(gray((o + j) mod 32)) with the digital shift folded in, and the kernels add the 32-path group's high-bit terms.  A CTA per 32 dimensions,
 // thread (k, i) on direction k, then lane k, of dimension i.  (Built on the host the tables took
 // 1.1 MB of upload per 1,000 steps of 3 assets, and 1 ms for a seed not seen before.)
 __global__ void __launch_bounds__(1024) sobol_lut_kernel(DevTrade tr, DevTables tb, int n, int nq, uint32_t o,
@@ -272,7 +282,6 @@ __global__ void __launch_bounds__(1024) sobol_lut_kernel(DevTrade tr, DevTables 
 #pragma unroll
     for (int b = 0; b < 5; ++b)
       if ((g >> b) & 1u) x ^= v[i][b];
-    if (o + k >= 32u) x ^= v[i][4];
     lut[(size_t)q * 32 + k] = x;
   }
   if (blockIdx.x * 32 + k < nq) st[(size_t)i * nq + blockIdx.x * 32 + k] = v[k][i];

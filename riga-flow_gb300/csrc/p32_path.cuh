@@ -1,9 +1,32 @@
-// p32_path.cuh — the path close shared by the FP32 kernels (phoenix32.cu, phoenix32d.cu).
+// p32_path.cuh — what the FP32 kernels (phoenix32.cu, phoenix32d.cu) share: path values in packed pairs,
+// the Phoenix state machine and the path close.
 #pragma once
 #include "rg_common.cuh"
 #include "rg_packed.cuh"
 
 namespace rg {
+
+// PPT path values of one thread: a float (one path per thread) or a float pair (two), so that the
+// stepping arithmetic of two paths issues as one packed FP32x2 instruction (__ffma2_rn etc.).
+template <int PPT> struct PVec;
+template <> struct PVec<1> {
+  float v[1];
+  __device__ __forceinline__ static PVec splat(float a) { return {{a}}; }
+  __device__ __forceinline__ static PVec fma(PVec a, PVec b, PVec c) { return {{fmaf(a.v[0], b.v[0], c.v[0])}}; }
+  __device__ __forceinline__ static PVec fma_rd(PVec a, PVec b, PVec c) { return {{__fmaf_rd(a.v[0], b.v[0], c.v[0])}}; }
+  __device__ __forceinline__ static PVec add(PVec a, PVec b) { return {{a.v[0] + b.v[0]}}; }
+  __device__ __forceinline__ static PVec mul(PVec a, PVec b) { return {{a.v[0] * b.v[0]}}; }
+};
+template <> struct alignas(8) PVec<2> {
+  float v[2];
+  __device__ __forceinline__ static PVec splat(float a) { return {{a, a}}; }
+  __device__ __forceinline__ static PVec from(float2 f) { return {{f.x, f.y}}; }
+  __device__ __forceinline__ float2 f2() const { return make_float2(v[0], v[1]); }
+  __device__ __forceinline__ static PVec fma(PVec a, PVec b, PVec c) { return from(__ffma2_rn(a.f2(), b.f2(), c.f2())); }
+  __device__ __forceinline__ static PVec fma_rd(PVec a, PVec b, PVec c) { return from(__ffma2_rd(a.f2(), b.f2(), c.f2())); }
+  __device__ __forceinline__ static PVec add(PVec a, PVec b) { return from(__fadd2_rn(a.f2(), b.f2())); }
+  __device__ __forceinline__ static PVec mul(PVec a, PVec b) { return from(__fmul2_rn(a.f2(), b.f2())); }
+};
 
 // The Phoenix state of one FP32 path of one scenario.
 struct P32Phoenix {
@@ -49,6 +72,23 @@ __device__ __forceinline__ void p32_phoenix_step(P32Phoenix& st, uint32_t fl, in
     } else if (tr.memory) {
       ++st.unpaid;
     }
+  }
+}
+
+// The knock-out branch of the Phoenix state machine (p32_phoenix_step) for one live path.
+template <bool REC>
+__device__ __forceinline__ void p32_knock_out(P32Phoenix& st, uint32_t fl, int t, const DevTrade& tr,
+                                              const DevTables& tb, const float* __restrict__ df, int period) {
+  st.alive = false;
+  st.ko_step = t;
+  const float due = (fl & STEP_FIXED_DUE) ? tr.coupon_f : (float)st.qual * __ldg(tb.accr_f + period);
+  const float carry = due > 0.0f ? (float)st.unpaid * tr.coupon_f : 0.0f;
+  if (due + carry > 0.0f) {
+    const float d = __ldg(df + t);
+    st.cpv = fmaf(due, d, st.cpv);
+    st.mpv = fmaf(carry, d, st.mpv);
+    st.received = true;
+    if (REC) ++st.paid;
   }
 }
 

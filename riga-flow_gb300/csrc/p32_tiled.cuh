@@ -77,47 +77,10 @@ __host__ __device__ inline P32Layout p32_layout(int N, int Pb, int TT, int NNmax
   put(L.plan, (uint32_t)(NNmax + (NNmax + 1) + (TT + 1) + stack_max) * 4u);
   put(L.z, zb);
   put(L.dw, (uint32_t)TT * (uint32_t)p32_dwstep(N, Pb, ppt) * 4u);  // dW[step][factor][path]
-  put(L.rows, 2u * row_words * 8u);                                  // [buffer][surface][step][grid point]
+  put(L.rows, 2u * row_words * 8u);                                  // [buffer][step][surface][grid point]
   put(L.bars, row_words ? 32u : 0u);                                 // full[2], empty[2]
   L.total = o;
   return L;
-}
-
-// PPT path values of one thread: a float (one path per thread) or a float pair (two), so that the
-// stepping arithmetic of two paths issues as one packed FP32x2 instruction (__ffma2_rn etc.).
-template <int PPT> struct PVec;
-template <> struct PVec<1> {
-  float v[1];
-  __device__ __forceinline__ static PVec splat(float a) { return {{a}}; }
-  __device__ __forceinline__ static PVec fma(PVec a, PVec b, PVec c) { return {{fmaf(a.v[0], b.v[0], c.v[0])}}; }
-  __device__ __forceinline__ static PVec fma_rd(PVec a, PVec b, PVec c) { return {{__fmaf_rd(a.v[0], b.v[0], c.v[0])}}; }
-  __device__ __forceinline__ static PVec add(PVec a, PVec b) { return {{a.v[0] + b.v[0]}}; }
-};
-template <> struct PVec<2> {
-  float v[2];
-  __device__ __forceinline__ static PVec splat(float a) { return {{a, a}}; }
-  __device__ __forceinline__ static PVec from(float2 f) { return {{f.x, f.y}}; }
-  __device__ __forceinline__ float2 f2() const { return make_float2(v[0], v[1]); }
-  __device__ __forceinline__ static PVec fma(PVec a, PVec b, PVec c) { return from(__ffma2_rn(a.f2(), b.f2(), c.f2())); }
-  __device__ __forceinline__ static PVec fma_rd(PVec a, PVec b, PVec c) { return from(__ffma2_rd(a.f2(), b.f2(), c.f2())); }
-  __device__ __forceinline__ static PVec add(PVec a, PVec b) { return from(__fadd2_rn(a.f2(), b.f2())); }
-};
-
-// The knock-out branch of the Phoenix state machine (p32_phoenix_step) for one live path.
-template <bool REC>
-__device__ __forceinline__ void p32_knock_out(P32Phoenix& st, uint32_t fl, int t, const DevTrade& tr,
-                                              const DevTables& tb, const float* __restrict__ df, int period) {
-  st.alive = false;
-  st.ko_step = t;
-  const float due = (fl & STEP_FIXED_DUE) ? tr.coupon_f : (float)st.qual * __ldg(tb.accr_f + period);
-  const float carry = due > 0.0f ? (float)st.unpaid * tr.coupon_f : 0.0f;
-  if (due + carry > 0.0f) {
-    const float d = __ldg(df + t);
-    st.cpv = fmaf(due, d, st.cpv);
-    st.mpv = fmaf(carry, d, st.mpv);
-    st.received = true;
-    if (REC) ++st.paid;
-  }
 }
 
 // Phase clocks, a build option (RG_PHASE_CLOCKS, see riga_gb300/build.py): thread 0 of every CTA
@@ -211,24 +174,26 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
   uint32_t* s_pstk = reinterpret_cast<uint32_t*>(s_poff + TT + 1);
   float* Z = reinterpret_cast<float*>(smem_raw + L.z);
   float* dW = reinterpret_cast<float*>(smem_raw + L.dw);
-  const float2* s_rows = reinterpret_cast<const float2*>(smem_raw + L.rows);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + L.bars);
   uint64_t* empty = full + 2;
 
+  // the warp's number by a shuffle, which makes what it decides warp-uniform to the compiler: row pointers,
+  // schedule words and loop counters then live in uniform registers
+  const int wid = __shfl_sync(0xffffffffu, tid >> 5, 0);
   // stepping: thread tid serves scenario s and paths pl0 .. pl0 + PPT - 1 of each tile
   const int tps = Pb / PPT;  // threads per scenario
   const int s = tid / tps, pl0 = (tid % tps) * PPT;
   const bool lane_ok = s < S;
   const int ss = lane_ok ? s : 0;
   // a warp whose first thread has no scenario (padded scenario slots) skips the stepping phase
-  const bool warp_on = ((tid & ~31) / tps) < S;
+  const bool warp_on = wid * 32 / tps < S;
   const int gx = tr.gx;
   const V gxm1 = V::splat((float)(gx - 1));
   const V two23 = V::splat(8388608.0f);
   const V nhdt = V::splat(tr.neg_half_dt_f);
   // generation and bridge: warp-wide items over 32-path groups of the tile
   const int ngrp = Pb >> 5, lg_ngrp = lg_pb - 5;
-  const int nwarp = (int)(blockDim.x >> 5), wid = tid >> 5;
+  const int nwarp = (int)(blockDim.x >> 5);
 
   // scenario constants in registers: the Cholesky factor, drifts, flat vols and the per-asset
   // local-vol lookup constants (a_u/(gx-1), inv_h/(gx-1), row offset - 0x4B000000, x0)
@@ -249,9 +214,8 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
       sig[f] = V::splat(s3.sig[f]);
       lva[f] = s3.a_u[f] * inv_gxm1;
       lvb[f] = s3.inv_h[f] * inv_gxm1;
-      // staged: the surface's first row in a buffer
-      lvo[f] = (LV == P32_LV_STAGED ? (uint32_t)(s3.surf_off[f] / (T * gx)) * (uint32_t)(RT * gx)
-                                    : (uint32_t)s3.surf_off[f]) - 0x4B000000u;
+      // byte offset of the surface's row, less the grid index's bias 0x4B000000 in bytes (modulo 2^32)
+      lvo[f] = ((uint32_t)s3.surf_off[f] - 0x4B000000u) * 8u;
       x0[f] = s3.x0[f];
     }
   }
@@ -262,7 +226,7 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
   const bool sob_lut = tr.vr == RG_VR_SOBOL && tb.sob_lut != nullptr && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o;
   const bool upper = (uint32_t)tb.sob_lut_o + (uint32_t)lane >= 32u;
   // staged rows: RT steps of every surface at a time in one of two buffers.  The first warp past the
-  // stepping ones fills them by bulk copies (one per surface) counted on a buffer's "full" barrier; every
+  // stepping ones fills them by bulk copies counted on a buffer's "full" barrier; every
   // stepping warp releases a buffer on its "empty" barrier.  (Filled by a stepping warp they cost 1.8 us
   // a buffer at 3 surfaces and 3.8 at 18: the whole CTA waits while that warp waits and copies.)  The
   // first two buffers of a time tile are filled while its normals are generated.  Waits are bounded: one
@@ -289,11 +253,12 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
       stuck = true;
       return;
     }
-    if (lane == 0) mbar_expect_tx(&full[b], (uint32_t)(n_surf * steps * gx) * 8u);
+    if (lane == 0) {
+      const uint32_t bytes = (uint32_t)(n_surf * steps * gx) * 8u;
+      mbar_expect_tx(&full[b], bytes);
+      bulk_g2s(smem_raw + L.rows + b * row_words * 8u, tb.lv_rows + (size_t)t * (n_surf * gx), bytes, &full[b]);
+    }
     __syncwarp();
-    float2* dst = reinterpret_cast<float2*>(smem_raw + L.rows) + b * row_words;
-    for (int k = lane; k < n_surf; k += 32)
-      bulk_g2s(dst + k * RT * gx, tb.lv_rows + ((size_t)k * T + t) * gx, (uint32_t)(steps * gx) * 8u, &full[b]);
   };
   RG_PHASE_BEGIN();
   const uint64_t ntiles = (npaths + Pb - 1) / Pb;
@@ -374,7 +339,8 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
             uint32_t h = 0;
             for (uint32_t g = ga; g; g &= g - 1u) h ^= __ldg(tb.sob_t + (size_t)(__ffs(g) - 1) * tb.sob_nq + q);
             s_hq[(hh * 2) * hs + ql] = h;
-            s_hq[(hh * 2 + 1) * hs + ql] = h ^ __ldg(tb.sob_t + (size_t)cw * tb.sob_nq + q);
+            s_hq[(hh * 2 + 1) * hs + ql] =
+                h ^ __ldg(tb.sob_t + (size_t)4 * tb.sob_nq + q) ^ __ldg(tb.sob_t + (size_t)cw * tb.sob_nq + q);
           }
         }
         __syncthreads();
@@ -395,14 +361,20 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
             jj[u] = it >> lg_ngrp;
             hh[u] = it & (ngrp - 1);
           }
-          // the normals of the items' points into their Z rows, two at a time
+          // the normals of the items' points into their Z rows
           auto store_normals = [&](const uint32_t (&xs)[kGB * N]) {
+            constexpr int kP = kGB * N / 2;
+            uint32_t xa[kP], xb[kP];
+            float2 z[kP];
 #pragma unroll
-            for (int i = 0; i < kGB * N; i += 2) {
-              const float2 z = rg_probit32x2(xs[i], xs[i + 1]);
-              Z[(size_t)jj[i / N] * zs + i % N * (Pb + 4) + (hh[i / N] << 5) + lane] = z.x;
-              Z[(size_t)jj[(i + 1) / N] * zs + (i + 1) % N * (Pb + 4) + (hh[(i + 1) / N] << 5) + lane] = z.y;
+            for (int i = 0; i < kP; ++i) {
+              xa[i] = xs[2 * i];
+              xb[i] = xs[2 * i + 1];
             }
+            rg_probit32x2(xa, xb, z);
+#pragma unroll
+            for (int i = 0; i < kGB * N; ++i)
+              Z[(size_t)jj[i / N] * zs + i % N * (Pb + 4) + (hh[i / N] << 5) + lane] = i % 2 ? z[i / 2].y : z[i / 2].x;
           };
           uint32_t xs[kGB * N];
           if (lut_tile) {
@@ -525,8 +497,11 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
         // one Euler step of every asset (correlated increment, local-vol lookup, log-space update);
         // returns the worst-of log performance of each path after the step
         auto euler = [&](int tt, float (&wmin)[PPT]) {
-          // the step's row within a surface (staged: within the buffer of steps from sub0)
-          const int tg = LV == P32_LV_STAGED ? (int)((use & 1u) * row_words) + (tt - sub0) * gx : (t0 + tt) * gx;
+          // the step's rows (staged: in the buffer of steps from sub0)
+          const char* rows =
+              LV == P32_LV_STAGED
+                  ? reinterpret_cast<const char*>(smem_raw) + L.rows + ((use & 1u) * RT + (tt - sub0)) * n_surf * gx * 8
+                  : reinterpret_cast<const char*>(tb.lv_rows + (size_t)(t0 + tt) * (n_surf * gx));
           V d[N], y[N];
 #pragma unroll
           for (int f = 0; f < N; ++f) {
@@ -557,8 +532,9 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
               const V fl = V::fma_rd(u01, gxm1, two23);
 #pragma unroll
               for (int j = 0; j < PPT; ++j) {
-                const uint32_t idx = lvo[f] + (uint32_t)tg + (uint32_t)__float_as_int(fl.v[j]);
-                const float2 r = LV == P32_LV_STAGED ? s_rows[idx] : __ldg(tb.lv_rows + idx);
+                const uint32_t off = (uint32_t)__float_as_int(fl.v[j]) * 8u + lvo[f];
+                const float2* cell = reinterpret_cast<const float2*>(rows + off);
+                const float2 r = LV == P32_LV_STAGED ? *cell : __ldg(cell);
                 sg.v[j] = fmaf(u01.v[j], r.y, r.x);
               }
             } else {

@@ -258,13 +258,10 @@ static int tiled_grid(const Prepared& P, const Fp32Shape& sh, uint64_t npaths, i
 Fp32Shape phoenix32_shape(const Prepared& P, const DevTables& tb, uint64_t path0, uint64_t npaths, int sm_count) {
   Fp32Shape sh{};
   if (P.n_scen > 32) raise(RG_ERR_INVALID_ARGUMENT, "at most 32 scenarios per fused launch");
-  if (p32_direct(P, npaths, tb.sob_lut && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o)) {
+  const bool lut = tb.sob_lut && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o;
+  if (p32_direct(P, npaths, lut)) {
     // nothing for the scenarios to share: the per-thread kernel without shared-memory tiles
-    sh.direct = 1;
-    sh.threads = 256;
-    sh.ppt = 1;
-    sh.grid = phoenix32d_grid(P, npaths, sm_count);
-    sh.smem = P.stack_max * P.n * 256 * (int)sizeof(float);  // the bridge stacks (dynamic)
+    phoenix32d_shape(P, npaths, lut, sm_count, sh);
     return sh;
   }
   formula_shape(P, sh, npaths, sm_count);
@@ -385,7 +382,7 @@ void launch_phoenix32(const Prepared& P, const DevTables& tb, const DevScenario*
                       const DevScen32* scen32, uint64_t path0, uint64_t npaths, const Fp32Shape& sh,
                       const LaunchOut& out, cudaStream_t st) {
   if (sh.direct) {
-    launch_phoenix32d(P, tb, scen, scen32, path0, npaths, sh.grid, out, st);
+    launch_phoenix32d(P, tb, scen32, path0, npaths, sh, out, st);
     return;
   }
   const float ln_ko = (float)P.ln_ko, ln_cb = (float)P.ln_cb, ln_ki = (float)P.ln_ki;

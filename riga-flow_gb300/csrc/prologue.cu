@@ -169,7 +169,9 @@ __global__ void calibrate_kernel(const CalibJob* __restrict__ jobs) {
 }
 
 // One CTA per (surface, step): the FP64 row sigma(step·dt, ·) of the surface, linear in tenor
-// (riga-market/src/lib.rs:345-364), stored as FP32 lines of its cells in the grid position.
+// (riga-market/src/lib.rs:345-364), stored as FP32 lines of its cells in the grid position.  The rows
+// of a step lie together, rows[step][surface][cell]: a lookup is a 32-bit offset from the step's rows,
+// and the rows of consecutive steps are one contiguous copy.
 __global__ void lvrows_kernel(const double* __restrict__ lv_v, const int32_t* __restrict__ cell_off,
                               const int32_t* __restrict__ surf_asset, const int2* __restrict__ lv_ti,
                               const double* __restrict__ lv_tw, int T, int gx, float2* __restrict__ rows) {
@@ -179,7 +181,7 @@ __global__ void lvrows_kernel(const double* __restrict__ lv_v, const int32_t* __
   const double wt = lv_tw[f * T + t];
   const double* v0 = lv_v + cell_off[sfc] + ti.x * gx;
   const double* v1 = lv_v + cell_off[sfc] + ti.y * gx;
-  float2* out = rows + ((size_t)sfc * T + t) * gx;
+  float2* out = rows + ((size_t)t * gridDim.x + sfc) * gx;
   // cell j as a line in the grid position u in [0, 1] (u·(gx - 1) = j at node j):
   // v(u) = v_j + (u·(gx - 1) - j)·(v_{j+1} - v_j) = c_j + u·d_j, with d = 0 on the last node, so
   // that a lookup is one FMA on the saturated position (flat beyond the grid)

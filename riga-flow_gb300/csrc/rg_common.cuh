@@ -167,7 +167,12 @@ __device__ __forceinline__ uint32_t rg_warp_sobol(const uint32_t* __restrict__ r
   return d;
 }
 
-// min of three (one instruction from sm_100 on).
+// max and min of three (one instruction from sm_100 on).
+__device__ __forceinline__ float rg_max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 __device__ __forceinline__ float rg_min3(float a, float b, float c) {
   float d;
   asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -213,11 +218,12 @@ __device__ __forceinline__ double rg_probit64(double p) {
 // 1.15e-9.
 // -ln(a) for a normal a by the hardware's base-2 logarithm (flush-to-zero form: no scaling of
 // subnormals, three instructions of the general form; the arguments here are at least 2e-12).
-__device__ __forceinline__ float rg_neg_ln(float a) {
+__device__ __forceinline__ float rg_lg2(float a) {
   float l;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(a));
-  return l * -0.6931471805599453f;
+  return l;
 }
+__device__ __forceinline__ float rg_neg_ln(float a) { return rg_lg2(a) * -0.6931471805599453f; }
 // The tail polynomial, w >= 5.
 __device__ __forceinline__ float rg_ninv32_tail(float w) {
   const float v = sqrtf(w) - 3.716110200f;

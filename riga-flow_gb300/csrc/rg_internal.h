@@ -83,7 +83,7 @@ struct DevScen32 {
   float sig[RG_NMAX];     // flat vol
   float a_u[RG_NMAX];     // (ln initial_spot - log_lo) / h
   float inv_h[RG_NMAX];   // 1 / h on the Dupire log-strike axis
-  int32_t surf_off[RG_NMAX];  // first FP32 step row of the scenario's surface: surface·T·gx
+  int32_t surf_off[RG_NMAX];  // the scenario's surface within a step's FP32 rows: surface·gx
   float L[RG_NMAX * RG_NMAX]; // the scenario's Cholesky factor rounded to FP32 (written by cholesky_kernel)
 };
 
@@ -261,9 +261,10 @@ struct Fp32Shape {
 };
 // A single scenario runs on the direct kernel (phoenix32d.cu) from a path count that fills the GPU with
 // one path per thread.  Where the two kernels cross was measured at 252 steps: on digitally shifted
-// Sobol points from the tables (`lut`) 2^16 paths for one asset (0.147 ms against the tiled kernel's
-// 0.151), 49,152 for two, 2^15 for three (0.20 against 0.21 flat, 0.24 against 0.27 local vol) and
-// 24,576 for four or five (2^15 paths: 0.31 against 0.46); lanes that cost more per normal spread it
+// Sobol points from the tables (`lut`) 2^16 paths for one asset (local vol 0.178 ms; the tiled kernel
+// 0.174 on 49,152), 49,152 for two (0.18 ms; the tiled kernel 0.15 on 2^15), 2^15 for three (0.18 flat
+// and 0.22 local vol; the tiled kernel 0.21 and 0.24 on 24,576) and 24,576 for four or five (5 assets
+// 0.28 against 0.46 on 2^15); lanes that cost more per normal spread it
 // over more threads in the tiled kernel, which keeps them up to 3·2^16 paths (1-3 assets) or 2^16.
 inline bool p32_direct(const Prepared& P, uint64_t npaths, bool lut) {
   const int n = P.n;
@@ -271,9 +272,17 @@ inline bool p32_direct(const Prepared& P, uint64_t npaths, bool lut) {
   const uint64_t from = !cheap ? (n >= 4 ? 65536 : 196608) : (n == 1 ? 65536 : (n == 2 ? 49152 : (n == 3 ? 32768 : 24576)));
   return P.n_scen == 1 && npaths >= from;
 }
-int phoenix32d_grid(const Prepared& P, uint64_t npaths, int sm_count);
-void launch_phoenix32d(const Prepared& P, const DevTables& tb, const DevScenario* scen, const DevScen32* scen32,
-                       uint64_t path0, uint64_t npaths, int grid, const LaunchOut& out, cudaStream_t st);
+// Paths per thread of a direct launch: two from 114,688 paths on digitally shifted Sobol points from the
+// tables, else one.  Below, half the warps leave latency uncovered (98,304 paths × 252 steps: 3 assets
+// 0.278 ms on two, 0.270 on one; 5 assets 0.42, 0.39; on 131,072 0.276, 0.348 and 0.425, 0.559).
+inline int p32_direct_ppt(const Prepared& P, uint64_t npaths, bool lut) {
+  if (!lut || P.trade.scrambler != RG_SCRAMBLE_DIGITAL_SHIFT) return 1;
+  return npaths >= 114688 ? 2 : 1;
+}
+// Sets a direct launch's shape (threads, grid, shared memory, paths per thread).
+void phoenix32d_shape(const Prepared& P, uint64_t npaths, bool lut, int sm_count, Fp32Shape& sh);
+void launch_phoenix32d(const Prepared& P, const DevTables& tb, const DevScen32* scen32, uint64_t path0,
+                       uint64_t npaths, const Fp32Shape& sh, const LaunchOut& out, cudaStream_t st);
 // `tb`, `path0`: whether the launch draws its points from staged Sobol tables.
 Fp32Shape phoenix32_shape(const Prepared& P, const DevTables& tb, uint64_t path0, uint64_t npaths, int sm_count);
 // Rows of the FP32 kernels' partial sums partial[chunk][scenario][RG_ACC]: one per 32 paths.

@@ -601,3 +601,32 @@ def test_staged_local_vol_rows_price_identically(engine, n, gx, steps):
             finally:
                 abi.check(lib, lib.rg_set_tiled_shape(0, 0, 0))
             assert got == want
+
+
+@pytest.mark.parametrize("n,lv", [(1, True), (2, False), (3, True), (4, False), (5, True)])
+@pytest.mark.parametrize("steps", [1, 2, 31, 64, 131])
+def test_two_path_direct_kernel_agrees(engine, n, lv, steps):
+    """From 114,688 paths a thread of the direct kernel walks two paths 32 apart: the same bytes as the
+    tiled kernel (the scenario twice) on ragged path counts, at every kind of offset within the 32-point
+    blocks, with bridge stacks within its fast slots and beyond; and the same path records as launches of
+    half as many paths, which run one path a thread."""
+    r = workloads.lv5_large(paths=114688, steps=steps)
+    r.trade = workloads.phoenix_trade(n, steps, 5.0 * steps / 1260)
+    r.local_vol, r.options = (r.local_vol[:n] if lv else None), workloads.production_options(40 if lv else 0)
+    m = r.market
+    m.spots, m.vols, m.dividend_yields = m.spots[:n], m.vols[:n], m.dividend_yields[:n]
+    m.correlation = [row[:n] for row in m.correlation[:n]]
+    r.config.variance_reduction = VarianceReduction("sobol", n * steps)
+    for first, paths in ((0, 114688), (31, 114688 + 33), (5, 114688 + 63), (32, 131072 + 1)):
+        r.options.first_path, r.config.paths = first, paths
+        one = engine.price_raw(r)
+        assert engine.last_timing().tile_steps == 0
+        two = engine.price_scenarios_raw(r, [(m, None)] * 2)
+        assert engine.last_timing().tile_steps > 0
+        assert bytes(one) == bytes(two[0])
+    r.options.first_path = 0
+    if steps == 31:
+        whole, low, high = (np.ctypeslib.as_array(engine.run_paths_raw(r, first, count))
+                            for first, count in ((7, 114690), (7, 57345), (57352, 57345)))
+        for field in whole.dtype.names:
+            np.testing.assert_array_equal(whole[field], np.concatenate([low[field], high[field]]))
