@@ -28,6 +28,15 @@ template <> struct alignas(8) PVec<2> {
   __device__ __forceinline__ static PVec mul(PVec a, PVec b) { return from(__fmul2_rn(a.f2(), b.f2())); }
 };
 
+// &p[i] as one 64-bit multiply-add, which becomes two shift-adds; spelt in C++, the compiler forms a 32-bit
+// offset first and spends three instructions (2^21 paths × 1260 steps of 5 assets 28.5 -> 27.7 ms, 16
+// scenarios of 3 assets on 2^18 paths × 756 steps 9.95 -> 9.88; with the size in a register 28.8 and 10.4).
+__device__ __forceinline__ const float2* p32_at(const float2* p, int32_t i) {
+  uint64_t r;
+  asm("mad.wide.s32 %0, %1, 8, %2;" : "=l"(r) : "r"(i), "l"(reinterpret_cast<uint64_t>(p)));
+  return reinterpret_cast<const float2*>(r);
+}
+
 // The Phoenix state of one FP32 path of one scenario.
 struct P32Phoenix {
   bool alive = true, received = false;

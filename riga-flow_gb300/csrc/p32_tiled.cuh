@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
   // local-vol lookup constants (a_u/(gx-1), inv_h/(gx-1), row offset - 0x4B000000, x0)
   V Lf[N * (N + 1) / 2], mu[N], sig[N];
   float lva[N], lvb[N], x0[N];
-  uint32_t lvo[N];
+  int32_t lvo[N];
   {
     const DevScen32& s3 = scen32[ss];
     const float inv_gxm1 = 1.0f / (float)(gx - 1);
@@ -214,8 +214,7 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
       sig[f] = V::splat(s3.sig[f]);
       lva[f] = s3.a_u[f] * inv_gxm1;
       lvb[f] = s3.inv_h[f] * inv_gxm1;
-      // byte offset of the surface's row, less the grid index's bias 0x4B000000 in bytes (modulo 2^32)
-      lvo[f] = ((uint32_t)s3.surf_off[f] - 0x4B000000u) * 8u;
+      lvo[f] = s3.surf_off[f] - 0x4B000000;  // less the bias of the grid index
       x0[f] = s3.x0[f];
     }
   }
@@ -498,10 +497,8 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
         // returns the worst-of log performance of each path after the step
         auto euler = [&](int tt, float (&wmin)[PPT]) {
           // the step's rows (staged: in the buffer of steps from sub0)
-          const char* rows =
-              LV == P32_LV_STAGED
-                  ? reinterpret_cast<const char*>(smem_raw) + L.rows + ((use & 1u) * RT + (tt - sub0)) * n_surf * gx * 8
-                  : reinterpret_cast<const char*>(tb.lv_rows + (size_t)(t0 + tt) * (n_surf * gx));
+          const uint32_t srows = (uint32_t)L.rows + ((use & 1u) * RT + (tt - sub0)) * (uint32_t)(n_surf * gx) * 8u;
+          const float2* grows = tb.lv_rows + (size_t)(t0 + tt) * (n_surf * gx);
           V d[N], y[N];
 #pragma unroll
           for (int f = 0; f < N; ++f) {
@@ -530,11 +527,15 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
 #pragma unroll
               for (int j = 0; j < PPT; ++j) u01.v[j] = __saturatef(fmaf(x[f].v[j], lvb[f], lva[f]));
               const V fl = V::fma_rd(u01, gxm1, two23);
+              const float2* row = p32_at(grows, lvo[f]);
 #pragma unroll
               for (int j = 0; j < PPT; ++j) {
-                const uint32_t off = (uint32_t)__float_as_int(fl.v[j]) * 8u + lvo[f];
-                const float2* cell = reinterpret_cast<const float2*>(rows + off);
-                const float2 r = LV == P32_LV_STAGED ? *cell : __ldg(cell);
+                const uint32_t idx = (uint32_t)__float_as_int(fl.v[j]);
+                float2 r;
+                if (LV == P32_LV_STAGED)
+                  r = *reinterpret_cast<const float2*>(smem_raw + (srows + (uint32_t)lvo[f] * 8u + idx * 8u));
+                else
+                  r = __ldg(p32_at(row, (int32_t)idx));
                 sg.v[j] = fmaf(u01.v[j], r.y, r.x);
               }
             } else {
@@ -609,10 +610,10 @@ __global__ void __launch_bounds__(p32_max_threads(N, PPT), 1) phoenix32_kernel(
               } else {
 #pragma unroll
                 for (int j = 0; j < PPT; ++j) {
-                  const bool a = ph[j].alive;
-                  const int acc = (int)(a & (w0[j] >= th0.x)) + (int)(a & (w1[j] >= th1.x));
-                  ph[j].qual += acc;
-                  if (REC) ph[j].qualified += acc;
+                  // (a dead path's count is not read again)
+                  if (w0[j] >= th0.x) ++ph[j].qual;
+                  if (w1[j] >= th1.x) ++ph[j].qual;
+                  if (REC && ph[j].alive) ph[j].qualified += (int)(w0[j] >= th0.x) + (int)(w1[j] >= th1.x);
                 }
               }
             }

@@ -67,13 +67,15 @@ static bool p32_set_shape(const Prepared& P, Fp32Shape& sh, int pb, int ppt, int
 // where a warp steps two scenarios.  When that leaves SMs without a tile, the fewest paths per tile
 // (at least 32) that still give every SM at most one: a tile's time hardly depends on its paths
 // (3 assets, 252 steps: 0.12 ms on 32 paths, 0.19 on 128, 0.29 on 256).  Then the deepest tile that
-// fits: phase changes cost more than occupancy gains (16 scenarios: 10.1 ms at 128 steps, 10.8 at 64,
-// 13.4 at 24).  Local-vol rows are staged when buffers of 32 steps fit beside that depth, or of 16 or 8
+// fits: phase changes cost more than occupancy gains (16 scenarios: 10.0 ms at 128 steps, 10.7 at 64,
+// 13.5 at 24).  Local-vol rows are staged when buffers of 32 steps fit beside that depth, or of 16 or 8
 // beside more than half of it.  Gathers in shared memory cost less latency than cached ones, which
 // counts at few warps: 4 scenarios of 3 assets, 756 steps 0.37 ms against 0.51; one to eight scenarios
 // at 4096 paths × 252 steps 0.06-0.08 against 0.10-0.12, 12 scenarios of one asset on 2^17 paths 0.83
 // against 1.21.  16 warps and 18 surfaces gain nothing: buffers of 8 steps beside half the depth
-// 10.08 ms against 10.04, 17 scenarios 2.98 against 2.92.
+// 9.77 ms against 9.88, 17 scenarios 2.95 against 2.89.  The CTA has all the threads it may have: those
+// past the scenarios share generation and bridge (640 against 512 or 544: 13 scenarios of 3 assets under
+// flat vol 1.055 ms against 1.072, 17 under local vol 1.867 against 1.889).
 static void formula_shape(const Prepared& P, Fp32Shape& sh, uint64_t npaths, int sm_count) {
   int pb = 256;
   while (pb > 32 && P.n_scen * pb / 2 > p32_max_threads(P.n, 2)) pb >>= 1;
@@ -82,9 +84,11 @@ static void formula_shape(const Prepared& P, Fp32Shape& sh, uint64_t npaths, int
   for (; pb >= 32; pb >>= 1)
     for (int i = nd - 1; i >= 0; --i)
       if (p32_set_shape(P, sh, pb, 2, kTileDepths[i], 0)) {
+        bool staged = false;
         for (int rt : kRowSteps)
-          for (int k = i; k >= 0 && (rt == 32 ? k == i : 2 * kTileDepths[k] > kTileDepths[i]); --k)
-            if (p32_set_shape(P, sh, pb, 2, kTileDepths[k], rt)) return;
+          for (int k = i; !staged && k >= 0 && (rt == 32 ? k == i : 2 * kTileDepths[k] > kTileDepths[i]); --k)
+            staged = p32_set_shape(P, sh, pb, 2, kTileDepths[k], rt);
+        sh.threads = p32_max_threads(P.n, 2);
         return;
       }
   raise(RG_ERR_GPU_ERROR, "phoenix32: the tile does not fit in shared memory");
@@ -320,9 +324,10 @@ Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenar
   cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
   const std::vector<int64_t> key{dev, sm_count, P.n, P.trade.has_lv, P.n_scen, P.T, P.stack_max,
                                  P.trade.vr, P.trade.scrambler, P.trade.gx};
-  auto apply = [&](TiledKnobs c, uint64_t paths) {
+  auto apply = [&](TiledKnobs c, uint64_t paths, bool forced = false) {
     Fp32Shape t = sh;
     if (!p32_set_shape(P, t, c.pb, c.ppt, c.tt, c.rt)) return sh;
+    if (c.ppt == 2 && !forced) t.threads = p32_max_threads(P.n, 2);
     t.grid = tiled_grid(P, t, paths, sm_count);
     t.tuned = 1;
     return t;
@@ -330,7 +335,7 @@ Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenar
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     if (g_forced.ppt) {
-      Fp32Shape t = apply({g_forced.pb ? g_forced.pb : sh.Pb, g_forced.ppt, g_forced.tt, 0}, npaths);
+      Fp32Shape t = apply({g_forced.pb ? g_forced.pb : sh.Pb, g_forced.ppt, g_forced.tt, 0}, npaths, true);
       if (!t.tuned) raise(RG_ERR_INVALID_ARGUMENT, "tiled shape: the forced tile does not fit in shared memory");
       return t;
     }

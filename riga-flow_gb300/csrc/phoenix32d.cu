@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
   // the scenario's constants: Cholesky factor, drifts, flat vols or local-vol lookup
   V Lf[N * (N + 1) / 2], mu[N], sig[N];
   float lva[N], lvb[N];
-  uint32_t lvo[N];
+  int32_t lvo[N];
   {
     const float inv_gxm1 = 1.0f / (float)(gx - 1);
     int q = 0;
@@ -96,13 +96,12 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
       sig[f] = V::splat(scen32->sig[f]);
       lva[f] = scen32->a_u[f] * inv_gxm1;
       lvb[f] = scen32->inv_h[f] * inv_gxm1;
-      // byte offset of the surface's row, less the grid index's bias 0x4B000000 in bytes (modulo 2^32)
-      lvo[f] = ((uint32_t)scen32->surf_off[f] - 0x4B000000u) * 8u;
+      lvo[f] = scen32->surf_off[f] - 0x4B000000;  // less the bias of the grid index
     }
   }
   V deep[PPT == 2 ? kSlowSlots : 1][N];
   const int slow = PPT == 2 ? p32d_slow(PPT, stack_max) : 0;
-  const size_t row_step = (size_t)n_surf * gx * sizeof(float2);
+  const int row_step = n_surf * gx;
   const uint64_t groups = (npaths + 32 * PPT - 1) / (32 * PPT);
   // Sobol points from the staged consumption-order tables when they were built for this launch's
   // offset within a 32-point block (else the warp cooperation of rg_warp_sobol)
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
     P32Phoenix ph[PPT];
 #pragma unroll
     for (int j = 0; j < PPT; ++j) ph[j].alive = grp * (32 * PPT) + 32 * j + lane < npaths;
-    const char* rows = reinterpret_cast<const char*>(tb.lv_rows);
+    const float2* rows = tb.lv_rows;
     int c = 0;
     for (int t = 0; t < T; ++t) {
       // bridge nodes consumed at this step: normals, then the streamed bridge (qmc.rs:158-191)
@@ -258,10 +257,10 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
 #pragma unroll
           for (int j = 0; j < PPT; ++j) u01.v[j] = __saturatef(fmaf(x[f].v[j], lvb[f], lva[f]));
           const V fl = V::fma_rd(u01, gxm1, two23);
+          const float2* row = p32_at(rows, lvo[f]);
 #pragma unroll
           for (int j = 0; j < PPT; ++j) {
-            const uint32_t off = (uint32_t)__float_as_int(fl.v[j]) * 8u + lvo[f];
-            const float2 r = __ldg(reinterpret_cast<const float2*>(rows + off));
+            const float2 r = __ldg(p32_at(row, __float_as_int(fl.v[j])));
             sg.v[j] = fmaf(u01.v[j], r.y, r.x);
           }
         } else {
