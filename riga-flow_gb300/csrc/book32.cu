@@ -16,9 +16,9 @@
 // compares, about equally).  Steps go four at a time: one knock-out test on the maximum of four
 // worst-of values serves them all, and the rare path that knocks out in them is settled from the
 // four kept values; accruals are counted as floats.  Three-operand minima halve the worst-of.
-// Measured: 128 trades × 16 scenarios × 2^14 paths 11.0 ms against 37.8 ms for one path and one
-// scenario a thread with a launch per underlying count (41 of 80 TFLOP/s); 64 trades × 2^17 paths
-// 42.4 ms against 193 ms (there the five launches' tails had left most SMs idle).
+// Measured: 128 trades × 16 scenarios × 2^14 paths 10.1 ms against 37.8 ms for one path and one
+// scenario a thread with a launch per underlying count (45 of 80 TFLOP/s); 64 trades × 2^17 paths
+// 38 ms against 193 ms (there the five launches' tails had left most SMs idle).
 // Per path the payoff values are FP32; each 32 paths are summed by a fixed butterfly and every sum
 // above that is FP64 in a fixed order, so an item's sums do not depend on which CTA ran it.
 #include <algorithm>
@@ -31,10 +31,11 @@ namespace rg {
 
 // ------------------------------------------------------------------ TMA-staged scan ----------
 // The increments a (trade, path tile) stage needs — for each of the trade's N underlyings, TT
-// steps × Pb paths — are one 3-D tensor-map box each (paths innermost).  One elected thread
-// issues the next stage's boxes into the other shared-memory buffer (cp.async.bulk.tensor,
-// completion counted on that buffer's "full" mbarrier) while every warp consumes the current
-// buffer, and each warp releases a buffer on its "empty" mbarrier when it is done with it.
+// steps × Pb paths — are one 3-D tensor-map box each (paths innermost), copied into one of two
+// shared-memory buffers (cp.async.bulk.tensor, completion counted on that buffer's "full" mbarrier).
+// The warp that is the last to be done with a buffer issues the boxes of the stage after next into it,
+// so no warp waits for another (with one thread that waited for all the others and then issued, a
+// book of 64 trades on 2^17 paths took 58.2 ms, 57.0 without).
 // Every wait is bounded: a wait that runs out sets the status word and the kernel returns.
 
 // Bounded wait for the phase of `bar` with the given parity to complete; sets the status word
@@ -73,7 +74,8 @@ __device__ __forceinline__ float2 worst_of_n(const float2 (&x)[N]) {
 // What a CTA's threads share over the launch.
 struct BookScanCta {
   float* bufs;                 // two stage buffers
-  uint64_t *full, *empty;      // their mbarriers
+  uint64_t* full;              // their mbarriers
+  int* done;                   // warps done with each buffer
   const CUtensorMap* tmap;     // of this item's underlying count
   int TT;                      // steps per stage of this item
   int* status;
@@ -116,19 +118,20 @@ __device__ __forceinline__ bool book_scan32(const BookDev& bk, const BookTradeDe
   const int ntt = (T + TT - 1) / TT;
   const int nst = ntiles * ntt;
   const uint32_t stage_floats = (uint32_t)(N * TT * PB);
-  // the producer: stage st of this item into buffer g & 1 (the (g >> 1)-th use of that buffer)
-  auto produce = [&](uint32_t g, int st) -> bool {
-    const uint32_t b = g & 1u, u = g >> 1;
-    if (u >= 1 && !mbar_wait(&cta.empty[b], (u - 1) & 1u, cta.status)) return false;
+  // stage st of this item into buffer g & 1, which no warp uses
+  auto produce = [&](uint32_t g, int st) {
+    const uint32_t b = g & 1u;
     const int tile = st / ntt, k = st % ntt;
     mbar_expect_tx(&cta.full[b], stage_floats * 4u);
     float* dst = cta.bufs + b * stage_floats;
 #pragma unroll
     for (int f = 0; f < N; ++f)
       tma_load_3d(dst + f * TT * PB, cta.tmap, &cta.full[b], (int)(p_lo + (uint64_t)tile * PB), tr.idx[f], k * TT);
-    return true;
   };
-  if (tid == 0 && !produce(G, 0)) return false;
+  if (tid == 0) {
+    produce(G, 0);
+    if (nst > 1) produce(G + 1, 1);
+  }
   // path state, [scenario][path of the pair]; a path that knocked out has a NaN threshold
   float2 x[NS][N], qual[NS], worst[NS];
   float ko_th[NS][2], unpaid[NS][2], cpv[NS][2], mpv[NS][2];
@@ -148,7 +151,6 @@ __device__ __forceinline__ bool book_scan32(const BookDev& bk, const BookTradeDe
     lo = a;
   };
   for (int st = 0; st < nst; ++st, ++G) {
-    if (tid == 0 && st + 1 < nst && !produce(G + 1, st + 1)) return false;
     if (k == 0) {
       // a new path tile: fresh path state
       received = 0;
@@ -296,9 +298,17 @@ __device__ __forceinline__ bool book_scan32(const BookDev& bk, const BookTradeDe
         ++tt;
       }
     }
-    // this warp is done with the buffer
+    // this warp is done with the buffer; the last one refills it
     __syncwarp();
-    if (lane == 0) mbar_arrive(&cta.empty[b]);
+    if (lane == 0) {
+      __threadfence_block();
+      if (atomicAdd(&cta.done[b], 1) == (int)(blockDim.x >> 5) - 1) {
+        cta.done[b] = 0;  // the next count starts after the refill has landed
+        __threadfence_block();
+        fence_proxy_async_smem();
+        if (st + 2 < nst) produce(G + 2, st + 2);
+      }
+    }
     if (++k == ntt) {
       // path close (note.rs:221-258) in FP32.  Each quantity is summed over the 32 paths of a half
       // warp by the butterfly over path offsets 16, 8, 4, 2, 1, the last one the thread's own pair;
@@ -375,7 +385,9 @@ __device__ __forceinline__ bool book_scan32_group(const BookMaps& maps, const Bo
   int& s_item = *cta.item;
   auto s_red = reinterpret_cast<double(*)[NS][32]>(cta.red);
   constexpr int PG = PB / 64;  // path groups: warps that share a scenario group
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the warp's number by a shuffle: warp-uniform to the compiler, whose loop state then needs no vector
+  // registers (276 bytes of spills gone, the book 57.0 -> 53.5 ms)
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int s0 = warp / PG * NS, pl = (warp % PG) * 64 + 2 * lane;
   const int ng = groups.n[N - 1];
   const int64_t n_items = (int64_t)((npaths + blk_paths - 1) / blk_paths) * ng;
@@ -417,7 +429,8 @@ __global__ void __launch_bounds__(512, 1) book_scan32_kernel(const __grid_consta
                                                              double* __restrict__ partial, int32_t* __restrict__ counter,
                                                              int* __restrict__ status) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ uint64_t s_bars[4];
+  __shared__ uint64_t s_bars[2];
+  __shared__ int s_done[2];
   __shared__ int s_item;
   __shared__ double s_red[16 * NS * 32];
   BookScanCta cta;
@@ -425,12 +438,12 @@ __global__ void __launch_bounds__(512, 1) book_scan32_kernel(const __grid_consta
   cta.red = s_red;
   cta.bufs = reinterpret_cast<float*>(smem_raw);
   cta.full = s_bars;
-  cta.empty = s_bars + 2;
+  cta.done = s_done;
   cta.status = status;
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(&cta.full[b], 1);
-      mbar_init(&cta.empty[b], blockDim.x >> 5);
+      s_done[b] = 0;
     }
     mbar_init_fence();
   }

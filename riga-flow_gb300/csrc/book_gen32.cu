@@ -64,7 +64,8 @@ __global__ void __launch_bounds__(32 * kGenWarps, 2) book_gen32_kernel(const __g
   constexpr int kRow = UP * kGenPaths;                  // floats per stack entry
   const DevTables& tb = A.tb;
   const int U = A.U, B = A.nodes, T = (int)A.gen.steps;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the warp's number by a shuffle: warp-uniform to the compiler
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const BookGenLayout lay = book_gen_layout(U, A.depth, B);
   float* z = reinterpret_cast<float*>(smem_raw + lay.z);      // [node][asset][path]
   float* stk = reinterpret_cast<float*>(smem_raw + lay.stk);  // [depth][asset][path]
