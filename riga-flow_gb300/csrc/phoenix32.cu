@@ -262,7 +262,7 @@ static int tiled_grid(const Prepared& P, const Fp32Shape& sh, uint64_t npaths, i
 Fp32Shape phoenix32_shape(const Prepared& P, const DevTables& tb, uint64_t path0, uint64_t npaths, int sm_count) {
   Fp32Shape sh{};
   if (P.n_scen > 32) raise(RG_ERR_INVALID_ARGUMENT, "at most 32 scenarios per fused launch");
-  const bool lut = tb.sob_lut && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o;
+  const bool lut = P.trade.vr == RG_VR_SOBOL && tb.sob_lut && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o;
   if (p32_direct(P, npaths, lut)) {
     // nothing for the scenarios to share: the per-thread kernel without shared-memory tiles
     phoenix32d_shape(P, npaths, lut, sm_count, sh);

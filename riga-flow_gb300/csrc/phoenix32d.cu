@@ -28,7 +28,10 @@
 // 2^21 paths × 1260 steps of 5 assets under local vol: 40 ms at one path a thread; 35.0 with the stack's
 // top in registers, a step's local-vol rows adjacent and the warp number, and so the loops, uniform to
 // the compiler; 34.4 at two paths; 28.5 with the deep stack outside shared memory and the kernel free of
-// the other lanes' generation code.
+// the other lanes' generation code; 27.3 with the cells' addresses by one multiply-add.  The lanes
+// without tables have a kernel of their own, whose long generation wants the registers: 2^20 paths on
+// Halton points 92.7 ms in one kernel for all lanes, 97.8 with the lookup's constants in registers, 70.8
+// with them in shared memory.
 // Every operation of the per-path arithmetic is the one phoenix32.cu performs, in the same order,
 // so a path's FP32 payoff values are identical in both kernels.  Each 32 consecutive paths are one
 // chunk of the sums, added by the same FP32 shuffle butterfly and written as FP64 to
@@ -61,7 +64,15 @@ __host__ __device__ constexpr uint32_t p32d_warp_bytes(int n, int ppt, int stack
   return (uint32_t)(p32d_slots(ppt, stack_max) * n * ppt * 128 + ((ppt + 1) * p32d_hi_row(n) * 4 + 15) / 16 * 16);
 }
 
-template <int N, bool LV, bool REC, int PPT>
+// Bytes of dynamic shared memory per CTA: its warps', and at one path a thread the lookup's constants.
+__host__ __device__ constexpr uint32_t p32d_smem(int n, int ppt, int stack_max) {
+  return p32d_warp_bytes(n, ppt, stack_max) * P32D_WARPS + (ppt == 1 ? (uint32_t)n * 16u : 0u);
+}
+
+// LUT: Sobol points from the staged consumption-order tables, built for this launch's offset within a
+// 32-point block; else, at one path a thread, any lane, Sobol points by the warp cooperation of
+// rg_warp_sobol.
+template <int N, bool LV, bool REC, int PPT, bool LUT>
 __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32d_kernel(
     DevTrade tr, DevTables tb, const DevScen32* __restrict__ scen32, int stack_max, int n_surf, float ln_ko, float ln_cb,
     float ln_ki, uint64_t path0, uint64_t npaths, double* __restrict__ partial, int32_t* __restrict__ ko_steps,
@@ -83,6 +94,8 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
   V Lf[N * (N + 1) / 2], mu[N], sig[N];
   float lva[N], lvb[N];
   int32_t lvo[N];
+  // at one path a thread, where registers are short, the lookup's constants are in shared memory
+  float4* const s_lv = reinterpret_cast<float4*>(s_raw + (size_t)P32D_WARPS * p32d_warp_bytes(N, PPT, stack_max));
   {
     const float inv_gxm1 = 1.0f / (float)(gx - 1);
     int q = 0;
@@ -97,15 +110,14 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
       lva[f] = scen32->a_u[f] * inv_gxm1;
       lvb[f] = scen32->inv_h[f] * inv_gxm1;
       lvo[f] = scen32->surf_off[f] - 0x4B000000;  // less the bias of the grid index
+      if (PPT == 1 && threadIdx.x == 0) s_lv[f] = make_float4(lva[f], lvb[f], __int_as_float(lvo[f]), 0.0f);
     }
+    if (PPT == 1) __syncthreads();
   }
   V deep[PPT == 2 ? kSlowSlots : 1][N];
   const int slow = PPT == 2 ? p32d_slow(PPT, stack_max) : 0;
   const int row_step = n_surf * gx;
   const uint64_t groups = (npaths + 32 * PPT - 1) / (32 * PPT);
-  // Sobol points from the staged consumption-order tables when they were built for this launch's
-  // offset within a 32-point block (else the warp cooperation of rg_warp_sobol)
-  const bool lut = PPT == 2 || (tr.vr == RG_VR_SOBOL && tb.sob_lut != nullptr && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o);
   constexpr int kNb = 32 / N;  // nodes per batch of high-bit terms
   constexpr int kRow = p32d_hi_row(N);
   const int upper = (uint32_t)tb.sob_lut_o + (uint32_t)lane >= 32u ? kRow : 0;  // point in the next 32-block
@@ -122,7 +134,7 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
     // overlaps the current step; both paths of a thread have the same (their points are 32 apart)
     uint32_t lnext[N];
 #pragma unroll
-    for (int f = 0; f < N; ++f) lnext[f] = lut ? __ldg(tb.sob_lut + (size_t)f * 32 + lane) : 0u;
+    for (int f = 0; f < N; ++f) lnext[f] = LUT ? __ldg(tb.sob_lut + (size_t)f * 32 + lane) : 0u;
     V x[N], wcur[N], top[N];  // `top`: the anchor stack's top; W(0) = 0 before the first node
 #pragma unroll
     for (int f = 0; f < N; ++f) {
@@ -159,8 +171,11 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
       // bridge nodes consumed at this step: normals, then the streamed bridge (qmc.rs:158-191)
       const int c1 = __ldg(tb.node_off + t + 1);
       for (; c < c1; ++c) {
-        V zf[N];
-        if (lut) {
+        const V cf = V::splat(__ldg(tb.node_cf + c));
+        push(sp++);
+        // the node's value of factor f, from its normal
+        auto node = [&](int f, V z) { top[f] = V::fma(z, cf, V::mul(V::splat(0.5f), V::add(wcur[f], top[f]))); };
+        if constexpr (LUT) {
           if (c >= cb + kNb) {
             // the high-bit terms X(gray(a)) of q = c·N .. (c + kNb)·N - 1, lane l holding q0 + l:
             // one coalesced row of transposed directions per set bit of gray(a)
@@ -207,29 +222,22 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
           rg_probit32x2(xa, xb, z);
 #pragma unroll
           for (int f = 0; f < N; ++f) {
-            if constexpr (PPT == 2) zf[f] = V::from(z[f]);
-            else zf[f] = V::splat(f % 2 ? z[f / 2].y : z[f / 2].x);
+            if constexpr (PPT == 2) node(f, V::from(z[f]));
+            else node(f, V::splat(f % 2 ? z[f / 2].y : z[f / 2].x));
           }
         } else if (tr.vr == RG_VR_SOBOL) {
 #pragma unroll
           for (int f = 0; f < N; ++f) {
             const uint32_t xs = rg_warp_sobol(tb.sobol + 32 * (size_t)__ldg(tb.nf_row + c * N + f), n1, lane);
-            zf[f] = V::splat(rg_probit32(tr.scrambler == RG_SCRAMBLE_DIGITAL_SHIFT
+            node(f, V::splat(rg_probit32(tr.scrambler == RG_SCRAMBLE_DIGITAL_SHIFT
                                              ? xs ^ __ldg(tb.nf_shift + c * N + f)
-                                             : rg_owen(xs, (uint64_t)__ldg(tb.node_k + c) * N + f, tr.seed)));
+                                             : rg_owen(xs, (uint64_t)__ldg(tb.node_k + c) * N + f, tr.seed))));
           }
         } else {
 #pragma unroll
           for (int f = 0; f < N; ++f)
-            zf[f] = V::splat(rg_qmc_normal32(tr, tb, path0 + grp * 32 + lane, (uint64_t)__ldg(tb.node_k + c) * N + f));
+            node(f, V::splat(rg_qmc_normal32(tr, tb, path0 + grp * 32 + lane, (uint64_t)__ldg(tb.node_k + c) * N + f)));
         }
-        const V cf = V::splat(__ldg(tb.node_cf + c));
-        push(sp);
-#pragma unroll
-        for (int f = 0; f < N; ++f) {
-          top[f] = V::fma(zf[f], cf, V::mul(V::splat(0.5f), V::add(wcur[f], top[f])));
-        }
-        ++sp;
       }
       V d[N], y[N];
 #pragma unroll
@@ -253,11 +261,12 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
           // the saturating grid lookup of the tiled kernel: u01 clamped by the FMA's saturation, the
           // grid index from a round-down FMA's bit pattern (its bias folded into lvo), one gather of
           // the cell's line (c, d) and sigma = c + u01·d
+          const float4 c4 = PPT == 1 ? s_lv[f] : make_float4(lva[f], lvb[f], __int_as_float(lvo[f]), 0.0f);
           V u01;
 #pragma unroll
-          for (int j = 0; j < PPT; ++j) u01.v[j] = __saturatef(fmaf(x[f].v[j], lvb[f], lva[f]));
+          for (int j = 0; j < PPT; ++j) u01.v[j] = __saturatef(fmaf(x[f].v[j], c4.y, c4.x));
           const V fl = V::fma_rd(u01, gxm1, two23);
-          const float2* row = p32_at(rows, lvo[f]);
+          const float2* row = p32_at(rows, __float_as_int(c4.z));
 #pragma unroll
           for (int j = 0; j < PPT; ++j) {
             const float2 r = __ldg(p32_at(row, __float_as_int(fl.v[j])));
@@ -332,21 +341,25 @@ __global__ void __launch_bounds__(P32D_THREADS, p32d_min_ctas(N, PPT)) phoenix32
   }
 }
 
-template <int N, int PPT>
-static const void* kernel_ptr(bool lv, bool rec) {
-  if (lv) return rec ? reinterpret_cast<const void*>(&phoenix32d_kernel<N, true, true, PPT>)
-                     : reinterpret_cast<const void*>(&phoenix32d_kernel<N, true, false, PPT>);
-  return rec ? reinterpret_cast<const void*>(&phoenix32d_kernel<N, false, true, PPT>)
-             : reinterpret_cast<const void*>(&phoenix32d_kernel<N, false, false, PPT>);
+template <int N, int PPT, bool LUT>
+static const void* kernel_of(bool lv, bool rec) {
+  if (lv) return rec ? reinterpret_cast<const void*>(&phoenix32d_kernel<N, true, true, PPT, LUT>)
+                     : reinterpret_cast<const void*>(&phoenix32d_kernel<N, true, false, PPT, LUT>);
+  return rec ? reinterpret_cast<const void*>(&phoenix32d_kernel<N, false, true, PPT, LUT>)
+             : reinterpret_cast<const void*>(&phoenix32d_kernel<N, false, false, PPT, LUT>);
+}
+template <int N>
+static const void* kernel_ptr(bool lv, bool rec, int ppt, bool lut) {
+  return ppt == 2 ? kernel_of<N, 2, true>(lv, rec) : (lut ? kernel_of<N, 1, true>(lv, rec) : kernel_of<N, 1, false>(lv, rec));
 }
 
-static const void* select_kernel(int n, bool lv, bool rec, int ppt) {
+static const void* select_kernel(int n, bool lv, bool rec, int ppt, bool lut) {
   switch (n) {
-    case 1: return ppt == 2 ? kernel_ptr<1, 2>(lv, rec) : kernel_ptr<1, 1>(lv, rec);
-    case 2: return ppt == 2 ? kernel_ptr<2, 2>(lv, rec) : kernel_ptr<2, 1>(lv, rec);
-    case 3: return ppt == 2 ? kernel_ptr<3, 2>(lv, rec) : kernel_ptr<3, 1>(lv, rec);
-    case 4: return ppt == 2 ? kernel_ptr<4, 2>(lv, rec) : kernel_ptr<4, 1>(lv, rec);
-    case 5: return ppt == 2 ? kernel_ptr<5, 2>(lv, rec) : kernel_ptr<5, 1>(lv, rec);
+    case 1: return kernel_ptr<1>(lv, rec, ppt, lut);
+    case 2: return kernel_ptr<2>(lv, rec, ppt, lut);
+    case 3: return kernel_ptr<3>(lv, rec, ppt, lut);
+    case 4: return kernel_ptr<4>(lv, rec, ppt, lut);
+    case 5: return kernel_ptr<5>(lv, rec, ppt, lut);
     default: raise(RG_ERR_INVALID_MARKET_SHAPE, "unsupported asset count");
   }
 }
@@ -366,11 +379,11 @@ void phoenix32d_shape(const Prepared& P, uint64_t npaths, bool lut, int sm_count
     if (!done[dev]) {
       int optin = 0;
       cuda_check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "smem opt-in");
-      for (int ppt = 1; ppt <= 2; ++ppt)
+      for (int ppt = 0; ppt <= 2; ++ppt)  // 0: one path a thread without the tables
         for (int n = 1; n <= RG_NMAX; ++n)
           for (int lv = 0; lv < 2; ++lv)
             for (int rec = 0; rec < 2; ++rec)
-              cuda_check(cudaFuncSetAttribute(select_kernel(n, lv != 0, rec != 0, ppt),
+              cuda_check(cudaFuncSetAttribute(select_kernel(n, lv != 0, rec != 0, std::max(ppt, 1), ppt != 0),
                                               cudaFuncAttributeMaxDynamicSharedMemorySize, optin),
                          "phoenix32d smem attribute");
       done[dev] = 1;
@@ -380,10 +393,10 @@ void phoenix32d_shape(const Prepared& P, uint64_t npaths, bool lut, int sm_count
   sh.direct = 1;
   sh.ppt = ppt;
   sh.threads = P32D_THREADS;
-  sh.smem = (int)(p32d_warp_bytes(P.n, ppt, P.stack_max) * P32D_WARPS);
+  sh.smem = (int)p32d_smem(P.n, ppt, P.stack_max);
   int per_sm = 0;
   cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                 &per_sm, select_kernel(P.n, P.trade.has_lv != 0, false, ppt), P32D_THREADS, sh.smem),
+                 &per_sm, select_kernel(P.n, P.trade.has_lv != 0, false, ppt, lut), P32D_THREADS, sh.smem),
              "phoenix32d occupancy");
   if (per_sm < 1 || p32d_slow(ppt, P.stack_max) > kSlowSlots) raise(RG_ERR_GPU_ERROR, "phoenix32d: launch shape does not fit on an SM");
   const uint64_t warps = (npaths + 32 * ppt - 1) / (32 * ppt);
@@ -393,9 +406,10 @@ void phoenix32d_shape(const Prepared& P, uint64_t npaths, bool lut, int sm_count
 
 void launch_phoenix32d(const Prepared& P, const DevTables& tb, const DevScen32* scen32, uint64_t path0,
                        uint64_t npaths, const Fp32Shape& sh, const LaunchOut& out, cudaStream_t st) {
-  const void* k = select_kernel(P.n, P.trade.has_lv != 0, out.records != nullptr, sh.ppt);
-  if (P.n_scen != 1 || sh.threads != P32D_THREADS ||
-      sh.smem < (int)(p32d_warp_bytes(P.n, sh.ppt, P.stack_max) * P32D_WARPS))
+  const bool lut = P.trade.vr == RG_VR_SOBOL && tb.sob_lut && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o;
+  const void* k = select_kernel(P.n, P.trade.has_lv != 0, out.records != nullptr, sh.ppt, lut);
+  if (P.n_scen != 1 || (sh.ppt == 2 && !lut) || sh.threads != P32D_THREADS ||
+      sh.smem < (int)p32d_smem(P.n, sh.ppt, P.stack_max))
     raise(RG_ERR_GPU_ERROR, "phoenix32d: invalid launch shape");
   DevTrade tr = P.trade;
   DevTables tables = tb;

@@ -92,7 +92,7 @@ struct DevTables {
   const float* df_f;
   const float* df_mat_f;
   int32_t lv_nt;
-  // the direct FP32 kernel's Sobol tables in consumption order q = node·n + factor (phoenix32d.cu):
+  // the FP32 kernels' Sobol tables in consumption order q = node·n + factor (book_gen32.cu):
   // directions transposed [32][n·T], and per q the 32 lanes' low-bit terms for points starting at
   // offset sob_lut_o within a 32-point block (digital shift folded in); null when not staged
   const uint32_t* sob_t;

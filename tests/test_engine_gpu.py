@@ -630,3 +630,21 @@ def test_two_path_direct_kernel_agrees(engine, n, lv, steps):
                             for first, count in ((7, 114690), (7, 57345), (57352, 57345)))
         for field in whole.dtype.names:
             np.testing.assert_array_equal(whole[field], np.concatenate([low[field], high[field]]))
+
+
+@pytest.mark.parametrize("n,lv", [(1, True), (3, False), (5, True)])
+def test_direct_kernel_without_tables_agrees(engine, n, lv):
+    """Lanes without Sobol tables have a direct kernel of their own: Halton points, one scenario on it and
+    the same scenario twice on the tiled kernel give the same bytes on a ragged path count."""
+    r = workloads.lv5_large(paths=196608 + 5, steps=33, kind="halton")
+    r.trade = workloads.phoenix_trade(n, 33, 0.13)
+    r.local_vol, r.options = (r.local_vol[:n] if lv else None), workloads.production_options(40 if lv else 0)
+    m = r.market
+    m.spots, m.vols, m.dividend_yields = m.spots[:n], m.vols[:n], m.dividend_yields[:n]
+    m.correlation = [row[:n] for row in m.correlation[:n]]
+    r.config.variance_reduction = VarianceReduction("halton", n * 33)
+    one = engine.price_raw(r)
+    assert engine.last_timing().tile_steps == 0
+    two = engine.price_scenarios_raw(r, [(m, None)] * 2)
+    assert engine.last_timing().tile_steps > 0
+    assert bytes(one) == bytes(two[0])
