@@ -67,13 +67,10 @@ def flops_per_launch(paths, steps, n_assets, n_scen):
     return float(paths) * steps * per_path_step
 
 
-def n_scen_slots(n_scen):
-    """Scenario slots of the tiled FP32 kernel's CTA: the scenario count rounded up to a power of two,
-    at least 4."""
-    sb = 4
-    while sb < n_scen:
-        sb <<= 1
-    return sb
+def tile_paths(threads, paths_per_thread, n_scen):
+    """Paths per CTA tile of a large tiled FP32 launch: the largest power of two whose stepping threads,
+    one per scenario and paths_per_thread paths, the CTA has (its other threads only generate)."""
+    return 1 << ((threads * paths_per_thread // n_scen).bit_length() - 1)
 
 
 def measured_peaks():
@@ -567,7 +564,7 @@ def run_gpu(args):
         "gpu_launches": int(tm.kernel_launches) * args.steps,
         "launch": {"grid": tm.grid, "block": tm.block, "smem_bytes": tm.smem_bytes,
                    "tile_steps": tm.tile_steps, "paths_per_thread": tm.paths_per_thread,
-                   "paths_per_cta_tile": tm.block * tm.paths_per_thread // n_scen_slots(n_scen),
+                   "paths_per_cta_tile": tile_paths(tm.block, tm.paths_per_thread, n_scen),
                    "tuned_by": (f"forced by --shape {args.shape} (rg_set_tiled_shape)" if args.shape else
                                 "autotuner (rg_set_autotune): paths per CTA tile, paths per thread and tile depth, "
                                 "timed during warm-up")},

@@ -336,20 +336,22 @@ typedef struct rg_timing {
 int32_t rg_engine_last_timing(rg_engine* engine, rg_timing* out);
 
 /* The tiled FP32 kernel's autotuner (on by default, process-wide).  The first pricing call of a
- * launch shape (asset count, local vol, scenario slots, steps, QMC lane, grid width) with at least
- * eight waves of path tiles times every candidate schedule — one or two paths per thread (two:
- * packed FP32x2 stepping on 512 threads) and the time-tile depths — on a prefix of its paths and
- * keeps the fastest for that shape; later calls reuse it.  Neither knob changes a path's arithmetic
+ * launch shape (asset count, local vol, scenarios, steps, QMC lane, grid width) with at least
+ * eight waves of path tiles times every candidate schedule — paths per CTA tile, one or two paths per
+ * thread (two: packed FP32x2 stepping), the time-tile depths, and how many steps of local-vol rows are
+ * staged in shared memory — on a prefix of its paths and
+ * keeps the fastest for that shape; later calls reuse it.  No knob changes a path's arithmetic
  * or the 32-path chunks of the sums, so prices are the same with the autotuner on or off.  Calls
  * through rg_price_put_leg_static never tune.  Disabling also clears the tuned shapes.  No
  * counterpart in the reference. */
 int32_t rg_set_autotune(int32_t enabled);
 /* Forces every tiled FP32 launch of the process onto one schedule: paths per thread 1 or 2, a tile
  * depth among the autotuner's candidates (24, 32, 48, 64, 80, 96, 128) and a block of
- * paths_per_block paths per CTA tile (0 = the formula block of 1024 / scenario slots; otherwise a
- * power of two of at least 32 × paths per thread); (0, 0, 0) returns to the formula shape or the
- * autotuner.  A forced shape that does not fit (shared memory, 1024 threads) fails the pricing
- * call with RG_ERR_INVALID_ARGUMENT.  For callers that need a fixed schedule, and for checking
+ * paths_per_block paths per CTA tile (0 = the formula's, which follows the scenario and path counts;
+ * otherwise a power of two of at least 32 × paths per thread); (0, 0, 0) returns to the formula shape
+ * or the autotuner.  A forced shape reads local-vol rows from global memory.  One that does not fit
+ * (shared memory; 1024 threads at one path per thread, 640 up to three assets and 512 beyond at two)
+ * fails the pricing call with RG_ERR_INVALID_ARGUMENT.  For callers that need a fixed schedule, and for checking
  * that schedules do not change prices.  No counterpart in the reference. */
 int32_t rg_set_tiled_shape(int32_t paths_per_thread, int32_t tile_steps, int32_t paths_per_block);
 /* Clock cycles the tiled FP32 kernel's CTAs spent in generation, bridge, stepping and path close
