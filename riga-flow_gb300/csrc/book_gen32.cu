@@ -9,14 +9,15 @@
 //   C. correlation — a warp takes a node: lane l holds the pair of paths 2l, 2l + 1 of all assets
 //      and forms y_u = Σ_{b<=u} L[u][b]·z_b from the last asset down, in place;
 //   B. bridge — a warp takes the assets u = warp, warp + 8, ...: the streamed bridge
-//      (note.rs:89-106, qmc.rs:158-191) of each pair with its anchor stack in shared memory
-//      [depth][asset][path], and the increments of every step that completes.
-// What bounds it: latency at 16 warps an SM (the bridge's stacks fill the shared memory) — 43% of
-// issue slots used by 117 instructions per (node, asset, 64 paths): two packed inverse normals, half
-// of the 21 multiply-adds an asset's row of the factor averages, the bridge and the stores.
+//      (note.rs:89-106, qmc.rs:158-191) of each pair with the busy end of its anchor stack in shared
+//      memory [depth][asset][path], and the increments of every step that completes.
+// What bounds it: issue and the waits at the phases' barriers: 117 instructions per (node, asset, 64
+// paths): two packed inverse normals, half of the 21 multiply-adds an asset's row of the factor averages,
+// the bridge and the stores.  Up to 20 assets three CTAs fit an SM since the deep stack slots left shared
+// memory (two with all of the stack there: a book of 64 trades on 2^17 paths 53.6 ms against 52.1).
 // Measured on 20 assets × 1260 steps: 1.66 ms per 19,456 paths (one wave), against 11.0 ms for one
 // thread per (path, asset) that formed every Sobol point from its own Gray code; 2^17 paths in three
-// chunks 15.6 ms against 74.
+// chunks 15.6 ms against 74 (two CTAs an SM, one pair of normals at a time).
 // Every normal, correlation and bridge value is formed by the same operations in the same order as
 // one thread per (path, asset) forms them.
 #include <type_traits>
@@ -29,6 +30,10 @@ namespace rg {
 constexpr int kGenPaths = 64;
 constexpr int kGenWarps = 8;
 constexpr int kGenTile = 8;  // nodes per tile where the shared memory holds them
+
+// The bridge stack's last slots, which nearly every node uses (slot d from the end every 2^d steps), are in
+// shared memory; the others in local memory.
+constexpr int kGenFast = 5, kGenSlow = 20;
 
 struct BookGenArgs {
   DevTrade gen;
@@ -48,7 +53,7 @@ __host__ __device__ inline BookGenLayout book_gen_layout(int U, int depth, int n
   const uint32_t up = (uint32_t)(U + 3) / 4u * 4u, row = up * kGenPaths * 4u;
   l.z = 0;
   l.stk = l.z + (uint32_t)nodes * row;
-  l.hi = l.stk + (uint32_t)depth * row;
+  l.hi = l.stk + (uint32_t)(depth < kGenFast ? depth : kGenFast) * row;
   l.L = l.hi + 2u * (uint32_t)nodes * up * 16u;
   l.node = l.L + up * up * 8u;
   l.total = l.node + 8u * kGenTile;
@@ -58,7 +63,7 @@ __host__ __device__ inline BookGenLayout book_gen_layout(int U, int depth, int n
 // UP: the universe's assets rounded up to four.  The loops over assets run to UP without a guard on
 // what they read: entries past U hold whatever the memory did, and nothing below U depends on them.
 template <int UP>
-__global__ void __launch_bounds__(32 * kGenWarps, 2) book_gen32_kernel(const __grid_constant__ BookGenArgs A) {
+__global__ void __launch_bounds__(32 * kGenWarps, UP <= 20 ? 3 : 2) book_gen32_kernel(const __grid_constant__ BookGenArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int KA = (UP + kGenWarps - 1) / kGenWarps;  // assets per warp of the bridge
   constexpr int kRow = UP * kGenPaths;                  // floats per stack entry
@@ -95,7 +100,13 @@ __global__ void __launch_bounds__(32 * kGenWarps, 2) book_gen32_kernel(const __g
   float* out = A.incr + (uint64_t)warp * A.rowlen + p0 + 2 * lane;  // this warp's first asset at step t
   const uint64_t out_asset = kGenWarps * A.rowlen, out_step = (uint64_t)U * A.rowlen;
   int t = 0, hi0 = 0;
-  float* sp = stk + warp * kGenPaths + 2 * lane;  // this warp's first asset in the next stack entry
+  float* const sp = stk + warp * kGenPaths + 2 * lane;  // this warp's first asset in the first fast slot
+  float2 deep[kGenSlow][KA];
+  const int slow = max(A.depth - kGenFast, 0);
+  int d = 0;  // stack entries
+  auto slot = [&](int e, int k) -> float2& {
+    return *reinterpret_cast<float2*>(sp + (e - slow) * kRow + k * kGenWarps * kGenPaths);
+  };
   for (int c0 = 0; c0 < T; c0 += B) {
     const int nb = min(B, T - c0);
     if (lut && (c0 == 0 || c0 >= hi0 + 2 * B)) {
@@ -209,14 +220,14 @@ __global__ void __launch_bounds__(32 * kGenWarps, 2) book_gen32_kernel(const __g
           const float2 y = *reinterpret_cast<const float2*>(zb + k * kGenWarps * kGenPaths);
           const float2 mid = __fmul2_rn(half, __fadd2_rn(wcur[k], top[k]));
           top[k] = first ? __fmul2_rn(y, c2) : __ffma2_rn(y, c2, mid);
-          *reinterpret_cast<float2*>(sp + k * kGenWarps * kGenPaths) = top[k];
+          if (d < slow) deep[d][k] = top[k];
+          else slot(d, k) = top[k];
         }
-      sp += kRow;
+      ++d;
       // every step whose nodes are all here takes the top of the stack
       for (; t < done; ++t, out += out_step) {
-        sp -= kRow;
-        // the entry below (none after the last step: what is read then is not used)
-        const float* below = sp - (t + 1 < T ? kRow : 0);
+        --d;
+        const int below = max(d - 1, 0);  // the entry below (none after the last step: not used then)
 #pragma unroll
         for (int k = 0; k < KA; ++k) {
           // rows are padded to whole CTAs' paths, so the last CTA stores all of its own
@@ -224,7 +235,7 @@ __global__ void __launch_bounds__(32 * kGenWarps, 2) book_gen32_kernel(const __g
             *reinterpret_cast<float2*>(out + k * out_asset) = __ffma2_rn(wcur[k], minus, top[k]);
           wcur[k] = top[k];
           if ((k + 1) * kGenWarps <= UP || warp + k * kGenWarps < UP)
-            top[k] = *reinterpret_cast<const float2*>(below + k * kGenWarps * kGenPaths);
+            top[k] = below < slow ? deep[below][k] : slot(below, k);
         }
       }
     }
@@ -240,7 +251,8 @@ void launch_book_gen32(const DevTrade& gen, const DevTables& tb, const float* L3
   int nodes = kGenTile;
   while (nodes > 1 && book_gen_layout(U, depth, nodes).total > kMax) nodes >>= 1;
   const uint32_t smem = book_gen_layout(U, depth, nodes).total;
-  if (smem > kMax) raise(RG_ERR_GPU_ERROR, "book generation: the bridge stack exceeds the shared-memory limit");
+  if (smem > kMax || depth > kGenFast + kGenSlow)
+    raise(RG_ERR_GPU_ERROR, "book generation: the bridge stack exceeds the shared-memory limit");
   if (rowlen % kGenPaths) raise(RG_ERR_GPU_ERROR, "book generation: rows must be padded to 64 paths");
   const BookGenArgs a{gen, tb, L32, U, depth, nodes, path0, npaths, rowlen, incr};
   const unsigned blocks = (unsigned)((npaths + kGenPaths - 1) / kGenPaths);
