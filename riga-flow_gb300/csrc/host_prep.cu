@@ -313,12 +313,34 @@ void bridge_schedule_into(int64_t T, double dt, Prepared& P) {
 }
 
 // The smallest spot s >= 0 with s / init >= barrier as FP64 rounds the ratio (rounding is monotone, so
-// every larger spot reaches the barrier too and no smaller one does).
-static double smallest_spot(double barrier, double init) {
-  double s = std::max(barrier * init, 0.0);
-  while (s > 0.0 && s / init >= barrier) s = std::nextafter(s, 0.0);
-  while (!(s / init >= barrier) && s < INFINITY) s = std::nextafter(s, INFINITY);
-  return s;
+// every larger spot reaches the barrier too and no smaller one does); init > 0, barrier > 0 or infinite.
+// A bisection over the bit patterns, which order non-negative doubles; it starts from the few doubles
+// around barrier·init that hold the answer unless the product or the quotient overflows or is subnormal.
+double smallest_spot(double barrier, double init) {
+  auto value = [](uint64_t bits) {
+    double s;
+    std::memcpy(&s, &bits, sizeof s);
+    return s;
+  };
+  auto reaches = [&](uint64_t bits) { return value(bits) / init >= barrier; };
+  uint64_t lo = 0, hi = 0x7ff0000000000000ULL;  // zero and infinity
+  if (reaches(lo)) return 0.0;
+  const double guess = barrier * init;
+  if (guess > 0.0 && guess < INFINITY) {
+    uint64_t at;
+    std::memcpy(&at, &guess, sizeof at);
+    const uint64_t below = at > 4 ? at - 4 : 0, above = std::min(at + 4, hi);
+    if (reaches(below)) hi = below;
+    else lo = below;
+    if (!reaches(above)) lo = std::max(lo, above);
+    else hi = std::min(hi, above);
+  }
+  while (hi - lo > 1) {
+    const uint64_t mid = lo + (hi - lo) / 2;
+    if (reaches(mid)) hi = mid;
+    else lo = mid;
+  }
+  return value(hi);
 }
 
 void prepare(const rg_price_request* r, const rg_scenario* sc, int n_scen, Prepared& P) {

@@ -160,6 +160,8 @@ int device_sm_count();
 void prepare(const rg_price_request* req, const rg_scenario* scen, int n_scen, Prepared& P);
 // The streamed bridge schedule (node_off, node_k, node_c, stack_max) of T steps.
 void bridge_schedule_into(int64_t T, double dt, Prepared& P);
+// The smallest spot whose ratio to `init`, as FP64 rounds it, reaches `barrier` (infinity: absent).
+double smallest_spot(double barrier, double init);
 // The Sobol direction table for `dim` dimensions (process-wide cache).
 const std::vector<uint32_t>& sobol_table(int64_t dim);
 std::vector<double> calib_axes(const rg_implied_vol_grid& g, double spot, double rate, int gx);

@@ -93,3 +93,15 @@ def test_extreme_paths_agree(engine, vol, years):
     req.trade.maturity_years = years
     req.market.vols = [vol] * 3
     _check(engine, req)
+
+
+@pytest.mark.parametrize("init", [1e-3, 0.73, 1.0, 3.1, 1e6])
+@pytest.mark.parametrize("terms", [dict(knock_out_barrier=None, coupon_barrier=None), dict(), dict(knock_out_barrier=1.0 / 3.0),
+                                   dict(knock_out_barrier=1e300, coupon_barrier=1e300)])
+def test_initial_spots_agree(engine, init, terms):
+    """The engine's kernels compare spots with thresholds, the static one's ratios with barriers: the same
+    events at initial spots whose ratios round differently, with barriers absent, ordinary and beyond reach."""
+    req = _request(3, 500, 60, None, **terms)
+    req.trade.initial_spots = [init * (1.0 + 0.1 * f) for f in range(3)]
+    req.market.spots = [s * 1.01 for s in req.trade.initial_spots]
+    _check(engine, req)
