@@ -2,7 +2,7 @@
 //
 // The reference's arithmetic (crates/riga-engine/src/note.rs:81-259) in its own operation order,
 // product by product, as phoenix64.cu performs it in one kernel; here the work is split where its
-// shape changes, through a buffer of a chunk of paths:
+// shape changes, through a buffer of a chunk of paths and, where schedules are long, a window of steps:
 //   * normals64_kernel — correlated normals y = L·z of every bridge node, y[node][asset][path].  A
 //     CTA forms the normals of 256 paths × a few nodes; the 5% that fall into the inverse normal's
 //     tails (a logarithm, a square root and a division) are queued in shared memory and taken 32 at
@@ -36,14 +36,14 @@ template <int N>
 __global__ void __launch_bounds__(kNormPaths) normals64_kernel(DevTrade tr, DevTables tb,
                                                                const DevScenario* __restrict__ scen, uint64_t path0,
                                                                uint64_t npaths, uint64_t stride, int path_blocks,
-                                                               double* __restrict__ y) {
+                                                               int node0, int node1, double* __restrict__ y) {
   constexpr int KN = norm_nodes(N);
   __shared__ double zs[KN * N][kNormPaths];
   __shared__ uint16_t queue[KN * N * kNormPaths];
   __shared__ int queued;
   const int tid = threadIdx.x, lane = tid & 31;
   const uint64_t p = (uint64_t)(blockIdx.x % path_blocks) * kNormPaths + tid;
-  const int c0 = (int)(blockIdx.x / path_blocks) * KN, nn = min(KN, (int)tr.steps - c0);
+  const int c0 = node0 + (int)(blockIdx.x / path_blocks) * KN, nn = min(KN, node1 - c0);
   if (tid == 0) queued = 0;
   __syncthreads();
   if (tr.vr == RG_VR_SOBOL) {
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kNormPaths) normals64_kernel(DevTrade tr, DevT
       double s = sc.L[a * N] * z[0];
 #pragma unroll
       for (int b = 1; b <= a; ++b) s += sc.L[a * N + b] * z[b];
-      y[((uint64_t)(c0 + j) * N + a) * stride + p] = s;
+      y[((uint64_t)(c0 - node0 + j) * N + a) * stride + p] = s;
     }
   }
 }
@@ -97,12 +97,12 @@ template <int N>
 __global__ void __launch_bounds__(kCorPaths * 8) correlate64_kernel(const DevScenario* __restrict__ scen,
                                                                    const double* __restrict__ z, int64_t T,
                                                                    uint64_t npaths, uint64_t stride, int path_blocks,
-                                                                   double* __restrict__ y) {
+                                                                   int64_t step0, int64_t step1, double* __restrict__ y) {
   __shared__ double zs[kCorPaths][kCorSteps * N + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t p0 = (uint64_t)(blockIdx.x % path_blocks) * kCorPaths;
-  const int64_t t0 = (int64_t)(blockIdx.x / path_blocks) * kCorSteps;
-  const int nt = (int)min((int64_t)kCorSteps, T - t0);
+  const int64_t t0 = step0 + (int64_t)(blockIdx.x / path_blocks) * kCorSteps;
+  const int nt = (int)min((int64_t)kCorSteps, step1 - t0);
   for (int r = warp; r < kCorPaths; r += 8)
     if (p0 + r < npaths)
       for (int i = lane; i < nt * N; i += 32) zs[r][i] = z[((p0 + r) * (uint64_t)T + t0) * N + i];
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kCorPaths * 8) correlate64_kernel(const DevSce
       double s = sc.L[a * N] * zs[lane][j * N];
 #pragma unroll
       for (int b = 1; b <= a; ++b) s += sc.L[a * N + b] * zs[lane][j * N + b];
-      y[((uint64_t)(t0 + j) * N + a) * stride + p] = s;
+      y[((uint64_t)(t0 - step0 + j) * N + a) * stride + p] = s;
     }
 }
 
@@ -160,14 +160,21 @@ __device__ __forceinline__ double sigma64(const double* __restrict__ v, const do
 }
 
 constexpr int kStepWarps = 2;
+constexpr int kCtaThreads = 32 * kStepWarps;
+// Words of a lane's state between two windows of steps, beside its bridge stack.
+constexpr int kStateWords = 7;
 
 struct Step64Args {
   DevTrade tr;
   DevTables tb;
   const DevScenario* scen;
-  const double* y;      // [node or step][asset][stride]
+  const double* y;      // [node or step of the window][asset][stride]
   const double2* axis;  // [surface][gx]
   uint64_t stride, path0, first, npaths;  // global index of path 0; the chunk's first path; its paths
+  int64_t t0, t1;       // the window's steps
+  int node0, node1;     // and the bridge nodes they consume
+  double* state;        // [word][thread of the chunk] between windows (unused when one covers all steps)
+  uint64_t state_row;
   double* partial;      // row of the chunk's first CTA
   int32_t* ko_steps;
   rg_path_record* records;
@@ -175,7 +182,7 @@ struct Step64Args {
 };
 
 template <int N, bool LV, bool MC>
-__global__ void __launch_bounds__(32 * kStepWarps) step64_kernel(const __grid_constant__ Step64Args A) {
+__global__ void __launch_bounds__(kCtaThreads) step64_kernel(const __grid_constant__ Step64Args A) {
   constexpr int G = 32 / N;  // paths per warp, a lane per asset
   extern __shared__ double stk_mem[];  // [depth][thread] bridge anchors
   __shared__ double red[kStepWarps * G][RG_ACC];
@@ -209,30 +216,49 @@ __global__ void __launch_bounds__(32 * kStepWarps) step64_kernel(const __grid_co
   float* cube = A.cube ? A.cube + (A.first + pl) * (uint64_t)T * N + f : nullptr;
   double* stk = stk_mem + tid;
   double spot = sc.spots[f], wcur = 0.0, top = 0.0;
-  int sp = 0, c = 0;
+  int sp = 0, c = A.node0;
   int qual = 0, ko_step = -1, qualified = 0, paid = 0;
   bool ko = false, received = false;
   double unpaid = 0.0, cpv = 0.0, mpv = 0.0;
+  double* const state = A.state + (uint64_t)blockIdx.x * kCtaThreads + tid;
+  if (A.t0 > 0) {  // what the window before left
+    spot = state[0];
+    wcur = state[A.state_row];
+    unpaid = state[2 * A.state_row];
+    cpv = state[3 * A.state_row];
+    mpv = state[4 * A.state_row];
+    qual = __double2loint(state[5 * A.state_row]);
+    ko_step = __double2hiint(state[5 * A.state_row]);
+    qualified = __double2loint(state[6 * A.state_row]);
+    paid = __double2hiint(state[6 * A.state_row]);
+    ko = ko_step >= 0;
+    received = paid > 0;
+    if (!MC) {
+      sp = A.node0 - (int)A.t0;
+      for (int i = 0; i < sp; ++i) stk[i * kCtaThreads] = state[(kStateWords + i) * A.state_row];
+      if (sp > 0) top = stk[(sp - 1) * kCtaThreads];
+    }
+  }
   double ynext = __ldg(yp);
-  for (int64_t t = 0; t < T; ++t) {
+  for (int64_t t = A.t0; t < A.t1; ++t) {
     double shock;
     if (MC) {
       shock = ynext;
-      if (t + 1 < T) ynext = __ldg(yp + (uint64_t)(t + 1) * ystep);
+      if (t + 1 < A.t1) ynext = __ldg(yp + (uint64_t)(t + 1 - A.t0) * ystep);
     } else {
       // bridge nodes consumed at this step (note.rs:89-105 and qmc.rs:158-191)
       const int c1 = __ldg(tb.node_off + t + 1);
       for (; c < c1; ++c) {
         const double yc = ynext * __ldg(tb.node_c + c);
-        if (c + 1 < (int)T) ynext = __ldg(yp + (uint64_t)(c + 1) * ystep);
+        if (c + 1 < A.node1) ynext = __ldg(yp + (uint64_t)(c + 1 - A.node0) * ystep);
         top = c == 0 ? yc : halve(wcur + top) + yc;
-        stk[sp * (32 * kStepWarps)] = top;
+        stk[sp * kCtaThreads] = top;
         ++sp;
       }
       --sp;
       shock = (top - wcur) * inv_sqrt_dt;
       wcur = top;
-      if (sp > 0) top = stk[(sp - 1) * (32 * kStepWarps)];
+      if (sp > 0) top = stk[(sp - 1) * kCtaThreads];
     }
     // GBM / Dupire step (note.rs:133-142)
     if (LV) {
@@ -294,6 +320,18 @@ __global__ void __launch_bounds__(32 * kStepWarps) step64_kernel(const __grid_co
         unpaid += tr.coupon_rate;
       }
     }
+  }
+  if (A.t1 < T) {
+    state[0] = spot;
+    state[A.state_row] = wcur;
+    state[2 * A.state_row] = unpaid;
+    state[3 * A.state_row] = cpv;
+    state[4 * A.state_row] = mpv;
+    state[5 * A.state_row] = __hiloint2double(ko_step, qual);
+    state[6 * A.state_row] = __hiloint2double(paid, qualified);
+    if (!MC)
+      for (int i = 0; i < sp; ++i) state[(kStateWords + i) * A.state_row] = stk[i * kCtaThreads];
+    return;
   }
   // path close (note.rs:221-258) on the path's first lane
   const double ratio = spot / init;
@@ -369,12 +407,47 @@ __global__ void __launch_bounds__(32 * kStepWarps) step64_kernel(const __grid_co
 // Paths of one step64 CTA.
 uint64_t cta_paths(int n) { return (uint64_t)kStepWarps * (32 / n); }
 
-// Paths per chunk, in whole CTAs: chunks about equal, their correlated normals within a GiB each.
-uint64_t chunk_of(int n, int64_t T, uint64_t npaths) {
-  const uint64_t unit = cta_paths(n), fit = (uint64_t(1) << 30) / ((uint64_t)T * n * sizeof(double));
-  const uint64_t cap = std::max<uint64_t>(fit / unit, 1), ctas = (npaths + unit - 1) / unit;
-  const uint64_t chunks = (ctas + cap - 1) / cap;
-  return (ctas + chunks - 1) / chunks * unit;
+// Deepest bridge stack of T steps.
+int stack_bound(int64_t T) {
+  int bits = 0;
+  while (T >> bits) ++bits;
+  return std::min(bits + 1, RG_STACK_MAX);
+}
+
+// How a launch passes through the buffer: `chunk` paths (whole CTAs) at a time, `window` steps at a time.
+struct Path64Plan {
+  uint64_t chunk;
+  int64_t window;
+  size_t y_bytes, state_bytes;
+};
+// Whole schedules of all paths where `limit` bytes hold them, else of chunks of about equal path counts
+// as long as a chunk has kFillCtas CTAs.  Long schedules, whose chunks would leave SMs without work, pass
+// all paths (up to twice that many CTAs) through windows of steps instead, the state of each path carried
+// from one to the next; a limit too small for windows of kMinWindow steps takes fewer paths.
+// Measured, 3 assets flat, 2^16 paths, a GiB, chunks against windows: 2000 steps (chunks of 1,093 CTAs)
+// 58.9 and 57.4 ms, 5000 (437) 158 and 143, 15,000 (149) 742 and 430, 50,000 (44) 6,839 and 1,434, where
+// one kernel took 5,096; 1000 paths x 200,000 steps 1,638 and 362.
+constexpr uint64_t kFillCtas = 152 * 8;
+constexpr int64_t kMinWindow = 16;
+Path64Plan path64_plan(int n, int64_t T, uint64_t npaths, size_t limit) {
+  const uint64_t unit = cta_paths(n), ctas = (npaths + unit - 1) / unit;
+  const uint64_t row = unit * n * sizeof(double);  // a CTA's normals of one node
+  const uint64_t fit = limit / (row * (uint64_t)T);
+  auto even = [&](uint64_t cap) {
+    const uint64_t chunks = (ctas + cap - 1) / cap;
+    return (ctas + chunks - 1) / chunks;
+  };
+  if (fit >= std::min(ctas, kFillCtas)) {
+    const uint64_t per = even(fit);
+    return {per * unit, T, (size_t)(per * row * (uint64_t)T), 0};
+  }
+  const uint64_t depth = (uint64_t)stack_bound(T), state = (kStateWords + depth) * kCtaThreads * sizeof(double);
+  const uint64_t shortest = std::min<uint64_t>(kMinWindow, (uint64_t)T);
+  const uint64_t per = even(std::max<uint64_t>(std::min(2 * kFillCtas, limit / (state + row * (shortest + depth))), 1));
+  // a window's steps consume at most `depth` nodes more than it has steps
+  const uint64_t nodes = per * state < limit ? (limit - per * state) / (per * row) : 0;
+  const uint64_t window = std::min<uint64_t>(std::max<uint64_t>(nodes, depth + 1) - depth, (uint64_t)T);
+  return {per * unit, (int64_t)window, (size_t)(per * row * (window + depth)), (size_t)(per * state)};
 }
 
 template <int N>
@@ -382,41 +455,49 @@ void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario
          const LaunchOut& out, cudaStream_t st) {
   const int64_t T = P.T;
   const bool lv = P.trade.has_lv != 0;
-  const uint64_t chunk = chunk_of(N, T, npaths);
+  const Path64Plan plan = path64_plan(N, T, npaths, W.normals64_limit);
+  const uint64_t chunk = plan.chunk, unit = cta_paths(N);
+  if (P.stack_max > stack_bound(T)) raise(RG_ERR_INVALID_SCHEDULE, "path64: the bridge stack is too deep");
   const size_t axis_bytes = lv ? (size_t)P.n_surf * P.trade.gx * sizeof(double2) : 0;
-  uint8_t* buf = static_cast<uint8_t*>(W.device(WS_NORMALS64, axis_bytes + chunk * (uint64_t)T * N * sizeof(double)));
-  double* y = reinterpret_cast<double*>(buf + axis_bytes);
-  Step64Args a{P.trade, tb, scen, y, reinterpret_cast<const double2*>(buf), chunk, path0, 0, 0, out.partial,
-               out.ko_steps, out.records, out.cube};
+  uint8_t* buf = static_cast<uint8_t*>(W.device(WS_NORMALS64, axis_bytes + plan.state_bytes + plan.y_bytes));
+  double* state = reinterpret_cast<double*>(buf + axis_bytes);
+  double* y = reinterpret_cast<double*>(buf + axis_bytes + plan.state_bytes);
+  Step64Args a{P.trade, tb, scen, y, reinterpret_cast<const double2*>(buf), chunk, path0, 0, 0, 0, 0, 0, 0, state,
+               chunk / unit * kCtaThreads, out.partial, out.ko_steps, out.records, out.cube};
   if (lv) {
     const int n = P.n_surf * P.trade.gx;
     axis64_kernel<<<(n + 127) / 128, 128, 0, st>>>(tb.lv_logs, P.trade.gx, n, reinterpret_cast<double2*>(buf));
     cuda_check(cudaGetLastError(), "axis64_kernel launch");
   }
-  const size_t smem = out.mcz ? 0 : (size_t)P.stack_max * 32 * kStepWarps * sizeof(double);
+  const size_t smem = out.mcz ? 0 : (size_t)P.stack_max * kCtaThreads * sizeof(double);
   for (a.first = 0; a.first < npaths; a.first += chunk) {
     a.npaths = std::min(chunk, npaths - a.first);
-    if (out.mcz) {
-      const int pb = (int)((a.npaths + kCorPaths - 1) / kCorPaths);
-      const int64_t tb_n = (T + kCorSteps - 1) / kCorSteps;
-      correlate64_kernel<N><<<(unsigned)(pb * tb_n), kCorPaths * 8, 0, st>>>(
-          scen, out.mcz + a.first * (uint64_t)T * N, T, a.npaths, chunk, pb, y);
-    } else {
-      const int pb = (int)((a.npaths + kNormPaths - 1) / kNormPaths);
-      const int64_t nb = (T + norm_nodes(N) - 1) / norm_nodes(N);
-      normals64_kernel<N><<<(unsigned)(pb * nb), kNormPaths, 0, st>>>(P.trade, tb, scen, path0 + a.first, a.npaths,
-                                                                      chunk, pb, y);
+    const unsigned blocks = (unsigned)((a.npaths + unit - 1) / unit);
+    for (a.t0 = 0; a.t0 < T; a.t0 = a.t1) {
+      a.t1 = std::min(a.t0 + plan.window, T);
+      a.node0 = P.node_off[a.t0];
+      a.node1 = P.node_off[a.t1];
+      if (out.mcz) {
+        const int pb = (int)((a.npaths + kCorPaths - 1) / kCorPaths);
+        const int64_t tiles = (a.t1 - a.t0 + kCorSteps - 1) / kCorSteps;
+        correlate64_kernel<N><<<(unsigned)(pb * tiles), kCorPaths * 8, 0, st>>>(
+            scen, out.mcz + a.first * (uint64_t)T * N, T, a.npaths, chunk, pb, a.t0, a.t1, y);
+      } else if (a.node1 > a.node0) {
+        const int pb = (int)((a.npaths + kNormPaths - 1) / kNormPaths);
+        const int64_t tiles = (a.node1 - a.node0 + norm_nodes(N) - 1) / norm_nodes(N);
+        normals64_kernel<N><<<(unsigned)(pb * tiles), kNormPaths, 0, st>>>(P.trade, tb, scen, path0 + a.first, a.npaths,
+                                                                           chunk, pb, a.node0, a.node1, y);
+      }
+      cuda_check(cudaGetLastError(), "normals64 launch");
+      if (lv) {
+        if (out.mcz) step64_kernel<N, true, true><<<blocks, kCtaThreads, smem, st>>>(a);
+        else step64_kernel<N, true, false><<<blocks, kCtaThreads, smem, st>>>(a);
+      } else {
+        if (out.mcz) step64_kernel<N, false, true><<<blocks, kCtaThreads, smem, st>>>(a);
+        else step64_kernel<N, false, false><<<blocks, kCtaThreads, smem, st>>>(a);
+      }
+      cuda_check(cudaGetLastError(), "step64_kernel launch");
     }
-    cuda_check(cudaGetLastError(), "normals64 launch");
-    const unsigned blocks = (unsigned)((a.npaths + cta_paths(N) - 1) / cta_paths(N));
-    if (lv) {
-      if (out.mcz) step64_kernel<N, true, true><<<blocks, 32 * kStepWarps, smem, st>>>(a);
-      else step64_kernel<N, true, false><<<blocks, 32 * kStepWarps, smem, st>>>(a);
-    } else {
-      if (out.mcz) step64_kernel<N, false, true><<<blocks, 32 * kStepWarps, smem, st>>>(a);
-      else step64_kernel<N, false, false><<<blocks, 32 * kStepWarps, smem, st>>>(a);
-    }
-    cuda_check(cudaGetLastError(), "step64_kernel launch");
     a.partial += (size_t)blocks * RG_ACC;
   }
 }
@@ -425,8 +506,9 @@ void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario
 
 uint64_t path64_rows(int n, uint64_t npaths) { return (npaths + cta_paths(n) - 1) / cta_paths(n); }
 
-size_t path64_bytes(int n, int64_t T, uint64_t npaths) {
-  return (size_t)(chunk_of(n, T, npaths) * (uint64_t)T * n * sizeof(double));
+size_t path64_bytes(int n, int64_t T, uint64_t npaths, size_t limit) {
+  const Path64Plan p = path64_plan(n, T, npaths, limit);
+  return p.y_bytes + p.state_bytes;
 }
 
 void launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen, uint64_t path0,

@@ -130,15 +130,18 @@ enum WsSlot {
   WS_ARENA = 0, WS_CALIB, WS_LVROWS, WS_PARTIAL, WS_SUMS, WS_KOSTEPS, WS_RECORDS,
   WS_MCZ, WS_MCKEYS, WS_MCAUX,  // the pseudo-random lane's normals, keystream and parse tables
   WS_CUBE,                      // f32 spot cube of a materialised path range
-  WS_NORMALS64,                 // correlated normals of a chunk of the FP64 lane's paths
+  WS_NORMALS64,                 // correlated normals and path states of a chunk of the FP64 lane's paths
   WS_NSLOTS
 };
+// The FP64 lane's buffer at most.
+constexpr size_t kNormals64Bytes = size_t(1) << 30;
 struct SurfaceCache;
 struct Workspace {
   cudaStream_t stream = nullptr;
   cudaEvent_t* ev = nullptr;    // six events for the timing breakdown, or null
   rg_timing* timing = nullptr;  // or null
   int sm_count = 0;
+  size_t normals64_limit = kNormals64Bytes;  // bytes of the FP64 lane's buffer (path64.cu)
   virtual void begin_launch() {}
   virtual void* device(int slot, size_t bytes) = 0;
   virtual void* host(size_t bytes) = 0;  // landing area of the FP64 sums
@@ -245,9 +248,9 @@ struct LaunchOut {
 // StandardNormal draws [first, first + count) of ChaCha8Rng::seed_from_u64(seed) into d_out.
 void mc_normals(uint64_t seed, uint64_t first, uint64_t count, double* d_out, Workspace& W);
 // The FP64 lane through a workspace that keeps its buffers (path64.cu): rows of partial sums for an
-// asset count, device bytes of its chunk buffer, and the launch.
+// asset count, device bytes of its buffer (about `limit` at most), and the launch.
 uint64_t path64_rows(int n, uint64_t npaths);
-size_t path64_bytes(int n, int64_t T, uint64_t npaths);
+size_t path64_bytes(int n, int64_t T, uint64_t npaths, size_t limit);
 void launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen_dev, uint64_t path0,
                    uint64_t npaths, const LaunchOut& out, cudaStream_t s);
 // The same in one kernel and no buffer, for the static entry point (phoenix64.cu).

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 
+import numpy as np
 import pytest
 
 from riga_gb300 import abi, workloads
@@ -105,3 +106,43 @@ def test_initial_spots_agree(engine, init, terms):
     req.trade.initial_spots = [init * (1.0 + 0.1 * f) for f in range(3)]
     req.market.spots = [s * 1.01 for s in req.trade.initial_spots]
     _check(engine, req)
+
+
+def _as_array(records):
+    return np.ctypeslib.as_array(records)
+
+
+@pytest.mark.parametrize("n,paths,steps,lane,smile", [
+    (1, 9001, 15001, "shift", None), (3, 3205, 14999, "shift", None), (2, 5000, 15000, "owen", (13, 2, 40)),
+    (5, 1801, 15013, "owen", None), (4, 2305, 15000, "none", None), (1, 8300, 16384, "none", (13, 2, 40))])
+def test_windows_of_long_schedules_agree(engine, n, paths, steps, lane, smile):
+    """Schedules too long for the buffer to hold all paths' normals pass through it in windows of steps, each
+    path's state carried between them: the records of every path have the bytes of launches of a few paths,
+    whose whole schedules it holds, and the path sums those of the records."""
+    req = _request(n, paths, steps, smile, "owen" if lane == "none" else lane)
+    if lane == "shift":
+        req.options.dim_mode = abi.DIM_WRAP_REFERENCE
+    if lane == "none":
+        req.config.variance_reduction = VarianceReduction("none", n * steps)
+    assert n * paths * steps * 8 > 1 << 30
+    whole = _as_array(engine.run_paths_raw(req, 0, paths)).copy()
+    cuts = [0, 1, 700, 1500, paths] if paths < 2400 else [0, 700, 701, paths // 2, paths]
+    parts = [_as_array(engine.run_paths_raw(req, a, b - a)).copy() for a, b in zip(cuts, cuts[1:])]
+    assert all(n * (b - a) * steps * 8 <= 1 << 30 for a, b in zip(cuts, cuts[1:]))
+    split = np.concatenate(parts)
+    for field in whole.dtype.names:
+        np.testing.assert_array_equal(whole[field], split[field])
+    got = engine.price_raw(req)
+    assert got.ko_count == int((whole["knocked_out"] != 0).sum())
+    assert abs(got.pv - whole["pv"].mean()) <= 10.0 * paths * 2.0 ** -53
+
+
+def test_windows_fill_the_spot_cube(engine):
+    """A cube of long paths, whose normals pass through the buffer in windows, equals its halves."""
+    req = _request(1, 600, 240001, None, "owen")
+    whole, _ = engine.materialize_paths(req, 0, 600)
+    low, _ = engine.materialize_paths(req, 0, 299)
+    high, _ = engine.materialize_paths(req, 299, 301)
+    w = np.asarray(whole.data)
+    assert np.array_equal(w[:299 * 240001], np.asarray(low.data))
+    assert np.array_equal(w[299 * 240001:], np.asarray(high.data))
