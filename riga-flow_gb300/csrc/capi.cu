@@ -712,11 +712,14 @@ size_t estimate_price_bytes(const rg_price_request* r, int n_scen) {
     if (fp32) b += surf * T * gx * 8;                                            // step rows
   }
   if (fp32) b += T * 160 + sobol_lut_words(r->config, (int)n, (int64_t)T) * 4;  // bridge plans, Sobol tables
-  // rows of partial sums: one per 32-path chunk (FP32 kernels) or per block (FP64 kernel)
-  const size_t grid = (size_t)(fp32 ? p32_chunks(r->config.paths) : path64_rows((int)std::min<size_t>(n, RG_NMAX), r->config.paths));
-  if (!fp32) b += path64_bytes((int)std::min<size_t>(n, RG_NMAX), (int64_t)T, r->config.paths, kNormals64Bytes);
-  b += grid * std::min<size_t>(S, 32) * RG_ACC * 8 + S * RG_ACC * 8;  // partial and reduced sums
-  b += reduce_scratch_doubles((int)std::min<size_t>(grid, INT32_MAX), (int)std::min<size_t>(S, 32)) * 8;
+  // the FP64 lane's kernels price FP64 requests and every request of the pseudo-random lane, one scenario
+  // a launch; rows of partial sums: one per 32-path chunk (FP32 kernels) or per block (FP64)
+  const bool lane64 = !fp32 || r->config.variance_reduction == RG_VR_NONE;
+  const int n64 = (int)std::min<size_t>(n, RG_NMAX), per_launch = lane64 ? 1 : (int)std::min<size_t>(S, 32);
+  const size_t grid = (size_t)(lane64 ? path64_rows(n64, r->config.paths) : p32_chunks(r->config.paths));
+  if (lane64) b += path64_bytes(n64, (int64_t)T, r->config.paths, kNormals64Bytes);
+  b += grid * per_launch * RG_ACC * 8 + S * RG_ACC * 8;  // partial and reduced sums
+  b += reduce_scratch_doubles((int)std::min<size_t>(grid, INT32_MAX), per_launch) * 8;
   if (r->config.trace_level != RG_TRACE_OFF) b += (size_t)r->config.paths * 4;
   return b + b / 4 + (size_t(1) << 20);
 }

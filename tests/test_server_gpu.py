@@ -269,3 +269,16 @@ def test_small_requests_pass_large_ones_waiting_for_a_large_slot():
         i1 = srv.wait(t1)
     assert i3.end_s <= i2.start_s, (i3.end_s, i2.start_s)
     assert i2.start_s >= i1.end_s, (i2.start_s, i1.end_s)
+
+
+def test_estimates_count_the_fp64_lane_of_pseudo_random_requests():
+    """Requests without variance reduction run on the FP64 lane's kernels whatever their precision, so the
+    estimate of one in FP32 holds the lane's buffer too: 2^14 paths x 252 steps x 3 assets of normals."""
+    from riga_gb300.types import VarianceReduction
+    est = {}
+    with Server(slots=1) as srv:
+        for fp32 in (False, True):
+            req = workloads.plain3(paths=1 << 14, steps=252, fp32=fp32)
+            req.config.variance_reduction = VarianceReduction("none", 3 * 252)
+            est[fp32] = srv.wait(srv.submit_price(req)).device_bytes
+    assert est[True] >= est[False] >= (1 << 14) * 252 * 3 * 8
