@@ -35,7 +35,7 @@ void cuda_check(cudaError_t e, const char* what) {
 
 // Capacity for n bytes: below 1 GiB the next power of two, so that requests of growing size
 // re-allocate a few times rather than at every step (cudaFree waits for the whole device).
-static size_t grown(size_t n) {
+size_t buffer_capacity(size_t n) {
   if (n < 256) return 256;
   if (n >= (size_t(1) << 30)) return n;
   size_t c = 256;
@@ -45,7 +45,7 @@ static size_t grown(size_t n) {
 void DevBuf::ensure(size_t n) {
   if (n <= bytes && ptr) return;
   release();
-  const size_t want = grown(n);
+  const size_t want = buffer_capacity(n);
   cuda_check(cudaMalloc(&ptr, want), "cudaMalloc");
   bytes = want;
 }
@@ -57,7 +57,7 @@ void DevBuf::release() {
 void HostBuf::ensure(size_t n) {
   if (n <= bytes && ptr) return;
   release();
-  const size_t want = grown(n);
+  const size_t want = buffer_capacity(n);
   cuda_check(cudaMallocHost(&ptr, want), "cudaMallocHost");
   bytes = want;
 }
@@ -666,11 +666,12 @@ int engine_sm_count(const rg_engine* E) {
   return E->sm_cap > 0 && E->sm_cap < sms ? E->sm_cap : sms;
 }
 
-void engine_set_class(rg_engine* E, bool high_priority, int sm_cap) {
+void engine_set_class(rg_engine* E, bool high_priority, int sm_cap, size_t normals64_limit) {
   std::lock_guard<std::mutex> lock(E->mu);
   E->stream = high_priority ? E->stream_hi : E->stream_lo;
   E->gen_stream = high_priority ? E->gen_stream_hi : E->gen_stream_lo;
   E->sm_cap = sm_cap;
+  E->normals64_limit = normals64_limit;
 }
 
 // The engine's workspace: growable device buffers, pinned host sums, timing events.
@@ -681,6 +682,7 @@ struct EngineWorkspace : Workspace {
     ev = e->ev;
     timing = &e->timing;
     sm_count = engine_sm_count(e);
+    normals64_limit = e->normals64_limit;
   }
   void* device(int slot, size_t bytes) override {
     E->bufs[slot].ensure(bytes);
@@ -693,7 +695,7 @@ struct EngineWorkspace : Workspace {
   SurfaceCache* surfaces() override { return &E->surfaces; }
 };
 
-size_t estimate_price_bytes(const rg_price_request* r, int n_scen) {
+size_t estimate_price_bytes(const rg_price_request* r, int n_scen, size_t normals64_limit) {
   const size_t S = n_scen > 0 ? (size_t)n_scen : 1;
   const size_t n = (size_t)(r->market.n_assets > 0 ? r->market.n_assets : 1);
   const size_t T = (size_t)(r->trade.steps > 0 ? r->trade.steps : 1);
@@ -717,11 +719,13 @@ size_t estimate_price_bytes(const rg_price_request* r, int n_scen) {
   const bool lane64 = !fp32 || r->config.variance_reduction == RG_VR_NONE;
   const int n64 = (int)std::min<size_t>(n, RG_NMAX), per_launch = lane64 ? 1 : (int)std::min<size_t>(S, 32);
   const size_t grid = (size_t)(lane64 ? path64_rows(n64, r->config.paths) : p32_chunks(r->config.paths));
-  if (lane64) b += path64_bytes(n64, (int64_t)T, r->config.paths, kNormals64Bytes);
   b += grid * per_launch * RG_ACC * 8 + S * RG_ACC * 8;  // partial and reduced sums
   b += reduce_scratch_doubles((int)std::min<size_t>(grid, INT32_MAX), per_launch) * 8;
   if (r->config.trace_level != RG_TRACE_OFF) b += (size_t)r->config.paths * 4;
-  return b + b / 4 + (size_t(1) << 20);
+  // the lane's buffer at its capacity; the rest with a margin for its smaller buffers' capacities
+  const size_t axis = r->n_local_vol ? n * (size_t)(r->config.lv_grid_x > 0 ? r->config.lv_grid_x : 96) * 16 : 0;
+  const size_t normals = lane64 ? buffer_capacity(path64_bytes(n64, (int64_t)T, r->config.paths, axis, normals64_limit)) : 0;
+  return b + b / 4 + normals + (size_t(1) << 20);
 }
 
 size_t engine_device_bytes(rg_engine* E) {

@@ -418,7 +418,8 @@ int stack_bound(int64_t T) {
 struct Path64Plan {
   uint64_t chunk;
   int64_t window;
-  size_t y_bytes, state_bytes;
+  size_t y_bytes, state_bytes, axis_bytes;
+  size_t bytes() const { return axis_bytes + state_bytes + y_bytes; }
 };
 // Whole schedules of all paths where `limit` bytes hold them, else of chunks of about equal path counts
 // as long as a chunk has kFillCtas CTAs.  Long schedules, whose chunks would leave SMs without work, pass
@@ -429,7 +430,8 @@ struct Path64Plan {
 // one kernel took 5,096; 1000 paths x 200,000 steps 1,638 and 362.
 constexpr uint64_t kFillCtas = 152 * 8;
 constexpr int64_t kMinWindow = 16;
-Path64Plan path64_plan(int n, int64_t T, uint64_t npaths, size_t limit) {
+Path64Plan path64_plan(int n, int64_t T, uint64_t npaths, size_t axis_bytes, size_t limit) {
+  limit -= std::min(limit, axis_bytes);
   const uint64_t unit = cta_paths(n), ctas = (npaths + unit - 1) / unit;
   const uint64_t row = unit * n * sizeof(double);  // a CTA's normals of one node
   const uint64_t fit = limit / (row * (uint64_t)T);
@@ -439,7 +441,7 @@ Path64Plan path64_plan(int n, int64_t T, uint64_t npaths, size_t limit) {
   };
   if (fit >= std::min(ctas, kFillCtas)) {
     const uint64_t per = even(fit);
-    return {per * unit, T, (size_t)(per * row * (uint64_t)T), 0};
+    return {per * unit, T, (size_t)(per * row * (uint64_t)T), 0, axis_bytes};
   }
   const uint64_t depth = (uint64_t)stack_bound(T), state = (kStateWords + depth) * kCtaThreads * sizeof(double);
   const uint64_t shortest = std::min<uint64_t>(kMinWindow, (uint64_t)T);
@@ -447,7 +449,7 @@ Path64Plan path64_plan(int n, int64_t T, uint64_t npaths, size_t limit) {
   // a window's steps consume at most `depth` nodes more than it has steps
   const uint64_t nodes = per * state < limit ? (limit - per * state) / (per * row) : 0;
   const uint64_t window = std::min<uint64_t>(std::max<uint64_t>(nodes, depth + 1) - depth, (uint64_t)T);
-  return {per * unit, (int64_t)window, (size_t)(per * row * (window + depth)), (size_t)(per * state)};
+  return {per * unit, (int64_t)window, (size_t)(per * row * (window + depth)), (size_t)(per * state), axis_bytes};
 }
 
 template <int N>
@@ -455,11 +457,11 @@ void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario
          const LaunchOut& out, cudaStream_t st) {
   const int64_t T = P.T;
   const bool lv = P.trade.has_lv != 0;
-  const Path64Plan plan = path64_plan(N, T, npaths, W.normals64_limit);
+  const size_t axis_bytes = lv ? (size_t)P.n_surf * P.trade.gx * sizeof(double2) : 0;
+  const Path64Plan plan = path64_plan(N, T, npaths, axis_bytes, W.normals64_limit);
   const uint64_t chunk = plan.chunk, unit = cta_paths(N);
   if (P.stack_max > stack_bound(T)) raise(RG_ERR_INVALID_SCHEDULE, "path64: the bridge stack is too deep");
-  const size_t axis_bytes = lv ? (size_t)P.n_surf * P.trade.gx * sizeof(double2) : 0;
-  uint8_t* buf = static_cast<uint8_t*>(W.device(WS_NORMALS64, axis_bytes + plan.state_bytes + plan.y_bytes));
+  uint8_t* buf = static_cast<uint8_t*>(W.device(WS_NORMALS64, plan.bytes()));
   double* state = reinterpret_cast<double*>(buf + axis_bytes);
   double* y = reinterpret_cast<double*>(buf + axis_bytes + plan.state_bytes);
   Step64Args a{P.trade, tb, scen, y, reinterpret_cast<const double2*>(buf), chunk, path0, 0, 0, 0, 0, 0, 0, state,
@@ -506,9 +508,8 @@ void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario
 
 uint64_t path64_rows(int n, uint64_t npaths) { return (npaths + cta_paths(n) - 1) / cta_paths(n); }
 
-size_t path64_bytes(int n, int64_t T, uint64_t npaths, size_t limit) {
-  const Path64Plan p = path64_plan(n, T, npaths, limit);
-  return p.y_bytes + p.state_bytes;
+size_t path64_bytes(int n, int64_t T, uint64_t npaths, size_t axis_bytes, size_t limit) {
+  return path64_plan(n, T, npaths, axis_bytes, limit).bytes();
 }
 
 void launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen, uint64_t path0,

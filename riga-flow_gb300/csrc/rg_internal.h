@@ -38,6 +38,8 @@ struct DevBuf {
   ~DevBuf() { release(); }
 };
 
+// The capacity that a growing buffer takes for n bytes.
+size_t buffer_capacity(size_t n);
 // A pinned host buffer that only grows.
 struct HostBuf {
   void* ptr = nullptr;
@@ -248,9 +250,10 @@ struct LaunchOut {
 // StandardNormal draws [first, first + count) of ChaCha8Rng::seed_from_u64(seed) into d_out.
 void mc_normals(uint64_t seed, uint64_t first, uint64_t count, double* d_out, Workspace& W);
 // The FP64 lane through a workspace that keeps its buffers (path64.cu): rows of partial sums for an
-// asset count, device bytes of its buffer (about `limit` at most), and the launch.
+// asset count, device bytes of its buffer (`limit` at most, or what one CTA needs) with the surfaces'
+// axes, and the launch.
 uint64_t path64_rows(int n, uint64_t npaths);
-size_t path64_bytes(int n, int64_t T, uint64_t npaths, size_t limit);
+size_t path64_bytes(int n, int64_t T, uint64_t npaths, size_t axis_bytes, size_t limit);
 void launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen_dev, uint64_t path0,
                    uint64_t npaths, const LaunchOut& out, cudaStream_t s);
 // The same in one kernel and no buffer, for the static entry point (phoenix64.cu).
@@ -433,12 +436,14 @@ namespace rg {
 size_t engine_device_bytes(rg_engine* E);
 void engine_trim(rg_engine* E);
 // Before a request on an idle engine: its streams' priority (high or default) and the SMs its
-// grids are sized for (0: all), so a server's large requests leave SMs and priority to small ones.
-void engine_set_class(rg_engine* E, bool high_priority, int sm_cap);
+// grids are sized for (0: all), so a server's large requests leave SMs and priority to small ones; and
+// the bytes its FP64 lane's buffer may have.
+void engine_set_class(rg_engine* E, bool high_priority, int sm_cap, size_t normals64_limit);
 // The SM count the engine's launches size their grids for.
 int engine_sm_count(const rg_engine* E);
-// Device bytes one call will hold at its peak (workspace buffers; upper estimates).
-size_t estimate_price_bytes(const rg_price_request* r, int n_scen);
+// Device bytes one call will hold at its peak (workspace buffers; upper estimates), with the FP64 lane's
+// buffer limited to `normals64_limit` bytes.
+size_t estimate_price_bytes(const rg_price_request* r, int n_scen, size_t normals64_limit);
 size_t estimate_book_bytes(const rg_book_request* r, int n_scen);
 size_t estimate_book_trade_bumps_bytes(const rg_book_request* r);
 }  // namespace rg
@@ -453,6 +458,7 @@ struct rg_engine {
   cudaStream_t stream_lo = nullptr, gen_stream_lo = nullptr;
   cudaStream_t stream_hi = nullptr, gen_stream_hi = nullptr;
   int sm_cap = 0;  // SMs the engine's grids are sized for (0: every SM of the device)
+  size_t normals64_limit = rg::kNormals64Bytes;  // bytes of the FP64 lane's buffer
   std::mutex mu;
   rg::DevBuf bufs[rg::WS_NSLOTS];
   rg::DevBuf book_bufs[8];

@@ -154,6 +154,7 @@ struct Job {
   std::vector<OwnedMarket> book_scen;
   std::vector<rg_market_snapshot> book_scen_views;
   size_t est = 0;
+  size_t normals64_limit = kNormals64Bytes;  // bytes of the FP64 lane's buffer that the estimate holds
   double work = 0;     // path-steps × scenarios the request prices
   bool large = false;  // work at or above the server's large-work mark
   bool waited_memory = false;  // was passed over at least once because it did not fit the budget
@@ -341,7 +342,7 @@ void worker(rg_server* S, int k) {
     }
     // large requests run at default priority on a share of the SMs; small ones at the highest
     // priority on all of them, so they pass a large request's kernels
-    engine_set_class(slot.engine, !job->large, job->large ? S->large_sms : 0);
+    engine_set_class(slot.engine, !job->large, job->large ? S->large_sms : 0, job->normals64_limit);
     run_job(slot.engine, job);
     const size_t held = engine_device_bytes(slot.engine);
     lock.lock();
@@ -367,6 +368,21 @@ void worker(rg_server* S, int k) {
     S->cv_done.notify_all();
     S->cv_work.notify_all();
   }
+}
+
+// The request's estimate and the FP64 lane's buffer.  The buffer only saves time (a smaller one is passed
+// through in windows of steps, with the same results), so it takes no more than leaves the request within
+// the sixteenth of the budget that may pass waiting books, or else within the budget, where the request
+// without it lies there: 2^14 paths x 756 steps x 3 assets (290 MB) are still priced by a server of 16 MiB.
+void set_price_estimate(const rg_server* S, Job* job, int n_scen) {
+  const rg_price_request* r = &job->req.r;
+  job->est = estimate_price_bytes(r, n_scen, job->normals64_limit);
+  const size_t least = estimate_price_bytes(r, n_scen, 0), line = least <= S->budget / 16 ? S->budget / 16 : S->budget;
+  if (job->est <= line || least > line) return;
+  // the largest capacity a buffer may have
+  job->normals64_limit = kNormals64Bytes;
+  while (job->normals64_limit > line - least) job->normals64_limit >>= 1;
+  job->est = estimate_price_bytes(r, n_scen, job->normals64_limit);
 }
 
 uint64_t enqueue(rg_server* S, std::unique_ptr<Job> job) {
@@ -502,7 +518,7 @@ extern "C" int32_t rg_server_submit_price(rg_server* S, const rg_price_request* 
     }
     job->n_results = n > 0 ? (uint64_t)n : 1;
     job->results.resize(job->n_results);
-    job->est = estimate_price_bytes(&job->req.r, n);
+    set_price_estimate(S, job.get(), n);
     job->work = (double)req->config.paths * (double)req->trade.steps * (double)job->n_results;
     *ticket = enqueue(S, std::move(job));
   })
@@ -518,7 +534,7 @@ extern "C" int32_t rg_server_submit_risk(rg_server* S, const rg_price_request* r
     job->req.copy(*req);
     job->risk_cfg = *cfg;
     job->n_results = 0;
-    job->est = estimate_price_bytes(&job->req.r, 1 + 4 * req->market.n_assets + 4);
+    set_price_estimate(S, job.get(), 1 + 4 * req->market.n_assets + 4);
     job->work = (double)req->config.paths * (double)req->trade.steps * (double)(1 + 4 * req->market.n_assets + 4);
     *ticket = enqueue(S, std::move(job));
   })

@@ -282,3 +282,17 @@ def test_estimates_count_the_fp64_lane_of_pseudo_random_requests():
             req.config.variance_reduction = VarianceReduction("none", 3 * 252)
             est[fp32] = srv.wait(srv.submit_price(req)).device_bytes
     assert est[True] >= est[False] >= (1 << 14) * 252 * 3 * 8
+
+
+def test_a_small_budget_shrinks_the_fp64_buffer(engine):
+    """The FP64 lane's buffer takes what the budget leaves: a request whose tables are a few MB is accepted and
+    priced as by an engine of its own, and where it can it keeps within the sixteenth of the budget that may
+    pass a waiting book."""
+    req = workloads.plain3(paths=1 << 14, steps=756)
+    want, want_risk = bytes(engine.price_raw(req)), bytes(engine.price_risk_batch_raw(req, default_risk_config()))
+    for mib in (8, 16, 100, 128, 512, 8192):
+        with Server(slots=1, memory_budget=mib << 20) as srv:
+            t, k = srv.submit_price(req), srv.submit_risk(req)
+            info = srv.wait(t)
+            assert info.device_bytes <= mib << (16 if mib >= 128 else 20)
+            assert bytes(srv.results(t)[0]) == want and bytes(srv.risk_report(k)) == want_risk
