@@ -219,8 +219,10 @@ size_t reserved(const rg_server* S) {
 }
 
 // Under S->mu: whether `job` can start on slot k now, counting as free the buffers of the idle
-// slots listed in `trim` (the smallest set, in slot order, that makes room).  Releasing buffers
-// (cudaFree) waits for the device, so the caller does it after dropping the lock.
+// slots listed in `trim` (the smallest set, in slot order, that makes room; slot k's own last: buffers
+// have larger capacities than was estimated, and a slot that held more than the budget would never
+// start anything again).  Releasing buffers (cudaFree) waits for the device, so the caller does it after
+// dropping the lock.
 bool admit(rg_server* S, int k, const Job* job, std::vector<int>& trim) {
   trim.clear();
   size_t freed = 0;
@@ -234,6 +236,10 @@ bool admit(rg_server* S, int k, const Job* job, std::vector<int>& trim) {
     trim.push_back((int)i);
     freed += s.held;
     if (need() <= S->budget) return true;
+  }
+  if (S->slots[k].held > job->est && reserved(S) - freed - S->slots[k].held + job->est <= S->budget) {
+    trim.push_back(k);
+    return true;
   }
   trim.clear();
   return false;

@@ -296,3 +296,18 @@ def test_a_small_budget_shrinks_the_fp64_buffer(engine):
             info = srv.wait(t)
             assert info.device_bytes <= mib << (16 if mib >= 128 else 20)
             assert bytes(srv.results(t)[0]) == want and bytes(srv.risk_report(k)) == want_risk
+
+
+def test_a_slot_that_holds_more_than_the_budget_starts_the_next_request(engine):
+    """Buffers are allocated with larger capacities than a request needs, and the pseudo-random lane's stream is
+    not estimated, so a slot may hold more than the budget after a request: the next one releases them."""
+    from riga_gb300.types import VarianceReduction
+    req = workloads.plain3(paths=1 << 14, steps=252)
+    req.config.variance_reduction = VarianceReduction("none", 3 * 252)
+    want = bytes(engine.price_raw(req))
+    with Server(slots=1, memory_budget=180 << 20) as srv:
+        for _ in range(3):
+            t = srv.submit_price(req)
+            assert srv.wait(t, timeout_ms=20000).state == abi.JOB_DONE
+            assert bytes(srv.results(t)[0]) == want
+        assert srv.stats().device_bytes_held > 180 << 20
