@@ -348,7 +348,8 @@ void* book_buf(rg_engine* E, int slot, size_t bytes) {
   return E->book_bufs[slot].ptr;
 }
 
-BookStaged stage_book_static(DevBuf& tables, cudaStream_t st, const rg_book_request* r, const BookPlan& B) {
+BookStaged stage_book_static(DevBuf& tables, cudaStream_t st, const rg_book_request* r, const BookPlan& B,
+                             const ScratchLimits& limits) {
   Pack pk;
   const int U = B.U;
   size_t o_sobol = 0, o_hb = 0, o_ho = 0, o_hp = 0;
@@ -369,7 +370,7 @@ BookStaged stage_book_static(DevBuf& tables, cudaStream_t st, const rg_book_requ
   const size_t o_tr = pk.add(B.trades), o_ord = pk.add(B.order);
   const size_t o_corr = pk.add(r->universe.correlation, (size_t)U * U);
   const size_t o_L = pk.reserve(sizeof(double) * U * U), o_L32 = pk.reserve(sizeof(float) * U * U);
-  const size_t lut_words = sobol_lut_words(r->config, U, B.TU), o_lut = (pk.host.size() + 255) & ~size_t(255);
+  const size_t lut_words = limits.sobol_tables ? sobol_lut_words(r->config, U, B.TU) : 0, o_lut = (pk.host.size() + 255) & ~size_t(255);
   tables.ensure(o_lut + lut_words * sizeof(uint32_t));
   uint8_t* dev = static_cast<uint8_t*>(tables.ptr);
   cuda_check(cudaMemcpyAsync(dev, pk.host.data(), pk.host.size(), cudaMemcpyHostToDevice, st), "book H2D");
@@ -463,7 +464,7 @@ uint64_t chunk_paths(uint64_t paths, int U, int64_t TU, size_t elem, uint64_t un
 
 }  // namespace bk
 
-size_t estimate_book_bytes(const rg_book_request* r, int n_scen) {
+size_t estimate_book_bytes(const rg_book_request* r, int n_scen, const ScratchLimits& limits) {
   using namespace bk;
   const size_t S = n_scen > 0 ? (size_t)n_scen : 1;
   const size_t U = (size_t)(r->universe.n_assets > 0 ? r->universe.n_assets : 1);
@@ -480,17 +481,18 @@ size_t estimate_book_bytes(const rg_book_request* r, int n_scen) {
   const uint64_t blocks = fp32 ? (P + unit - 1) / unit : ((PC + 127) / 128) * chunks;
   b += (size_t)blocks * pairs * RG_ACC * 8 + pairs * RG_ACC * 8;
   size_t sob_rows = r->config.dim_mode == RG_DIM_FULL ? U * TU : 512;
-  b += sob_rows * 128 + sobol_lut_words(r->config, (int64_t)U, (int64_t)TU) * 4 + TU * 32 + S * TU * 12 + pairs * 100 + (size_t)r->n_trades * 256 + (size_t(64) << 10);
+  if (limits.sobol_tables) b += sobol_lut_words(r->config, (int64_t)U, (int64_t)TU) * 4;
+  b += sob_rows * 128 + TU * 32 + S * TU * 12 + pairs * 100 + (size_t)r->n_trades * 256 + (size_t(64) << 10);
   return b + b / 8 + (size_t(1) << 20);
 }
 
 // Under per-trade bump sets a book prices 16 (trade, scenario) pairs per trade, as under 16 common
 // scenarios, and plans one market per distinct bumped universe market (at most 16 per trade), each
 // with its per-step tables.
-size_t estimate_book_trade_bumps_bytes(const rg_book_request* r) {
+size_t estimate_book_trade_bumps_bytes(const rg_book_request* r, const ScratchLimits& limits) {
   const size_t TU = (size_t)(r->universe_steps > 0 ? r->universe_steps : 1);
   const size_t markets = std::min<size_t>((size_t)(r->n_trades > 0 ? r->n_trades : 1) * RG_BOOK_TRADE_SCENARIOS, 4096);
-  return estimate_book_bytes(r, RG_BOOK_TRADE_SCENARIOS) + markets * (TU * 16 + 256);
+  return estimate_book_bytes(r, RG_BOOK_TRADE_SCENARIOS, limits) + markets * (TU * 16 + 256);
 }
 
 namespace {
@@ -526,7 +528,7 @@ void run_book(rg_engine* E, const rg_book_request* r, const BookScenarios& sc, r
   plan_book(r, sc, B);
   const int pairs = B.n_trades * B.S;
   const bool fp32 = r->config.precision == RG_PRECISION_FP32 && !records;
-  BookStaged st = stage_book_static(E->book_bufs[BK_TABLES], E->stream, r, B);
+  BookStaged st = stage_book_static(E->book_bufs[BK_TABLES], E->stream, r, B, E->limits);
   {
     const ScenarioPack sp = pack_book_scenarios(B);
     uint8_t* dev = static_cast<uint8_t*>(book_buf(E, BK_SCEN, sp.pk.host.size()));

@@ -216,7 +216,7 @@ extern "C" int32_t rg_book_create(rg_engine* e, const rg_book_request* request, 
     b->universe.correlation = b->corr.data();
     b->config = request->config;
     bk::plan_book(request, bk::BookScenarios{}, b->B);
-    b->st = bk::stage_book_static(b->tables, e->stream, request, b->B);
+    b->st = bk::stage_book_static(b->tables, e->stream, request, b->B, e->limits);
     b->P = request->config.paths;
     b->rowlen = (b->P + 63) / 64 * 64;
     const size_t ibytes = sizeof(float) * (size_t)U * (size_t)b->B.TU * (size_t)b->rowlen;

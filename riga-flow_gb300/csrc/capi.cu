@@ -374,8 +374,8 @@ static Staged stage(Workspace& W, const rg_price_request* req, Prepared& P) {
   // without, and 4 us to build; 2^14 paths 0.50 against 0.55 ms); the static region holds them from
   // 2^16 paths only
   const size_t o_lut = (pk.host.size() + 255) & ~size_t(255);
-  const uint64_t lut_from = W.persistent() ? uint64_t(1) << 13 : uint64_t(1) << 16;
-  const size_t lut_words = req->config.paths >= lut_from ? sobol_lut_words(req->config, P.n, P.T) : 0;
+  const uint64_t lut_from = W.persistent() ? kSobolLutPaths : uint64_t(1) << 16;
+  const size_t lut_words = W.limits.sobol_tables && req->config.paths >= lut_from ? sobol_lut_words(req->config, P.n, P.T) : 0;
   uint8_t* base = static_cast<uint8_t*>(W.device(WS_ARENA, o_lut + lut_words * sizeof(uint32_t)));
   if (tr.has_lv) {
     if (SurfaceCache* cache = W.surfaces()) cache->begin_call();
@@ -666,12 +666,12 @@ int engine_sm_count(const rg_engine* E) {
   return E->sm_cap > 0 && E->sm_cap < sms ? E->sm_cap : sms;
 }
 
-void engine_set_class(rg_engine* E, bool high_priority, int sm_cap, size_t normals64_limit) {
+void engine_set_class(rg_engine* E, bool high_priority, int sm_cap, const ScratchLimits& limits) {
   std::lock_guard<std::mutex> lock(E->mu);
   E->stream = high_priority ? E->stream_hi : E->stream_lo;
   E->gen_stream = high_priority ? E->gen_stream_hi : E->gen_stream_lo;
   E->sm_cap = sm_cap;
-  E->normals64_limit = normals64_limit;
+  E->limits = limits;
 }
 
 // The engine's workspace: growable device buffers, pinned host sums, timing events.
@@ -682,7 +682,7 @@ struct EngineWorkspace : Workspace {
     ev = e->ev;
     timing = &e->timing;
     sm_count = engine_sm_count(e);
-    normals64_limit = e->normals64_limit;
+    limits = e->limits;
   }
   void* device(int slot, size_t bytes) override {
     E->bufs[slot].ensure(bytes);
@@ -695,7 +695,7 @@ struct EngineWorkspace : Workspace {
   SurfaceCache* surfaces() override { return &E->surfaces; }
 };
 
-size_t estimate_price_bytes(const rg_price_request* r, int n_scen, size_t normals64_limit) {
+size_t estimate_price_bytes(const rg_price_request* r, int n_scen, const ScratchLimits& limits) {
   const size_t S = n_scen > 0 ? (size_t)n_scen : 1;
   const size_t n = (size_t)(r->market.n_assets > 0 ? r->market.n_assets : 1);
   const size_t T = (size_t)(r->trade.steps > 0 ? r->trade.steps : 1);
@@ -713,7 +713,8 @@ size_t estimate_price_bytes(const rg_price_request* r, int n_scen, size_t normal
     b += surf * ((2 * nt * gx + gx) * 8 + (4 * nt * gx + gx + 6 * nt * nk) * 8);  // calibration
     if (fp32) b += surf * T * gx * 8;                                            // step rows
   }
-  if (fp32) b += T * 160 + sobol_lut_words(r->config, (int)n, (int64_t)T) * 4;  // bridge plans, Sobol tables
+  if (fp32) b += T * 160;  // bridge plans
+  if (limits.sobol_tables && r->config.paths >= kSobolLutPaths) b += sobol_lut_words(r->config, (int)n, (int64_t)T) * 4;
   // the FP64 lane's kernels price FP64 requests and every request of the pseudo-random lane, one scenario
   // a launch; rows of partial sums: one per 32-path chunk (FP32 kernels) or per block (FP64)
   const bool lane64 = !fp32 || r->config.variance_reduction == RG_VR_NONE;
@@ -724,7 +725,7 @@ size_t estimate_price_bytes(const rg_price_request* r, int n_scen, size_t normal
   if (r->config.trace_level != RG_TRACE_OFF) b += (size_t)r->config.paths * 4;
   // the lane's buffer at its capacity; the rest with a margin for its smaller buffers' capacities
   const size_t axis = r->n_local_vol ? n * (size_t)(r->config.lv_grid_x > 0 ? r->config.lv_grid_x : 96) * 16 : 0;
-  const size_t normals = lane64 ? buffer_capacity(path64_bytes(n64, (int64_t)T, r->config.paths, axis, normals64_limit)) : 0;
+  const size_t normals = lane64 ? buffer_capacity(path64_bytes(n64, (int64_t)T, r->config.paths, axis, limits.normals64)) : 0;
   return b + b / 4 + normals + (size_t(1) << 20);
 }
 

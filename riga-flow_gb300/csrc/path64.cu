@@ -458,7 +458,7 @@ void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario
   const int64_t T = P.T;
   const bool lv = P.trade.has_lv != 0;
   const size_t axis_bytes = lv ? (size_t)P.n_surf * P.trade.gx * sizeof(double2) : 0;
-  const Path64Plan plan = path64_plan(N, T, npaths, axis_bytes, W.normals64_limit);
+  const Path64Plan plan = path64_plan(N, T, npaths, axis_bytes, W.limits.normals64);
   const uint64_t chunk = plan.chunk, unit = cta_paths(N);
   if (P.stack_max > stack_bound(T)) raise(RG_ERR_INVALID_SCHEDULE, "path64: the bridge stack is too deep");
   uint8_t* buf = static_cast<uint8_t*>(W.device(WS_NORMALS64, plan.bytes()));

@@ -53,7 +53,8 @@ struct BookStaged {
 };
 // QMC tables, bridge schedule, trades, work order and the universe factor (FP64 Cholesky on the
 // device, then its FP32 copy) into `tables`, enqueued on `st`.
-BookStaged stage_book_static(DevBuf& tables, cudaStream_t st, const rg_book_request* r, const BookPlan& B);
+BookStaged stage_book_static(DevBuf& tables, cudaStream_t st, const rg_book_request* r, const BookPlan& B,
+                             const ScratchLimits& limits);
 
 // The scenario tables packed for one H2D copy; point_scenarios aims `bk` at their device copy.
 struct ScenarioPack {

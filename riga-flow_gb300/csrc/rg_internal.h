@@ -135,15 +135,19 @@ enum WsSlot {
   WS_NORMALS64,                 // correlated normals and path states of a chunk of the FP64 lane's paths
   WS_NSLOTS
 };
-// The FP64 lane's buffer at most.
-constexpr size_t kNormals64Bytes = size_t(1) << 30;
+// Device memory that only saves time: the FP64 lane's buffer at most, and whether the FP32 kernels' Sobol
+// tables are built.  A server's budget may want less.
+struct ScratchLimits {
+  size_t normals64 = size_t(1) << 30;
+  bool sobol_tables = true;
+};
 struct SurfaceCache;
 struct Workspace {
   cudaStream_t stream = nullptr;
   cudaEvent_t* ev = nullptr;    // six events for the timing breakdown, or null
   rg_timing* timing = nullptr;  // or null
   int sm_count = 0;
-  size_t normals64_limit = kNormals64Bytes;  // bytes of the FP64 lane's buffer (path64.cu)
+  ScratchLimits limits;
   virtual void begin_launch() {}
   virtual void* device(int slot, size_t bytes) = 0;
   virtual void* host(size_t bytes) = 0;  // landing area of the FP64 sums
@@ -176,6 +180,8 @@ inline size_t sobol_lut_words(const rg_simulation_config& c, int64_t n, int64_t 
   const size_t w = (size_t)64 * (size_t)n * (size_t)T;
   return c.precision == RG_PRECISION_FP32 && c.variance_reduction == RG_VR_SOBOL && w <= (size_t(1) << 27) ? w : 0;
 }
+// Paths from which a price's launches build those tables.
+constexpr uint64_t kSobolLutPaths = uint64_t(1) << 13;
 // The first `count` primes (a copy of a process-wide cache; at least `count` entries).
 std::vector<uint32_t> first_primes(int count);
 // Halton bases and permutations.
@@ -437,15 +443,14 @@ size_t engine_device_bytes(rg_engine* E);
 void engine_trim(rg_engine* E);
 // Before a request on an idle engine: its streams' priority (high or default) and the SMs its
 // grids are sized for (0: all), so a server's large requests leave SMs and priority to small ones; and
-// the bytes its FP64 lane's buffer may have.
-void engine_set_class(rg_engine* E, bool high_priority, int sm_cap, size_t normals64_limit);
+// its scratch limits.
+void engine_set_class(rg_engine* E, bool high_priority, int sm_cap, const ScratchLimits& limits);
 // The SM count the engine's launches size their grids for.
 int engine_sm_count(const rg_engine* E);
-// Device bytes one call will hold at its peak (workspace buffers; upper estimates), with the FP64 lane's
-// buffer limited to `normals64_limit` bytes.
-size_t estimate_price_bytes(const rg_price_request* r, int n_scen, size_t normals64_limit);
-size_t estimate_book_bytes(const rg_book_request* r, int n_scen);
-size_t estimate_book_trade_bumps_bytes(const rg_book_request* r);
+// Device bytes one call will hold at its peak (workspace buffers; upper estimates).
+size_t estimate_price_bytes(const rg_price_request* r, int n_scen, const ScratchLimits& limits);
+size_t estimate_book_bytes(const rg_book_request* r, int n_scen, const ScratchLimits& limits);
+size_t estimate_book_trade_bumps_bytes(const rg_book_request* r, const ScratchLimits& limits);
 }  // namespace rg
 
 // The engine behind the opaque C handle.
@@ -458,7 +463,7 @@ struct rg_engine {
   cudaStream_t stream_lo = nullptr, gen_stream_lo = nullptr;
   cudaStream_t stream_hi = nullptr, gen_stream_hi = nullptr;
   int sm_cap = 0;  // SMs the engine's grids are sized for (0: every SM of the device)
-  size_t normals64_limit = rg::kNormals64Bytes;  // bytes of the FP64 lane's buffer
+  rg::ScratchLimits limits;
   std::mutex mu;
   rg::DevBuf bufs[rg::WS_NSLOTS];
   rg::DevBuf book_bufs[8];

@@ -154,7 +154,7 @@ struct Job {
   std::vector<OwnedMarket> book_scen;
   std::vector<rg_market_snapshot> book_scen_views;
   size_t est = 0;
-  size_t normals64_limit = kNormals64Bytes;  // bytes of the FP64 lane's buffer that the estimate holds
+  ScratchLimits limits;  // what the estimate holds
   double work = 0;     // path-steps × scenarios the request prices
   bool large = false;  // work at or above the server's large-work mark
   bool waited_memory = false;  // was passed over at least once because it did not fit the budget
@@ -348,7 +348,7 @@ void worker(rg_server* S, int k) {
     }
     // large requests run at default priority on a share of the SMs; small ones at the highest
     // priority on all of them, so they pass a large request's kernels
-    engine_set_class(slot.engine, !job->large, job->large ? S->large_sms : 0, job->normals64_limit);
+    engine_set_class(slot.engine, !job->large, job->large ? S->large_sms : 0, job->limits);
     run_job(slot.engine, job);
     const size_t held = engine_device_bytes(slot.engine);
     lock.lock();
@@ -376,19 +376,27 @@ void worker(rg_server* S, int k) {
   }
 }
 
-// The request's estimate and the FP64 lane's buffer.  The buffer only saves time (a smaller one is passed
-// through in windows of steps, with the same results), so it takes no more than leaves the request within
-// the sixteenth of the budget that may pass waiting books, or else within the budget, where the request
-// without it lies there: 2^14 paths x 756 steps x 3 assets (290 MB) are still priced by a server of 16 MiB.
-void set_price_estimate(const rg_server* S, Job* job, int n_scen) {
-  const rg_price_request* r = &job->req.r;
-  job->est = estimate_price_bytes(r, n_scen, job->normals64_limit);
-  const size_t least = estimate_price_bytes(r, n_scen, 0), line = least <= S->budget / 16 ? S->budget / 16 : S->budget;
-  if (job->est <= line || least > line) return;
-  // the largest capacity a buffer may have
-  job->normals64_limit = kNormals64Bytes;
-  while (job->normals64_limit > line - least) job->normals64_limit >>= 1;
-  job->est = estimate_price_bytes(r, n_scen, job->normals64_limit);
+// The request's estimate and its scratch limits.  The FP64 lane's buffer and the Sobol tables only save
+// time (a smaller buffer is passed through in windows of steps, points without tables are formed one by
+// one, with the same results), so they take no more than leaves the request within the sixteenth of the
+// budget that may pass waiting books, or else within the budget, where the request without them lies there:
+// 2^14 paths x 756 steps x 3 assets in FP64 (290 MB) are still priced by a server of 16 MiB.
+template <class Estimate>
+void set_estimate(const rg_server* S, Job* job, Estimate estimate) {
+  ScratchLimits& l = job->limits;
+  job->est = estimate(l);
+  ScratchLimits least;
+  least.normals64 = 0;
+  least.sobol_tables = false;
+  const size_t low = estimate(least), line = low <= S->budget / 16 ? S->budget / 16 : S->budget;
+  if (job->est <= line || low > line) return;
+  least.sobol_tables = true;
+  l.sobol_tables = estimate(least) <= line;
+  least.sobol_tables = l.sobol_tables;
+  // the largest capacity the buffer may have
+  const size_t room = line - estimate(least);
+  while (l.normals64 > room) l.normals64 >>= 1;
+  job->est = estimate(l);
 }
 
 uint64_t enqueue(rg_server* S, std::unique_ptr<Job> job) {
@@ -524,7 +532,7 @@ extern "C" int32_t rg_server_submit_price(rg_server* S, const rg_price_request* 
     }
     job->n_results = n > 0 ? (uint64_t)n : 1;
     job->results.resize(job->n_results);
-    set_price_estimate(S, job.get(), n);
+    set_estimate(S, job.get(), [&](const ScratchLimits& l) { return estimate_price_bytes(&job->req.r, n, l); });
     job->work = (double)req->config.paths * (double)req->trade.steps * (double)job->n_results;
     *ticket = enqueue(S, std::move(job));
   })
@@ -540,7 +548,8 @@ extern "C" int32_t rg_server_submit_risk(rg_server* S, const rg_price_request* r
     job->req.copy(*req);
     job->risk_cfg = *cfg;
     job->n_results = 0;
-    set_price_estimate(S, job.get(), 1 + 4 * req->market.n_assets + 4);
+    const int n_scen = 1 + 4 * req->market.n_assets + 4;
+    set_estimate(S, job.get(), [&](const ScratchLimits& l) { return estimate_price_bytes(&job->req.r, n_scen, l); });
     job->work = (double)req->config.paths * (double)req->trade.steps * (double)(1 + 4 * req->market.n_assets + 4);
     *ticket = enqueue(S, std::move(job));
   })
@@ -562,7 +571,7 @@ extern "C" int32_t rg_server_submit_book(rg_server* S, const rg_book_request* re
     const uint64_t S_ = n > 0 ? (uint64_t)n : 1;
     job->n_results = (uint64_t)(req->n_trades > 0 ? req->n_trades : 0) * S_;
     job->results.resize(job->n_results);
-    job->est = estimate_book_bytes(&job->book.r, n);
+    set_estimate(S, job.get(), [&](const ScratchLimits& l) { return estimate_book_bytes(&job->book.r, n, l); });
     double steps = (double)req->universe_steps * (double)req->universe.n_assets;  // the universe generation
     for (int32_t j = 0; j < req->n_trades; ++j) steps += (double)req->trades[j].terms.steps * (double)S_;
     job->work = (double)req->config.paths * steps;
@@ -584,7 +593,7 @@ extern "C" int32_t rg_server_submit_book_trade_bumps(rg_server* S, const rg_book
     const uint64_t S_ = RG_BOOK_TRADE_SCENARIOS;
     job->n_results = (uint64_t)(req->n_trades > 0 ? req->n_trades : 0) * S_;
     job->results.resize(job->n_results);
-    job->est = estimate_book_trade_bumps_bytes(&job->book.r);
+    set_estimate(S, job.get(), [&](const ScratchLimits& l) { return estimate_book_trade_bumps_bytes(&job->book.r, l); });
     double steps = (double)req->universe_steps * (double)req->universe.n_assets;  // the universe generation
     for (int32_t j = 0; j < req->n_trades; ++j) steps += (double)req->trades[j].terms.steps * (double)S_;
     job->work = (double)req->config.paths * steps;

@@ -311,3 +311,36 @@ def test_a_slot_that_holds_more_than_the_budget_starts_the_next_request(engine):
             assert srv.wait(t, timeout_ms=20000).state == abi.JOB_DONE
             assert bytes(srv.results(t)[0]) == want
         assert srv.stats().device_bytes_held > 180 << 20
+
+
+@pytest.mark.parametrize("kind", ["price", "book"])
+def test_a_small_budget_does_without_sobol_tables(engine, kind):
+    """The FP32 kernels' Sobol tables are counted for the launches that build them, and a request that crosses
+    the budget (or the sixteenth of it that may pass a waiting book) only by them is priced without: the
+    same bytes.  Sizes of both estimates from servers with room: 256 bytes of tables per step and asset."""
+    if kind == "price":
+        req = workloads.lv3(paths=20011, steps=252, fp32=True)
+        want, margin, tables = [bytes(engine.price_raw(req))], 4, 256 * 3 * 252
+        submit = lambda srv: srv.submit_price(req)
+    else:
+        req = workloads.small_book(paths=3001, n_trades=4, steps_per_year=52, fp32=True)
+        want, margin = [bytes(r) for r in engine.price_book_raw(req)], 8
+        tables = 256 * len(req.universe.spots) * req.universe_steps
+        submit = lambda srv: srv.submit_book(req)
+    with Server(slots=1, memory_budget=1 << 62) as srv:
+        full = srv.wait(submit(srv)).device_bytes
+    without = full - tables - tables // margin
+    for budget, est in ((full, full), (full - 1, without), (without + 16, without), (16 * full, full),
+                        (16 * full - 16, without)):
+        with Server(slots=1, memory_budget=budget) as srv:
+            for _ in range(2):
+                t = submit(srv)
+                info = srv.wait(t, timeout_ms=20000)
+                assert abs(info.device_bytes - est) <= 16
+                assert [bytes(r) for r in srv.results(t)] == want
+    if kind == "price":
+        req.config.paths = 8191
+        with Server(slots=1, memory_budget=1 << 62) as srv:
+            short = srv.wait(srv.submit_price(req)).device_bytes
+            req.config.paths = 8192
+            assert srv.wait(srv.submit_price(req)).device_bytes - short >= tables
