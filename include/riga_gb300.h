@@ -347,8 +347,8 @@ int32_t rg_engine_last_timing(rg_engine* engine, rg_timing* out);
 int32_t rg_set_autotune(int32_t enabled);
 /* Forces every tiled FP32 launch of the process onto one schedule: paths per thread 1 or 2, a tile
  * depth among the autotuner's candidates (24, 32, 48, 64, 80, 96, 128) and a block of
- * paths_per_block paths per CTA tile (0 = the formula's, which follows the scenario and path counts;
- * otherwise a power of two of at least 32 × paths per thread); (0, 0, 0) returns to the formula shape
+ * paths_per_block paths per CTA tile (0 = the formula's, which follows the scenario and path counts, or
+ * the largest below it that fits; otherwise a power of two of at least 32 × paths per thread); (0, 0, 0) returns to the formula shape
  * or the autotuner.  A forced shape reads local-vol rows from global memory.  One that does not fit
  * (shared memory; 1024 threads at one path per thread, 640 up to three assets and 512 beyond at two)
  * fails the pricing call with RG_ERR_INVALID_ARGUMENT.  For callers that need a fixed schedule, and for checking

@@ -336,6 +336,10 @@ Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenar
     std::lock_guard<std::mutex> lock(g_tune_mu);
     if (g_forced.ppt) {
       Fp32Shape t = apply({g_forced.pb ? g_forced.pb : sh.Pb, g_forced.ppt, g_forced.tt, 0}, npaths, true);
+      // the formula's block is chosen for two paths a thread and its own depth: the largest below it that
+      // fits what is forced
+      for (int pb = sh.Pb / 2; !t.tuned && g_forced.pb == 0 && pb >= 32; pb >>= 1)
+        t = apply({pb, g_forced.ppt, g_forced.tt, 0}, npaths, true);
       if (!t.tuned) raise(RG_ERR_INVALID_ARGUMENT, "tiled shape: the forced tile does not fit in shared memory");
       return t;
     }

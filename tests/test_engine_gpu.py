@@ -648,3 +648,31 @@ def test_direct_kernel_without_tables_agrees(engine, n, lv):
     two = engine.price_scenarios_raw(r, [(m, None)] * 2)
     assert engine.last_timing().tile_steps > 0
     assert bytes(one) == bytes(two[0])
+
+
+@pytest.mark.parametrize("n", [1, 3, 5])
+@pytest.mark.parametrize("paths", [700, 20000])
+def test_forced_shapes_take_a_block_that_fits(engine, n, paths):
+    """A forced schedule with the formula's block runs at every scenario count: one path a thread needs twice
+    the threads of the formula's two, and deep tiles more shared memory, so the block shrinks to fit."""
+    lib = engine.lib
+    req = workloads.plain3(paths, steps=140, fp32=True)
+    req.trade = workloads.phoenix_trade(n, 140, 140 / 252)
+    req.market.spots, req.market.vols = [100.0] * n, [0.2 + 0.03 * f for f in range(n)]
+    req.market.dividend_yields = [0.01] * n
+    req.market.correlation = [[1.0 if i == j else 0.4 for j in range(n)] for i in range(n)]
+    scen = []
+    for k in range(32):
+        m = copy.deepcopy(req.market)
+        m.spots[k % n] *= 1.0 + 0.002 * k
+        scen.append((m, None))
+    full = [bytes(r) for r in engine.price_scenarios_raw(req, scen)]
+    try:
+        for ppt, tt in ((1, 24), (1, 64), (1, 128), (2, 24), (2, 128)):
+            abi.check(lib, lib.rg_set_tiled_shape(ppt, tt, 0))
+            for S in (2, 5, 9, 10, 16, 17, 20, 21, 32):
+                assert [bytes(r) for r in engine.price_scenarios_raw(req, scen[:S])] == full[:S], (ppt, tt, S)
+                tm = engine.last_timing()
+                assert (tm.paths_per_thread, tm.tile_steps) == (ppt, tt)
+    finally:
+        abi.check(lib, lib.rg_set_tiled_shape(0, 0, 0))
