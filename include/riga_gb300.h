@@ -336,8 +336,8 @@ typedef struct rg_timing {
 int32_t rg_engine_last_timing(rg_engine* engine, rg_timing* out);
 
 /* The tiled FP32 kernel's autotuner (on by default, process-wide).  The first pricing call of a
- * launch shape (asset count, local vol, scenarios, steps, QMC lane, grid width) with at least
- * eight waves of path tiles times every candidate schedule — paths per CTA tile, one or two paths per
+ * launch shape (asset count, local vol, surfaces, scenarios, steps, QMC lane, grid width, the formula's
+ * paths per CTA tile) with at least eight waves of path tiles times every candidate schedule — paths per CTA tile, one or two paths per
  * thread (two: packed FP32x2 stepping), the time-tile depths, and how many steps of local-vol rows are
  * staged in shared memory — on a prefix of its paths and
  * keeps the fastest for that shape; later calls reuse it.  No knob changes a path's arithmetic

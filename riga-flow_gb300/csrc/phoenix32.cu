@@ -312,8 +312,8 @@ void p32_force_shape(int ppt, int tt, int pb) {
   g_forced = TiledKnobs{pb, ppt, tt, 0};
 }
 
-// Times every (block, paths per thread, tile depth) candidate on a prefix of the launch's paths and
-// keeps the fastest for the launch shape.  No knob changes a path's arithmetic or the 32-path
+// Times every (block, paths per thread, tile depth, staged rows) candidate on a prefix of the launch's paths
+// and keeps the fastest for the launch shape.  No knob changes a path's arithmetic or the 32-path
 // chunks of the sums, so prices are identical whichever wins.  Blocks: the formula's Pb paths per
 // tile and half of it (two smaller CTAs per SM where they fit).
 Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenario* scen,
@@ -322,8 +322,11 @@ Fp32Shape phoenix32_tune(const Prepared& P, const DevTables& tb, const DevScenar
   if (sh.direct) return sh;
   int dev = 0;
   cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-  const std::vector<int64_t> key{dev, sm_count, P.n, P.trade.has_lv, P.n_scen, P.T, P.stack_max,
-                                 P.trade.vr, P.trade.scrambler, P.trade.gx};
+  // the formula's block stands for the path count: a launch of few paths keeps its small tiles after a large
+  // one has tuned; the surfaces decide whether their rows fit shared memory
+  const bool lut = P.trade.vr == RG_VR_SOBOL && tb.sob_lut && (int32_t)((path0 + 1) & 31) == tb.sob_lut_o;
+  const std::vector<int64_t> key{dev, sm_count, P.n, P.trade.has_lv, P.n_scen, P.T, P.stack_max, P.trade.vr,
+                                 P.trade.scrambler, P.trade.gx, P.n_surf, sh.Pb, lut};
   auto apply = [&](TiledKnobs c, uint64_t paths, bool forced = false) {
     Fp32Shape t = sh;
     if (!p32_set_shape(P, t, c.pb, c.ppt, c.tt, c.rt)) return sh;

@@ -676,3 +676,26 @@ def test_forced_shapes_take_a_block_that_fits(engine, n, paths):
                 assert (tm.paths_per_thread, tm.tile_steps) == (ppt, tt)
     finally:
         abi.check(lib, lib.rg_set_tiled_shape(0, 0, 0))
+
+
+def test_a_tuned_large_launch_leaves_small_ones_their_tiles(engine):
+    """The tuned shape of a large launch serves launches of the same formula block only: afterwards a small
+    batch still has the tiles that give every SM one."""
+    lib = engine.lib
+    r = workloads.lv3(paths=1 << 12, steps=40)
+    scen = [(m, s) for _, m, s in workloads.crn15_scenarios(r)][:4]
+
+    def small():
+        r.config.paths = 1 << 12
+        got = [bytes(x) for x in engine.price_scenarios_raw(r, scen)]
+        tm = engine.last_timing()
+        return got, (tm.grid, tm.block, tm.smem_bytes, tm.tile_steps, tm.paths_per_thread)
+
+    abi.check(lib, lib.rg_set_autotune(0))
+    try:
+        want = small()
+    finally:
+        abi.check(lib, lib.rg_set_autotune(1))
+    r.config.paths = 1 << 19
+    engine.price_scenarios_raw(r, scen)
+    assert small() == want and want[1][0] == (1 << 12) // 32
