@@ -328,10 +328,10 @@ int32_t rg_merge_results(const rg_price_result* parts, int32_t n_parts, uint64_t
 typedef struct rg_timing {
   double h2d_ms, prologue_ms, kernel_ms, reduce_ms, d2h_ms, device_ms;
   uint64_t h2d_bytes, d2h_bytes;
-  int32_t kernel_launches; /* kernels this call launched (prologue + fused + reduce) */
-  int32_t grid, block, smem_bytes; /* launch shape of the fused kernel */
+  int32_t kernel_launches; /* kernels this call launched (the autotuner's timed ones aside) */
+  int32_t grid, block, smem_bytes; /* launch shape of the fused kernel (FP64: the first stepping launch) */
   int32_t tile_steps; /* steps per time tile of the tiled FP32 kernel (0 for the other kernels) */
-  int32_t paths_per_thread; /* paths each thread of the tiled FP32 kernel steps (1 or 2) */
+  int32_t paths_per_thread; /* paths each thread of the FP32 kernel steps (1 or 2; 1 for FP64) */
 } rg_timing;
 int32_t rg_engine_last_timing(rg_engine* engine, rg_timing* out);
 

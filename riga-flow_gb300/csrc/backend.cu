@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const double* __restrict__ 
 
 int reduce_groups(int rows) { return rows > kReduceRows ? (rows + kReduceRows - 1) / kReduceRows : 0; }
 
-void launch_reduce(const double* partial, int rows, int S, double* out, cudaStream_t st) {
+int launch_reduce(const double* partial, int rows, int S, double* out, cudaStream_t st) {
   const int G = reduce_groups(rows);
   if (G == 0) {
     reduce_kernel<<<dim3(S, 1), 256, 0, st>>>(partial, rows, rows, S, out);
@@ -67,6 +67,7 @@ void launch_reduce(const double* partial, int rows, int S, double* out, cudaStre
     reduce_kernel<<<dim3(S, 1), 256, 0, st>>>(groups, G, G, S, out);
   }
   cuda_check(cudaGetLastError(), "reduce_kernel launch");
+  return G == 0 ? 1 : 2;
 }
 
 size_t reduce_scratch_doubles(int rows, int S) { return (size_t)reduce_groups(rows) * S * RG_ACC; }

@@ -579,12 +579,12 @@ void price_with(Workspace& W, const rg_price_request* req, const rg_scenario* sc
     validate_request(&r2);
   }
   const int total = n_scen ? n_scen : 1;
+  if (W.timing) *W.timing = rg_timing{};
   const double* mcz = mc_lane_normals(W, req, 0, req->config.paths);
   const bool fp32 = req->config.precision == RG_PRECISION_FP32 && !mcz;
   const int per_launch = fp32 ? 32 : 1;
   const uint64_t paths = req->config.paths;
   const bool trace = req->config.trace_level != RG_TRACE_OFF;
-  if (W.timing) *W.timing = rg_timing{};
   for (int first = 0; first < total; first += per_launch) {
     const int cnt = total - first < per_launch ? total - first : per_launch;
     Prepared P;
@@ -614,25 +614,27 @@ void price_with(Workspace& W, const rg_price_request* req, const rg_scenario* sc
       lo.ko_steps = static_cast<int32_t*>(W.device(WS_KOSTEPS, paths * sizeof(int32_t)));
     }
     const uint64_t path0 = req->config.first_path;
+    Path64Launch l64{1, grid, 128, 0};  // the one-kernel form's
     if (fp32) {
       sh = phoenix32_tune(P, S.tb, S.scen, S.scen32, path0, paths, sh, lo, W.may_tune(), W.sm_count, W.stream);
       launch_phoenix32(P, S.tb, S.scen, S.scen32, path0, paths, sh, lo, W.stream);
     } else if (W.persistent()) {
-      launch_path64(W, P, S.tb, S.scen, path0, paths, lo, W.stream);
+      l64 = launch_path64(W, P, S.tb, S.scen, path0, paths, lo, W.stream);
     } else {
       launch_phoenix64(P, S.tb, S.scen, path0, paths, lo, W.stream);
     }
     if (W.timing) {
-      W.timing->block = fp32 ? sh.threads : 64;
-      W.timing->smem_bytes = fp32 ? sh.smem : 0;
+      W.timing->block = fp32 ? sh.threads : l64.block;
+      W.timing->smem_bytes = fp32 ? sh.smem : l64.smem;
       W.timing->tile_steps = fp32 && !sh.direct ? sh.TT : 0;
-      W.timing->paths_per_thread = fp32 && !sh.direct ? sh.ppt : 1;
-      W.timing->grid = fp32 ? sh.grid : grid;
-      W.timing->kernel_launches += 2;
+      W.timing->paths_per_thread = fp32 ? sh.ppt : 1;
+      W.timing->grid = fp32 ? sh.grid : l64.grid;
+      W.timing->kernel_launches += fp32 ? 1 : l64.kernels;
       W.timing->d2h_bytes += sums_bytes;
     }
     if (W.ev) cuda_check(cudaEventRecord(W.ev[3], W.stream), "event");
-    launch_reduce(lo.partial, grid, P.n_scen, dsums, W.stream);
+    const int reduces = launch_reduce(lo.partial, grid, P.n_scen, dsums, W.stream);
+    if (W.timing) W.timing->kernel_launches += reduces;
     if (W.ev) cuda_check(cudaEventRecord(W.ev[4], W.stream), "event");
     double* hs = static_cast<double*>(W.host(sums_bytes));
     cuda_check(cudaMemcpyAsync(hs, dsums, sums_bytes, cudaMemcpyDeviceToHost, W.stream), "D2H sums");

@@ -469,6 +469,7 @@ void mc_normals(uint64_t seed, uint64_t first, uint64_t count, double* d_out, Wo
     zig_emit_kernel<<<(unsigned)segs, kSegThreads, 0, s>>>(U, limit, segs, d_zt, d_accept, entry, base, first, count, d_out,
                                                            &head->status);
     cuda_check(cudaGetLastError(), "zig_emit_kernel launch");
+    if (W.timing) W.timing->kernel_launches += 6;
     Head h{};
     cuda_check(cudaMemcpyAsync(&h, head, sizeof h, cudaMemcpyDeviceToHost, s), "D2H");
     cuda_check(cudaStreamSynchronize(s), "mc parse");

@@ -453,8 +453,8 @@ Path64Plan path64_plan(int n, int64_t T, uint64_t npaths, size_t axis_bytes, siz
 }
 
 template <int N>
-void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen, uint64_t path0, uint64_t npaths,
-         const LaunchOut& out, cudaStream_t st) {
+Path64Launch run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen, uint64_t path0,
+                 uint64_t npaths, const LaunchOut& out, cudaStream_t st) {
   const int64_t T = P.T;
   const bool lv = P.trade.has_lv != 0;
   const size_t axis_bytes = lv ? (size_t)P.n_surf * P.trade.gx * sizeof(double2) : 0;
@@ -471,6 +471,7 @@ void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario
     axis64_kernel<<<(n + 127) / 128, 128, 0, st>>>(tb.lv_logs, P.trade.gx, n, reinterpret_cast<double2*>(buf));
     cuda_check(cudaGetLastError(), "axis64_kernel launch");
   }
+  Path64Launch done{lv ? 1 : 0, 0, kCtaThreads, 0};
   const size_t smem = out.mcz ? 0 : (size_t)P.stack_max * kCtaThreads * sizeof(double);
   for (a.first = 0; a.first < npaths; a.first += chunk) {
     a.npaths = std::min(chunk, npaths - a.first);
@@ -490,6 +491,11 @@ void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario
         normals64_kernel<N><<<(unsigned)(pb * tiles), kNormPaths, 0, st>>>(P.trade, tb, scen, path0 + a.first, a.npaths,
                                                                            chunk, pb, a.node0, a.node1, y);
       }
+      done.kernels += out.mcz || a.node1 > a.node0 ? 2 : 1;
+      if (done.grid == 0) {
+        done.grid = (int)blocks;
+        done.smem = (int)smem;
+      }
       cuda_check(cudaGetLastError(), "normals64 launch");
       if (lv) {
         if (out.mcz) step64_kernel<N, true, true><<<blocks, kCtaThreads, smem, st>>>(a);
@@ -502,6 +508,7 @@ void run(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario
     }
     a.partial += (size_t)blocks * RG_ACC;
   }
+  return done;
 }
 
 }  // namespace
@@ -512,14 +519,14 @@ size_t path64_bytes(int n, int64_t T, uint64_t npaths, size_t axis_bytes, size_t
   return path64_plan(n, T, npaths, axis_bytes, limit).bytes();
 }
 
-void launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen, uint64_t path0,
-                   uint64_t npaths, const LaunchOut& out, cudaStream_t st) {
+Path64Launch launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen,
+                           uint64_t path0, uint64_t npaths, const LaunchOut& out, cudaStream_t st) {
   switch (P.n) {
-    case 1: run<1>(W, P, tb, scen, path0, npaths, out, st); break;
-    case 2: run<2>(W, P, tb, scen, path0, npaths, out, st); break;
-    case 3: run<3>(W, P, tb, scen, path0, npaths, out, st); break;
-    case 4: run<4>(W, P, tb, scen, path0, npaths, out, st); break;
-    case 5: run<5>(W, P, tb, scen, path0, npaths, out, st); break;
+    case 1: return run<1>(W, P, tb, scen, path0, npaths, out, st);
+    case 2: return run<2>(W, P, tb, scen, path0, npaths, out, st);
+    case 3: return run<3>(W, P, tb, scen, path0, npaths, out, st);
+    case 4: return run<4>(W, P, tb, scen, path0, npaths, out, st);
+    case 5: return run<5>(W, P, tb, scen, path0, npaths, out, st);
     default: raise(RG_ERR_INVALID_MARKET_SHAPE, "unsupported asset count");
   }
 }

@@ -260,8 +260,11 @@ void mc_normals(uint64_t seed, uint64_t first, uint64_t count, double* d_out, Wo
 // axes, and the launch.
 uint64_t path64_rows(int n, uint64_t npaths);
 size_t path64_bytes(int n, int64_t T, uint64_t npaths, size_t axis_bytes, size_t limit);
-void launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen_dev, uint64_t path0,
-                   uint64_t npaths, const LaunchOut& out, cudaStream_t s);
+struct Path64Launch {
+  int kernels, grid, block, smem;  // kernels launched; the first stepping launch's shape
+};
+Path64Launch launch_path64(Workspace& W, const Prepared& P, const DevTables& tb, const DevScenario* scen_dev,
+                           uint64_t path0, uint64_t npaths, const LaunchOut& out, cudaStream_t s);
 // The same in one kernel and no buffer, for the static entry point (phoenix64.cu).
 int phoenix64_grid(uint64_t npaths);
 void launch_phoenix64(const Prepared& P, const DevTables& tb, const DevScenario* scen_dev,
@@ -328,7 +331,8 @@ void launch_phoenix32(const Prepared& P, const DevTables& tb, const DevScenario*
                       const Fp32Shape& shape, const LaunchOut& out, cudaStream_t s);
 // out[S][RG_ACC] = Σ over rows of partial[rows][S][RG_ACC] in a fixed order; `out` must hold
 // reduce_scratch_doubles(rows, S) more doubles after its S·RG_ACC (the first pass's group sums).
-void launch_reduce(const double* partial, int rows, int n_scen, double* out, cudaStream_t s);
+// Returns the kernels launched (one or two).
+int launch_reduce(const double* partial, int rows, int n_scen, double* out, cudaStream_t s);
 size_t reduce_scratch_doubles(int rows, int n_scen);
 
 // Cholesky factor (with the reference's PSD clamp) of one n×n correlation, n <= RG_BOOK_MAX_UNIVERSE,

@@ -699,3 +699,26 @@ def test_a_tuned_large_launch_leaves_small_ones_their_tiles(engine):
     r.config.paths = 1 << 19
     engine.price_scenarios_raw(r, scen)
     assert small() == want and want[1][0] == (1 << 12) // 32
+
+
+def test_timing_reports_what_was_launched(engine):
+    """rg_timing's launch count and shape: FP64 flat (factor, normals, steps, one reduction), the pseudo-random
+    lane (its stream's six kernels more), local vol (calibration and axes more), two reductions from 513 rows
+    of partial sums, and the direct FP32 kernel at two paths a thread (tables, factor, kernel, two reductions)."""
+    def launched(r):
+        engine.price_raw(r)
+        tm = engine.last_timing()
+        return tm.kernel_launches, tm.grid, tm.block, tm.paths_per_thread
+
+    r = workloads.plain3(paths=1000, steps=24)
+    assert launched(r) == (4, 50, 64, 1)
+    assert engine.last_timing().smem_bytes >= 5 * 64 * 8  # the bridge stack of 24 steps
+    r.config.paths = 513 * 20
+    assert launched(r) == (5, 513, 64, 1)
+    r.config.variance_reduction = VarianceReduction("none", 72)
+    assert launched(r) == (11, 513, 64, 1) and engine.last_timing().smem_bytes == 0
+    lv = workloads.lv3(paths=1000, steps=24, fp32=False)
+    assert launched(lv) == (6, 50, 64, 1)
+    two = workloads.plain3(paths=114688, steps=24, fp32=True)
+    assert launched(two)[0] == 5 and launched(two)[2:] == (256, 2)
+    assert engine.last_timing().tile_steps == 0
