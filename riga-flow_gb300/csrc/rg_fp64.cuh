@@ -32,8 +32,8 @@ __device__ __forceinline__ long long order_key(double x) {
   return (b << 1) == 0 ? 0 : b ^ ((b >> 63) & 0x7fffffffffffffffLL);
 }
 
-// 1 / d to about half an ulp for |d| in FP32's normal range: an FP32 reciprocal of d's leading bits
-// (relative error below 2^-22) and one cubic step y(1 + e + e²), e = 1 - d·y.
+// 1 / d within half an ulp and 2^-66 of itself for |d| in FP32's normal range: an FP32 reciprocal of d's
+// leading bits (|e| below 2^-22 with the bits cut off) and one cubic step y(1 + e + e²), e = 1 - d·y.
 __device__ __forceinline__ double reciprocal(double d) {
   const int h = __double2hiint(d);
   const uint32_t f = ((uint32_t)h & 0x80000000u) | ((((uint32_t)h & 0x7fffffffu) - (896u << 20)) << 3) |
@@ -47,7 +47,12 @@ __device__ __forceinline__ double reciprocal(double d) {
   return __fma_rn(y, e, y);
 }
 // n / d rounded to nearest, given y = 1 / d: the quotient estimate corrected by its exact remainder
-// (Markstein, IBM J. Res. Dev. 34, 1990).  For normal n (or zero) and quotients.
+// (Markstein, IBM J. Res. Dev. 34, 1990).  For normal n (or zero) and quotients.  With significands d in
+// [1, 2) and quotients in [1, 2), the corrected value is off by |q - n/d|·d·|y - 1/d| before it is rounded,
+// at most about 2^-107·d near a midpoint of two doubles, and an exact quotient stays 2^-105 / d or more away from
+// every midpoint, so the result is correctly rounded for a rounded y, and for `reciprocal`'s unless d is
+// within 2^-12 of 2.  There no case is known: the hardest quotients of the 2^22 divisors next below 2 and of
+// 2^25 others all round correctly (tests/test_fp64_blocks_gpu.py).
 __device__ __forceinline__ double divide_by(double n, double d, double y) {
   const double q = n * y;
   return __fma_rn(__fma_rn(-d, q, n), y, q);

@@ -146,3 +146,21 @@ def test_windows_fill_the_spot_cube(engine):
     w = np.asarray(whole.data)
     assert np.array_equal(w[:299 * 240001], np.asarray(low.data))
     assert np.array_equal(w[299 * 240001:], np.asarray(high.data))
+
+
+@pytest.mark.parametrize("n,lane,smile", [(1, "shift", None), (2, "owen", (13, 3, 40)), (3, "shift", (20, 5, 96)),
+                                          (4, "owen", None), (5, "shift", (13, 3, 25))])
+def test_records_have_the_oracles_bits(engine, n, lane, smile):
+    """Per path the lane performs the oracle's operations (its portable exponential and logarithm) in the
+    oracle's order, so every field of every record has the oracle's bits."""
+    import oracle as O
+    req = _request(n, 2000, 130, smile, lane)
+    O.set_portable_math(True)
+    try:
+        want = O.run_paths(req, 0, 2000)
+    finally:
+        O.set_portable_math(False)
+    got = _as_array(engine.run_paths_raw(req, 0, 2000))
+    for f in ("worst_final", "ko_step", "ki_hit", "qualified_steps", "paid_periods", "put_payoff", "coupon_pv",
+              "memory_coupon_pv", "funding", "pv"):
+        np.testing.assert_array_equal(got[f], np.array([getattr(r, f) for r in want], got[f].dtype), err_msg=f)
