@@ -1,5 +1,6 @@
 // backend.cu — the final fixed-order reduction and the drop-ins for the reference's `gpu`
 // backend (crates/riga-engine/src/gpu.rs): worst_of, lv_terminal_spots and the resident objects.
+#include <cfloat>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -130,10 +131,11 @@ struct LvArgs {
 
 // A log-spot below which exp(ls) / ref >= bar cannot hold: the computed exponential is within 2 ulp and
 // the division, the product and the logarithm here within 1, together below 1e-6 relative and 1e-6
-// absolute on a log-spot of up to 128.  No bound where the barrier spot is not a positive number.
+// absolute on a log-spot of up to 128.  No bound where the barrier or its spot is not a positive normal
+// number: a subnormal product or ratio is rounded by more.
 __device__ __forceinline__ float lv_ko_floor(float bar, float ref) {
   const float b = bar * ref;
-  return ref > 0.0f && b > 0.0f && b < INFINITY ? logf(b) - 1.0e-4f : -INFINITY;
+  return ref > 0.0f && bar >= FLT_MIN && b >= FLT_MIN && b < INFINITY ? logf(b) - 1.0e-4f : -INFINITY;
 }
 
 // STAGED: the rows pass through shared memory (as long as two tiles of them fit).

@@ -40,3 +40,22 @@ def test_results_do_not_depend_on_the_split(paths, steps, gx):
             assert np.array_equal(early, np.where((ko >= 0) & (ko < half), ko, -1))
         assert (ko == 0).all() if bar < 0 else True
         assert (ko == -1).all() if bar > 1e20 else True
+
+
+@pytest.mark.parametrize("bar,ref", [(1e-44, 1e30), (1e-10, 1e-34), (1e-20, 1e-24), (1.1754944e-38, 1.0), (1.0, 1.1754944e-38),
+                                     (0.7, 3.0), (1e30, 1e8)])
+def test_knock_out_at_the_rounding_of_tiny_barriers(bar, ref):
+    """Without drift and volatility a path stays at its spot, and it knocks out at once exactly where the ratio
+    of the returned spot, rounded in FP32, reaches the barrier: also where the ratio or the barrier's spot is
+    subnormal and rounds by percents, far below what separates log-spots from the barrier's."""
+    bar, ref = np.float32(bar), np.float32(ref)
+    axis = np.concatenate([np.linspace(-110.0, 89.0, 4)] * 2).astype(np.float32)
+    rows, z, q = np.zeros((2, 3, 4), np.float32), np.zeros(6, np.float32), np.zeros(2, np.float32)
+    seen = set()
+    for k in np.linspace(0.9, 1.1, 401):
+        s0 = np.float32(np.float64(bar) * np.float64(ref) * k)
+        out, ko = gpu.lv_terminal_spots(z, rows.ravel(), axis, np.float32([s0, s0]), np.float32([ref, ref]), float(bar), 1, 3, 1 / 52, 0.0, q)
+        want = 0 if out[0] / ref >= bar else -1
+        assert ko[0] == want, (k, out[0], out[0] / ref, bar)
+        seen.add(want)
+    assert seen == {0, -1}
