@@ -67,12 +67,6 @@ def flops_per_launch(paths, steps, n_assets, n_scen):
     return float(paths) * steps * per_path_step
 
 
-def tile_paths(threads, paths_per_thread, n_scen):
-    """Paths per CTA tile of a large tiled FP32 launch: the largest power of two whose stepping threads,
-    one per scenario and paths_per_thread paths, the CTA has (its other threads only generate)."""
-    return 1 << ((threads * paths_per_thread // n_scen).bit_length() - 1)
-
-
 def measured_peaks():
     try:
         return json.loads((ROOT / "MEASURED_PEAKS.json").read_text())
@@ -564,7 +558,6 @@ def run_gpu(args):
         "gpu_launches": int(tm.kernel_launches) * args.steps,
         "launch": {"grid": tm.grid, "block": tm.block, "smem_bytes": tm.smem_bytes,
                    "tile_steps": tm.tile_steps, "paths_per_thread": tm.paths_per_thread,
-                   "paths_per_cta_tile": tile_paths(tm.block, tm.paths_per_thread, n_scen),
                    "tuned_by": (f"forced by --shape {args.shape} (rg_set_tiled_shape)" if args.shape else
                                 "autotuner (rg_set_autotune): paths per CTA tile, paths per thread and tile depth, "
                                 "timed during warm-up")},
