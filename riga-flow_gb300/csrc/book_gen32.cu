@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(32 * kGenWarps, UP <= 20 ? 3 : 2) book_gen32_k
 // `rowlen` is a multiple of 64 (at least npaths).
 void launch_book_gen32(const DevTrade& gen, const DevTables& tb, const float* L32, int U, int depth, uint64_t path0,
                        uint64_t npaths, uint64_t rowlen, float* incr, cudaStream_t s) {
-  // eight nodes a tile while two CTAs fit an SM or one does (deep grids on large universes take fewer)
+  // eight nodes a tile, fewer where one CTA's shared memory would not hold them
   constexpr uint32_t kMax = 227u * 1024u;
   int nodes = kGenTile;
   while (nodes > 1 && book_gen_layout(U, depth, nodes).total > kMax) nodes >>= 1;

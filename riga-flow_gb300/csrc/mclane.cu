@@ -47,7 +47,7 @@ constexpr int kSegWords = 2048;  // B
 constexpr int kEntries = 32;     // E: a normal spans at most E words past a segment end
 constexpr int kTailIters = 64;   // tail-loop bound (each pass succeeds with probability > 0.9)
 
-constexpr int kGroupSegs = 128;  // segments one warp composes
+constexpr int kGroupSegs = 128;  // segments one CTA composes, four a warp
 constexpr int kSegThreads = 256;
 
 struct ZigTables {

@@ -14,15 +14,15 @@
 // scenario share generation and bridge only.  Time is walked in tiles of TT steps, each in three
 // phases separated by CTA barriers:
 //   G. generation — warp-wide items (bridge node, 32-path group): the Sobol integers of the group's
-//      32 consecutive points by a warp cooperation (rg_warp_sobol: shuffle reduction of the first
-//      point's Gray code, XOR scan of the Gray recurrence), the digital shift (or Owen scramble) and
-//      the FP32 inverse normal, for every factor; the standard normals of every node the tile
-//      consumes land in shared memory, 32 consecutive floats per store.  The tile's step schedule
-//      is staged beside them.
+//      32 consecutive points from the consumption-order tables (the group's high-bit term and the
+//      lane's low-bit term; without tables by a warp cooperation, rg_warp_sobol), the digital shift
+//      (or Owen scramble) and the FP32 inverse normals in packed pairs; the standard normals of every
+//      node the tile consumes land in shared memory, 32 consecutive floats per store.  The tile's step
+//      schedule is staged beside them.
 //   B. bridge — the tile's bridge nodes level by level from a host plan of the streamed Brownian
-//      bridge's dependencies, each level's (node, factor, 32-path group) items spread over all
-//      warps; then the uncorrelated increments dW[step][factor][path] and the state carried to
-//      the next tile.
+//      bridge's dependencies: a chain (factor, path) on two lanes of a warp, 16 chains a warp, with a
+//      warp barrier between levels; then the uncorrelated increments dW[step][factor][path] and the
+//      state carried to the next tile.
 //   S. scenario stepping — every (path, scenario) correlates dW with its scenario's Cholesky
 //      factor (the bridge is linear, so L·bridge(z) = bridge(L·z)), steps ln(S/S0) under flat vol
 //      or its scenario's Dupire surface and runs the Phoenix state machine.  The surfaces' rows are

@@ -297,7 +297,7 @@ __device__ static void cholesky_columns(FactorSmem& sh, int n, int lane) {
 
 // Whether the factor in `sh.l` shows every eigenvalue of its matrix to be at least 1e-5, by
 // λ_min >= 1 / Σ 1/λ_i = 1 / trace(C⁻¹) = 1 / |L⁻¹|²_F: lane j forms column j of L⁻¹ in FP32, whose
-// error (below n²·√(n·1e5)·2⁻²⁴, 13% at n = 32) is nothing against the margin to 1e-10.
+// error (below n²·√(n·1e5)·2⁻²⁴, 11% at n = 32) is nothing against the margin to 1e-10.
 __device__ static bool well_conditioned(FactorSmem& sh, int n, int lane) {
   float* inv = reinterpret_cast<float*>(sh.eig);  // [row][column]
   float* lf = inv + kFactorMax * kFactorMax;

@@ -65,9 +65,3 @@ __device__ __forceinline__ void rg_probit32x2(const uint32_t (&xa)[K], const uin
 #pragma unroll
   for (int k = 0; k < K; ++k) out[k] = __fmul2_rn(s[k], g[k]);
 }
-__device__ __forceinline__ float2 rg_probit32x2(uint32_t xa, uint32_t xb) {
-  const uint32_t a[1] = {xa}, b[1] = {xb};
-  float2 z[1];
-  rg_probit32x2(a, b, z);
-  return z[0];
-}
