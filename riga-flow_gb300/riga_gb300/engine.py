@@ -103,7 +103,7 @@ class Engine:
             if shift is not None:
                 buf = (C.c_double * len(shift))(*shift)
                 keep.append(buf)
-                arr[i].implied_vol_shift = C.cast(buf, C.POINTER(C.c_double))
+                arr[i].implied_vol_shift = buf
         out = (abi.PriceResult * len(scenarios))()
         check(self.lib, self.lib.rg_price_scenarios(self.handle, a.ptr, arr, len(scenarios), out))
         return list(out)
@@ -120,7 +120,7 @@ class Engine:
             if shift is not None:
                 buf = (C.c_double * len(shift))(*shift)
                 keep.append(buf)
-                arr[i].implied_vol_shift = C.cast(buf, C.POINTER(C.c_double))
+                arr[i].implied_vol_shift = buf
         n = C.c_int32(0)
         check(self.lib, self.lib.rg_surfaces_upload(self.handle, a.ptr, arr, len(scenarios), C.byref(n)))
         return n.value

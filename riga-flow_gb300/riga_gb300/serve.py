@@ -78,7 +78,7 @@ class Server:
                 if shift is not None:
                     buf = (C.c_double * len(shift))(*shift)
                     keep.append(buf)
-                    arr[i].implied_vol_shift = C.cast(buf, C.POINTER(C.c_double))
+                    arr[i].implied_vol_shift = buf
             n = len(scenarios)
         t = C.c_uint64()
         check(self.lib, self.lib.rg_server_submit_price(self.handle, a.ptr, arr, n, C.byref(t)))

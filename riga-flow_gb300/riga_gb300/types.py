@@ -257,12 +257,12 @@ class AbiRequest:
             for i, g in enumerate(req.local_vol):
                 grids[i].n_maturities = len(g.maturities_years)
                 grids[i].n_strikes = len(g.strikes)
-                grids[i].maturities_years = C.cast(keep(_darr(g.maturities_years)), C.POINTER(C.c_double))
-                grids[i].strikes = C.cast(keep(_darr(g.strikes)), C.POINTER(C.c_double))
-                grids[i].vols = C.cast(keep(_darr(list(chain.from_iterable(g.vols)))), C.POINTER(C.c_double))
+                grids[i].maturities_years = keep(_darr(g.maturities_years))
+                grids[i].strikes = keep(_darr(g.strikes))
+                grids[i].vols = keep(_darr(list(chain.from_iterable(g.vols))))
             keep(grids)
             r.n_local_vol = len(req.local_vol)
-            r.local_vol = C.cast(grids, C.POINTER(abi.ImpliedVolGrid))
+            r.local_vol = grids
         else:
             r.n_local_vol = 0
             r.local_vol = None
@@ -274,7 +274,7 @@ def trade_to_abi(t: PhoenixTrade, keep) -> abi.Trade:
     tr = abi.Trade()
     tr.trade_id = keep(t.trade_id.encode())
     tr.n_assets = len(t.initial_spots)
-    tr.initial_spots = C.cast(keep(_darr(t.initial_spots)), C.POINTER(C.c_double))
+    tr.initial_spots = keep(_darr(t.initial_spots))
     tr.maturity_years = t.maturity_years
     tr.steps = t.steps
     tr.strike = t.strike
@@ -346,14 +346,14 @@ class AbiBookRequest:
         for i, bt in enumerate(book.trades):
             arr[i].terms = trade_to_abi(bt.terms, keep)
             idx = (C.c_int32 * max(1, len(bt.underlyings)))(*[int(a) for a in bt.underlyings])
-            arr[i].underlyings = C.cast(keep(idx), C.POINTER(C.c_int32))
+            arr[i].underlyings = keep(idx)
         keep(arr)
         r = abi.BookRequest()
         r.universe = market_to_abi(book.universe, keep)
         r.universe_steps = int(book.universe_steps)
         r.universe_maturity_years = float(book.universe_maturity_years)
         r.n_trades = len(book.trades)
-        r.trades = C.cast(arr, C.POINTER(abi.BookTrade))
+        r.trades = arr
         cfg = config_to_abi(book.config, book.options)
         r.config = cfg
         self.req = r
@@ -381,11 +381,11 @@ def market_to_abi(m: MarketSnapshot, keep) -> abi.Market:
     mk = abi.Market()
     mk.as_of = keep(m.as_of.encode())
     mk.n_assets = len(m.spots)
-    mk.spots = C.cast(keep(_darr(m.spots)), C.POINTER(C.c_double))
-    mk.vols = C.cast(keep(_darr(m.vols)), C.POINTER(C.c_double))
+    mk.spots = keep(_darr(m.spots))
+    mk.vols = keep(_darr(m.vols))
     mk.risk_free_rate = m.risk_free_rate
-    mk.dividend_yields = C.cast(keep(_darr(m.dividend_yields)), C.POINTER(C.c_double))
-    mk.correlation = C.cast(keep(_darr([v for row in m.correlation for v in row])), C.POINTER(C.c_double))
+    mk.dividend_yields = keep(_darr(m.dividend_yields))
+    mk.correlation = keep(_darr([v for row in m.correlation for v in row]))
     return mk
 
 

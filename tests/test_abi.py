@@ -119,3 +119,23 @@ def test_per_trade_bump_rule(lib):
     assert three[11:14] == [(abi.BUMP_SPOT_PAIR, 0, 1, 0.01), (abi.BUMP_SPOT_PAIR, 0, 2, 0.01),
                             (abi.BUMP_SPOT_PAIR, 1, 2, 0.01)]
     assert trade_bump(2, 1, (0.02, 0.0, 0.0))[3] == 0.02
+
+
+def test_requests_leave_nothing_to_the_garbage_collector():
+    """A request's C form is freed with its last reference: no cycles that wait for the collector, whose pauses
+    come between a server's submissions.  (The array types of the last one live on: a few objects each.)"""
+    import gc
+
+    from riga_gb300 import workloads
+    lv, book = workloads.lv3(paths=64, steps=63), workloads.small_book(paths=64, n_trades=4, steps_per_year=52)
+    for req in (lv, book):
+        req.to_abi()  # types made on first use
+        gc.collect()
+        gc.disable()
+        try:
+            before = len(gc.get_objects())
+            for _ in range(20):
+                req.to_abi()
+            assert len(gc.get_objects()) - before < 200
+        finally:
+            gc.enable()
