@@ -11,13 +11,13 @@
 //   B. bridge — a warp takes the assets u = warp, warp + 8, ...: the streamed bridge
 //      (note.rs:89-106, qmc.rs:158-191) of each pair with the busy end of its anchor stack in shared
 //      memory [depth][asset][path], and the increments of every step that completes.
-// What bounds it: issue and the waits at the phases' barriers: 117 instructions per (node, asset, 64
-// paths): two packed inverse normals, half of the 21 multiply-adds an asset's row of the factor averages,
+// What bounds it: issue (54% active) and the waits at the phases' barriers: 132 instructions per (node, asset,
+// 64 paths): two packed inverse normals, half of the 21 multiply-adds an asset's row of the factor averages,
 // the bridge and the stores.  Up to 20 assets three CTAs fit an SM since the deep stack slots left shared
 // memory (two with all of the stack there: a book of 64 trades on 2^17 paths 53.6 ms against 52.1).
-// Measured on 20 assets × 1260 steps: 1.66 ms per 19,456 paths (one wave), against 11.0 ms for one
-// thread per (path, asset) that formed every Sobol point from its own Gray code; 2^17 paths in three
-// chunks 15.6 ms against 74 (two CTAs an SM, one pair of normals at a time).
+// Measured on 20 assets × 1260 steps: 2.22 ms per 29,184 paths (one wave of three CTAs an SM; 1.66 per 19,456
+// at two), against 11.0 ms per 19,456 for one thread per (path, asset) that formed every Sobol point from its
+// own Gray code; 2^17 paths in three chunks 15.6 ms against 74 (two CTAs an SM, one pair of normals at a time).
 // Every normal, correlation and bridge value is formed by the same operations in the same order as
 // one thread per (path, asset) forms them.
 #include <type_traits>
